@@ -181,7 +181,7 @@ struct Pair {
         r2 = x * x + y * y + z * z;
         // r and 1 / r from rsqrt, as the forward sweeps (within a few ulp)
         float r;
-        const float ri = pair_rinv_pos(r2, r);
+        const float ri = pair_rinv(r2, r);
         const float q = r * v.inv_h;
         g = kwg(q) * v.sig_h * ri;
         W2 = kwgg(q) * v.sig_h * v.inv_h;

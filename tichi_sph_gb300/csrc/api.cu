@@ -383,6 +383,9 @@ int create_impl(const tsph_params *ps, int S, const int64_t *fn, const int64_t *
         return fail(TSPH_ERR_INVALID, "total grid cells of the batch exceed 2^31");
     }
     c.st_on = st_on;
+    c.scan_r1 = ps[0].neighb_range == 1;
+    for (const SceneConst &q : sc)
+        if (!q.row_trim || q.node_num + 2 * (q.nx + q.nxny + 2) > 0x7fffffffll) c.scan_r1 = 0;
     // at least one chunk per set, owned by a scene without particles of that set
     const long long fcap = fslot > 0 ? fslot : kChunk, bcap = bslot > 0 ? bslot : kChunk;
     const long long nn = cbase, P = ps[0].phase_num;
@@ -419,7 +422,7 @@ int create_impl(const tsph_params *ps, int S, const int64_t *fn, const int64_t *
     F.inv = A.get<int>((long long)fus.size());
     F.perm = A.get<int>(fcap);
     F.perm_u = A.get<int>(fcap);
-    F.pos = A.get<float4>(fcap);
+    F.pos = A.get<float4>(fcap + kScanPad);
     F.mv = A.get<float2>(fcap);
     F.mpsi = A.get<float4>(fcap);
     F.psilo = A.get<float>(fcap);
@@ -450,7 +453,7 @@ int create_impl(const tsph_params *ps, int S, const int64_t *fn, const int64_t *
     B.inv = A.get<int>((long long)bus.size());
     B.perm = A.get<int>(bcap);
     B.perm_u = A.get<int>(bcap);
-    B.pos = A.get<float4>(bcap);
+    B.pos = A.get<float4>(bcap + kScanPad);
     B.mv = A.get<float2>(bcap);
     B.vadv = A.get<float4>(bcap);
     B.kappa = A.get<float>(bcap);

@@ -240,32 +240,28 @@ struct Scratch {
 // Kernel functions of the reference, sph_util.py:4-43 (q = r / h).
 __device__ __forceinline__ float kw(float q) {
     float a = 6.f * (q * q * q - q * q) + 1.f;
-    float b = 1.f - q;
-    return q <= 0.5f ? a : (q < 1.f ? 2.f * b * b * b : 0.f);
+    float b = fmaxf(1.f - q, 0.f);
+    return q <= 0.5f ? a : 2.f * b * b * b;
 }
 __device__ __forceinline__ float kwg(float q) {
     float a = 6.f * (3.f * q * q - 2.f * q);
-    float b = 1.f - q;
-    return q <= 0.5f ? a : (q < 1.f ? -6.f * b * b : 0.f);
+    float b = fmaxf(1.f - q, 0.f);
+    return q <= 0.5f ? a : -6.f * b * b;
 }
-// r = |x| and 1 / r from r^2 with the hardware reciprocal square root (rsqrtf,
-// within a few ulp): cheaper than an IEEE square root plus an IEEE division
-// per pair.  r^2 = 0 gives r = 0 and 1 / r = 0.
+// r = |x| and 1 / r from r^2 with the hardware reciprocal square root (within a
+// few ulp): cheaper than an IEEE square root plus an IEEE division per pair.
+// Flushing subnormals spares the instruction the scaling around it; r^2 is
+// kept at least the smallest normal number, so r^2 = 0 gives r = 0 and a finite
+// factor, and W'(0) = 0 makes the pair's gradient exactly zero.
 __device__ __forceinline__ float pair_rinv(float r2, float &r) {
-    const float inv = r2 > 0.f ? rsqrtf(r2) : 0.f;
+    float inv;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(fmaxf(r2, 1.17549435e-38f)));
     r = r2 * inv;
     return inv;
 }
 
-// The density sweeps' per-pair quotient uses __fdividef (two instructions,
-// within 2 ulp) instead of an IEEE division: far inside the 1e-5 tolerance.
-
-// pair_rinv for r^2 known to be positive (list entries).
-__device__ __forceinline__ float pair_rinv_pos(float r2, float &r) {
-    const float inv = rsqrtf(r2);
-    r = r2 * inv;
-    return inv;
-}
+// The per-pair quotients use __fdividef (a reciprocal and a product, within 2 ulp)
+// instead of an IEEE division: far inside the 1e-5 tolerance.
 
 __device__ __forceinline__ float kcoh(float q) {
     float b = 1.f - q;
@@ -442,6 +438,102 @@ __device__ __forceinline__ void visit_candidates_within(const int *__restrict__ 
     if (g.R == 1) visit_within_r1<DIM, TPP>(start, g, p, code, shift, q, f);
     else visit_within_any<DIM, TPP>(start, g, p, code, shift, q, f);
 }
+
+// The radius-1 scan in two phases per template row: test every candidate of the
+// row without a branch, its outcome one bit of a mask, then call f(j) for the
+// set bits, in candidate order.  f sees exactly the candidates with r2 < h2
+// that the one-phase visitors would show it (among the rows and end cells kept
+// by the same geometry; see visit_within_any), r2 = 0 included.  The test loop
+// is straight-line: four independent 16-byte loads, and per candidate the
+// distance, one subtraction whose sign bit is the outcome and one shift; the
+// per-hit work runs about 7 times per row and warp instead of on most of the
+// row's 18 candidates (some lane of a warp hits nearly every candidate).
+// Takes row_trim scenes whose codes stay within 32 bits over the template's
+// reach (tsph_ctx::scan_r1): a row then never aliases another.  `pos` is read
+// through the read-only path and up to kScanPad entries past the row.
+template <int DIM, class F>
+__device__ __forceinline__ void visit_hits_r1(const int *__restrict__ start, const float4 *__restrict__ pos,
+                                              const Geo &g, float4 p, long long code64, long long shift, F &&f) {
+    const int zr = (DIM == 3) ? 1 : 0;
+    const int nx = (int)g.nx, nxny = DIM == 3 ? (int)g.nxny : 0, nn = (int)g.node_num;
+    // outside by more than the template: no row holds a valid code
+    const int reach = nxny + nx + 1;
+    if (code64 + reach < 1 || code64 - reach > nn - 1) return;
+    const int code = (int)code64;
+    const float qx = __fdiv_rn(p.x - g.lb[0], g.h);
+    const float qy = __fdiv_rn(p.y - g.lb[1], g.h), qz = DIM == 3 ? __fdiv_rn(p.z - g.lb[2], g.h) : 0.f;
+    const float fx = qx - floorf(qx), fy = qy - floorf(qy), fz = qz - floorf(qz);
+    const float qm = fmaxf(fabsf(qx), fmaxf(fabsf(qy), fabsf(qz))) + 2.f;
+    const float skip2 = g.h2 * (1.f + 1e-5f + 2e-6f * qm);
+    const int *st = start + g.cbase;
+    // three bits per row, worked out once (the face distances then need no
+    // registers in the row loop): beyond h, first cell beyond h, last cell beyond h
+    unsigned int trim = 0;
+    {
+        const float ey[3] = {fy * g.h, 0.f, (1.f - fy) * g.h}, ez[3] = {fz * g.h, 0.f, (1.f - fz) * g.h};
+        const float exm = fx * g.h, exp_ = (1.f - fx) * g.h;
+#pragma unroll
+        for (int r = 0; r < (DIM == 3 ? 9 : 3); ++r) {
+            const float y = ey[r % 3], z = DIM == 3 ? ez[r / 3] : 0.f;
+            const float eyz = y * y + z * z;
+            if (eyz > skip2) trim |= 1u << (3 * r);
+            if (eyz + exm * exm > skip2) trim |= 2u << (3 * r);
+            if (eyz + exp_ * exp_ > skip2) trim |= 4u << (3 * r);
+        }
+    }
+    // the slots of template row (dy, dz), its bits lowest in t; none: beg >= end
+    auto row = [&](int dy, int dz, unsigned int t, int &beg, int &end) {
+        const int rc = code + dy * nx + dz * nxny;
+        const int lo = max((t & 2u) ? rc : rc - 1, 1);
+        const int hi = min((t & 4u) ? rc : rc + 1, nn - 1);
+        beg = end = 0;
+        if (!(t & 1u) && lo <= hi) {
+            beg = (int)(__ldg(st + lo) + shift);
+            end = (int)(__ldg(st + hi + 1) + shift);
+        }
+    };
+    int dy = -1, dz = -zr, beg, end;
+    row(dy, dz, trim, beg, end);
+#pragma unroll 1
+    for (int r = 0; r < (DIM == 3 ? 9 : 3); ++r) {
+        // the next row's slots are loaded while this row's candidates are tested
+        if (++dy > 1) {
+            dy = -1;
+            ++dz;
+        }
+        int nbeg = 0, nend = 0;
+        trim >>= 3;
+        if (r < (DIM == 3 ? 8 : 2)) row(dy, dz, trim, nbeg, nend);
+        for (int j0 = beg; j0 < end; j0 += 32) {
+            const int n = min(end - j0, 32);
+            const float4 *P = pos + j0;
+            unsigned int m = 0;
+            for (int k = 0; k < n; k += 4) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float4 pj = __ldg(P + k + e);
+                    const float dx = p.x - pj.x, dy_ = p.y - pj.y, dz_ = p.z - pj.z;
+                    const float r2 = dx * dx + dy_ * dy_ + dz_ * dz_;
+                    // r2 < h2 exactly when the rounded difference is negative
+                    m = __funnelshift_l(__float_as_uint(__fsub_rn(r2, g.h2)), m, 1);
+                }
+            }
+            // bit 31 - k: candidate j0 + k; the padding candidates drop out
+            m <<= 32 - ((n + 3) & ~3);
+            m &= 0xffffffffu << (32 - n);
+            while (m) {
+                const int b = __clz(m);
+                m ^= 0x80000000u >> b;
+                f(j0 + b);
+            }
+        }
+        beg = nbeg;
+        end = nend;
+    }
+}
+
+// entries past the end of a position array that visit_hits_r1 may read
+constexpr int kScanPad = 4;
 
 // ---------------------------------------------------------------------------------
 // Programmatic dependent launch.  The first statement of every kernel of the

@@ -20,6 +20,9 @@ struct tsph_ctx {
     int n_scenes;
     int batch;                // 0: one scene whose particle counts follow the caller's sets
     int st_on;                // some scene has surface tension
+    // the density scan's radius-1 form (visit_hits_r1) covers every scene: radius
+    // 1, row_trim, and codes with the template's reach within 32 bits
+    int scan_r1;
     int use_graph;
     int stepped;
     // cached per-substep graphs (plain, recording), keyed on the particle counts,

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kBlock, P <= 2 ? 5 : 1) k_fbm_pass(KConst k, F
                     // pair geometry from rsqrt and a fast quotient (as the other
                     // sweeps; within a few ulp)
                     float r;
-                    const float ri = pair_rinv_pos(r2, r);
+                    const float ri = pair_rinv(r2, r);
                     const float wg = kwg(r * g.inv_h) * g.sig_h;
                     const float Vj = k.vfsph ? pj.w : F.mv[j].y;  // VFSPH: X = rest volume
                     const float gx = dx * ri * wg, gy = dy * ri * wg, gz = dz * ri * wg;

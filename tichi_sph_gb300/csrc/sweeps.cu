@@ -56,6 +56,8 @@ __device__ __forceinline__ void publish_any(const KConst &k, int SceneStep::*fie
 // an FP32 sum's own rounding (a few 1e-7 of psi over ~40 terms) would be a
 // large part of it; with the error term the sum is exact to about one rounding
 // of psi, and psi's low part is kept beside it (FluidBuf::psilo).
+// (The two-lane instructions, add.rn.f32x2 and sub.rn.f32x2, did not keep the
+// remainder here: the results were those of a plain sum.)
 __device__ __forceinline__ void acc2(float &s, float &e, float y) {
     const float t = __fadd_rn(s, y);
     const float yp = __fsub_rn(t, s);
@@ -64,76 +66,12 @@ __device__ __forceinline__ void acc2(float &s, float &e, float y) {
     s = t;
 }
 
-// SPH_clean_value + SPH_prepare_attr (f,f)(f,b) + SPH_prepare_alpha_1 (f,f)(f,b)
-// + SPH_prepare_alpha_2 (f,f) + SPH_prepare_alpha (sph.py:22-38, 50-105), and the
-// neighbour list of the step.
-//
-// Two phases keep the warps converged: the candidate scan only tests r < h and
-// records the pairs with 0 < r < h (the r = 0 terms -- the particle itself and
-// coincident particles -- go straight into W / rho / compression), then the
-// recorded list is walked for the kernel arithmetic.  A particle whose pairs do
-// not fit the list redoes the scan with the arithmetic inline.
-// L (list entries, 0 < r < h known): mass / volume load beside the position,
-// no range tests; same arithmetic.
-template <int DIM, bool L = false>
-__device__ __forceinline__ void density_pair_fluid(const Geo &g, const FluidBuf &F, float4 pi, int j, float &wsum,
-                                                   float &rho, float &comp, float &a1x, float &a1y, float &a1z,
-                                                   float &a2, float &rho_e, float &comp_e) {
-    const float4 pj = F.pos[j];
-    float2 mv = make_float2(0.f, 0.f);
-    if (L) mv = F.mv[j];
-    const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    if (L || r2 < g.h2) {
-        if (!L) mv = F.mv[j];
-        float r;
-        const float ri = L ? pair_rinv_pos(r2, r) : pair_rinv(r2, r);
-        const float q = r * g.inv_h;
-        const float w = kw(q) * g.sig;
-        wsum += w;
-        acc2(rho, rho_e, __fmul_rn(w, mv.x));
-        acc2(comp, comp_e, __fmul_rn(w, mv.y));
-        if (L || r2 > 0.f) {
-            const float wg = kwg(q) * g.sig_h;
-            const float f = pj.w * wg * ri;
-            a1x += f * dx;
-            a1y += f * dy;
-            a1z += f * dz;
-            a2 += __fdividef(wg * wg * pj.w * pj.w, mv.x);
-        }
-    }
-}
-
-template <int DIM, bool L = false>
-__device__ __forceinline__ void density_pair_bound(const Geo &g, const BoundBuf &B, float4 pi, int j, float &wsum,
-                                                   float &rho, float &comp, float &a1x, float &a1y, float &a1z,
-                                                   float &rho_e, float &comp_e) {
-    const float4 pj = B.pos[j];
-    float2 mv = make_float2(0.f, 0.f);
-    if (L) mv = B.mv[j];
-    const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    if (L || r2 < g.h2) {
-        if (!L) mv = B.mv[j];
-        float r;
-        const float ri = L ? pair_rinv_pos(r2, r) : pair_rinv(r2, r);
-        const float q = r * g.inv_h;
-        const float w = kw(q) * g.sig;
-        wsum += w;
-        acc2(rho, rho_e, __fmul_rn(w, mv.x));
-        acc2(comp, comp_e, __fmul_rn(w, mv.y));
-        if (L || r2 > 0.f) {
-            const float f = pj.w * kwg(q) * g.sig_h * ri;
-            a1x += f * dx;
-            a1y += f * dy;
-            a1z += f * dz;
-        }
-    }
-}
-
-// Sums of the density sweep for one fluid particle.
+// Sums of the density sweep for one fluid particle; rho_e, comp_e: the rounding
+// errors of the additions to rho and comp.
 struct DensAcc {
-    float wsum, rho, comp, a2, a1x, a1y, a1z, pacc, rho_e, comp_e;
+    float rho, comp, rho_e, comp_e;
+    float wsum, a2, a1x, a1y, a1z, pacc;
+    int zeros;  // entries at the particle's own position (r = 0)
 };
 
 // One recorded pair (0 < r < h known) of the density sweep's list pass: the
@@ -142,14 +80,16 @@ struct DensAcc {
 // spline gradient serve all of them.  The gradient factor is formed in k_psi's
 // order, ((W'(q) sig / h) / r) X_j, so the psi term is k_psi's bit for bit.
 // FLUIDJ: the neighbour is a fluid particle (alpha_2 has no boundary term,
-// main.py:194-195).
+// main.py:194-195).  A neighbour at the particle's own position (r = 0) is counted:
+// density_exact then does the particle again.
 template <bool FLUIDJ, bool P0>
 __device__ __forceinline__ void density_list_pair(const Geo &g, float4 pi, float4 pj, float2 mv, float4 vi,
                                                   float4 vj, DensAcc &a) {
     const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
     const float r2 = dx * dx + dy * dy + dz * dz;
     float r;
-    const float ri = pair_rinv_pos(r2, r);
+    const float ri = pair_rinv(r2, r);
+    a.zeros += !(r2 > 0.f);
     const float q = r * g.inv_h;
     const float w = kw(q) * g.sig;
     a.wsum += w;
@@ -164,6 +104,118 @@ __device__ __forceinline__ void density_list_pair(const Geo &g, float4 pi, float
     if (P0) a.pacc += f * (dx * (vi.x - vj.x) + dy * (vi.y - vj.y) + dz * (vi.z - vj.z));
 }
 
+// Appends neighbour entries to sorted particle s's list, four at a time: a block
+// is collected in registers and stored as one int4 (a store per entry, each to its
+// own 16-byte piece of L2, took the density sweep 4% longer at 1M particles).
+struct ListWriter {
+    int4 *wp;
+    int64_t stride;
+    int4 blk;
+    int n, cap;
+    __device__ __forceinline__ ListWriter(int *list, int64_t s, int64_t stride_, int cap_)
+        : wp(reinterpret_cast<int4 *>(list) + s), stride(stride_), blk(make_int4(0, 0, 0, 0)), n(0), cap(cap_) {}
+    __device__ __forceinline__ void put(int j) {
+        blk = make_int4(blk.y, blk.z, blk.w, j);
+        ++n;
+        if ((n & 3) == 0 && n <= cap) {
+            *wp = blk;
+            wp += stride;
+        }
+    }
+    // stores the last, partly filled block
+    __device__ __forceinline__ void finish() {
+        const int t = n & 3;
+        if (t == 0 || n > cap) return;
+        if (t == 1) blk.x = blk.w;
+        else if (t == 2) { blk.x = blk.z; blk.y = blk.w; }
+        else { blk.x = blk.y; blk.y = blk.z; blk.z = blk.w; }
+        *wp = blk;
+    }
+};
+
+// The density sums of a particle with others at its exact position, or with
+// more neighbours than the first scan could record: the scan with the range tests
+// per candidate, which leaves the particles at r = 0 out of the list (their W(0)
+// terms go straight into the sums), then the arithmetic over the list; a list
+// that overflows without them too gives the sums of one scan and the overflow
+// mark.  Rare, so kept out of line.
+template <int DIM, bool M>
+__device__ __noinline__ void density_exact(const KConst &k, const FluidBuf &F, const BoundBuf &B, int sc, int64_t s,
+                                           bool psi0, DensAcc &out) {
+    const SceneConst &c = scene<M>(k, sc);
+    const SceneStep &st = k.ss[sc];
+    Geo g;
+    g.load(c, k.R);
+    const long long f_shift = shift_of<M>(st.f_shift), b_shift = shift_of<M>(st.b_shift);
+    const float4 pi = F.pos[s];
+    const float4 *vin = F.vadv + st.cur * F.cap;
+    const float4 vi = psi0 ? vin[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float w0 = kw(0.f) * g.sig;
+    DensAcc a = {};
+    bool ok;
+    const long long code = cell_code<DIM>(pi, g, ok);
+    ListWriter w(F.nbr, s, F.cap, k.nbr_max);
+    int nfl = 0;
+    auto scan = [&](const float4 *P, const float2 *mvs, int j) {
+        const float4 pj = P[j];
+        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+        const float r2 = dx * dx + dy * dy + dz * dz;
+        if (r2 < g.h2) {
+            if (r2 > 0.f) {
+                w.put(j);
+            } else {
+                a.wsum += w0;
+                const float2 mv = mvs[j];
+                acc2(a.rho, a.rho_e, __fmul_rn(w0, mv.x));
+                acc2(a.comp, a.comp_e, __fmul_rn(w0, mv.y));
+            }
+        }
+    };
+    if (ok) {
+        visit_candidates_within<DIM>(F.start, g, pi, code, f_shift, 0, [&](int j) { scan(F.pos, F.mv, j); });
+        nfl = w.n;
+        visit_candidates_within<DIM>(B.start, g, pi, code, b_shift, 0, [&](int j) { scan(B.pos, B.mv, j); });
+        w.finish();
+    }
+    if (w.n <= w.cap) {
+        walk_blocks<1, false>(F.nbr, s, F.cap, 0, nfl, w.n,
+            [&](int j) { density_list_pair<true, true>(g, pi, F.pos[j], F.mv[j], vi, vin[j], a); },
+            [&](int j) { density_list_pair<false, true>(g, pi, B.pos[j], B.mv[j], vi, B.vadv[j], a); });
+        F.nbr_cnt[s] = (unsigned int)nfl | ((unsigned int)(w.n - nfl) << 16);
+    } else {
+        a = {};
+        auto within = [&](float4 pj) {
+            const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+            return dx * dx + dy * dy + dz * dz < g.h2;
+        };
+        visit_candidates<DIM>(F.start, g, code, f_shift, 0, [&](int j) {
+            const float4 pj = F.pos[j];
+            if (within(pj)) density_list_pair<true, true>(g, pi, pj, F.mv[j], vi, vin[j], a);
+        });
+        visit_candidates<DIM>(B.start, g, code, b_shift, 0, [&](int j) {
+            const float4 pj = B.pos[j];
+            if (within(pj)) density_list_pair<false, true>(g, pi, pj, B.mv[j], vi, B.vadv[j], a);
+        });
+        F.nbr_cnt[s] = kNbrOverflow;
+    }
+    out = a;
+}
+
+// SPH_clean_value + SPH_prepare_attr (f,f)(f,b) + SPH_prepare_alpha_1 (f,f)(f,b)
+// + SPH_prepare_alpha_2 (f,f) + SPH_prepare_alpha (sph.py:22-38, 50-105), and the
+// neighbour list of the step.
+//
+// Two phases keep the warps converged: the candidate scan only tests r < h and
+// records the pairs, then the recorded list is walked for the kernel
+// arithmetic.  Bound by instruction issue and, nearly as much, by L1 wavefronts
+// (about 290 warp instructions per particle, L1 at 68%): the scan tests without
+// a branch (visit_hits_r1), and what only a few particles need is out of line
+// (density_exact).  64 registers, 4 blocks per SM: at 80 or 48 registers 1M
+// particles take 391 and 395 us against 365 (48 registers spill the scan's
+// loads in flight); scan and arithmetic as two launches took 389 us.  From
+// 463 us before (one test and branch per candidate, 40 registers); 205k
+// particles 120 -> 100 us, 8k 78 -> 41 us.
+//
 // In the one-scene instance the divergence solve's first psi sweep (k_psi's
 // work for its iteration 0) is done here as well when that solve will run
 // (iter_min > 0 or the carried-over compression above the tolerance, the test
@@ -173,8 +225,10 @@ __device__ __forceinline__ void density_list_pair(const Geo &g, float4 pi, float
 // scene's psi_sum goes through the same partials and ticket.  psi_ready tells
 // k_psi to skip that iteration.  (Measured: a saving in the one-scene case;
 // in the batched instance, whose scene lookups leave fewer registers, a loss.)
-template <int DIM, bool M>
-__global__ void __launch_bounds__(kBlock, 6) k_density_fluid(KConst k, FluidBuf F, BoundBuf B, double *partials) {
+template <int DIM, bool M, bool R1>
+__global__ void __launch_bounds__(kBlock, 4) k_density_fluid(const __grid_constant__ KConst k,
+                                                             const __grid_constant__ FluidBuf F,
+                                                             const __grid_constant__ BoundBuf B, double *partials) {
     pdl_entry();
     __shared__ double sh[kBlock / 32];
     __shared__ unsigned int arrived;
@@ -189,118 +243,79 @@ __global__ void __launch_bounds__(kBlock, 6) k_density_fluid(KConst k, FluidBuf 
     if (s - c.f_slot < c.f_n) {
         Geo g;
         g.load(c, k.R);
-        const long long f_shift = shift_of<M>(st.f_shift), b_shift = shift_of<M>(st.b_shift);
         const float4 pi = F.pos[s];
         const float4 *vin = F.vadv + st.cur * F.cap;
-        const float4 vi = psi0 ? vin[s] : make_float4(0.f, 0.f, 0.f, 0.f);
         bool ok;
         const long long code = cell_code<DIM>(pi, g, ok);
-        float wsum = 0.f, rho = 0.f, comp = 0.f, a2 = 0.f, pacc = 0.f, rho_e = 0.f, comp_e = 0.f;
-        float a1x = 0.f, a1y = 0.f, a1z = 0.f;
-        int nfl = 0, nbo = 0;
-        int *L = F.nbr;
-        const int64_t stride = F.cap;
-        const int cap = k.nbr_max;
-        const float w0 = kw(0.f) * g.sig;
-        // k_psi's pair term (IPPE_adv_psi), the same expression
-        auto psi_pair = [&](const float4 *P, const float4 *V, int j, auto listed) {
-            constexpr bool Ls = decltype(listed)::value;
-            const float4 pj = P[j];
-            const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-            const float r2 = dx * dx + dy * dy + dz * dz;
-            if (Ls || (r2 < g.h2 && r2 > 0.f)) {
-                const float4 vj = V[j];
-                float r;
-                const float ri = Ls ? pair_rinv_pos(r2, r) : pair_rinv(r2, r);
-                const float f = kwg(r * g.inv_h) * g.sig_h * ri * pj.w;
-                pacc += f * (dx * (vi.x - vj.x) + dy * (vi.y - vj.y) + dz * (vi.z - vj.z));
-            }
-        };
+        // phase 1: every particle within h but s itself, in candidate order, fluid
+        // first (particles at its exact position are still among them)
+        ListWriter w(F.nbr, s, F.cap, k.nbr_max);
+        int nfl = 0;
         if (ok) {
-            // phase 1: record the pairs.  The write position walks the blocked
-            // layout (entry t at nbr_index(t, s, stride)): +1 within a block of
-            // four, +4 stride - 3 to the next block.  Candidate positions load
-            // through the read-only path (no step writes them in this kernel),
-            // so they need not wait for the list stores before them
-            int nrec = 0;
-            int *wp = L + (int64_t)s * 4;
-            const int64_t next_block = stride * 4 - 3;
-            auto record = [&](int j) {
-                if (nrec < cap) {
-                    *wp = j;
-                    wp += ((nrec & 3) == 3) ? next_block : 1;
-                }
-                ++nrec;
+            const int self = (int)s;
+            auto ff = [&](int j) {
+                if (j != self) w.put(j);
             };
-            visit_candidates_within<DIM>(F.start, g, pi, code, f_shift, 0, [&](int j) {
-                const float4 pj = __ldg(&F.pos[j]);
-                const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-                const float r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 < g.h2) {
-                    if (r2 > 0.f) {
-                        record(j);
-                    } else {
-                        const float2 mv = F.mv[j];
-                        wsum += w0;
-                        acc2(rho, rho_e, __fmul_rn(w0, mv.x));
-                        acc2(comp, comp_e, __fmul_rn(w0, mv.y));
-                    }
-                }
-            });
-            nfl = nrec;
-            visit_candidates_within<DIM>(B.start, g, pi, code, b_shift, 0, [&](int j) {
-                const float4 pj = __ldg(&B.pos[j]);
-                const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-                const float r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 < g.h2) {
-                    if (r2 > 0.f) {
-                        record(j);
-                    } else {
-                        const float2 mv = B.mv[j];
-                        wsum += w0;
-                        acc2(rho, rho_e, __fmul_rn(w0, mv.x));
-                        acc2(comp, comp_e, __fmul_rn(w0, mv.y));
-                    }
-                }
-            });
-            nbo = nrec - nfl;
-            if (nfl + nbo <= cap) {
-                // phase 2: the arithmetic over the recorded pairs
-                DensAcc a = {wsum, rho, comp, 0.f, 0.f, 0.f, 0.f, 0.f, rho_e, comp_e};
-                if (psi0) {
-                    walk_blocks<1, false>(F.nbr, s, stride, 0, nfl, nfl + nbo,
-                        [&](int j) { density_list_pair<true, true>(g, pi, F.pos[j], F.mv[j], vi, vin[j], a); },
-                        [&](int j) { density_list_pair<false, true>(g, pi, B.pos[j], B.mv[j], vi, B.vadv[j], a); });
-                } else {
-                    walk_blocks<1, false>(F.nbr, s, stride, 0, nfl, nfl + nbo,
-                        [&](int j) { density_list_pair<true, false>(g, pi, F.pos[j], F.mv[j], vi, vi, a); },
-                        [&](int j) { density_list_pair<false, false>(g, pi, B.pos[j], B.mv[j], vi, vi, a); });
-                }
-                wsum = a.wsum; rho = a.rho; comp = a.comp; a2 = a.a2; pacc = a.pacc;
-                a1x = a.a1x; a1y = a.a1y; a1z = a.a1z; rho_e = a.rho_e; comp_e = a.comp_e;
+            auto fb = [&](int j) { w.put(j); };
+            if (R1) {
+                visit_hits_r1<DIM>(F.start, F.pos, g, pi, code, shift_of<M>(st.f_shift), ff);
+                nfl = w.n;
+                visit_hits_r1<DIM>(B.start, B.pos, g, pi, code, shift_of<M>(st.b_shift), fb);
             } else {
-                // list overflow: one scan with the arithmetic inline
-                wsum = rho = comp = a2 = a1x = a1y = a1z = rho_e = comp_e = 0.f;
-                visit_candidates<DIM>(F.start, g, code, f_shift, 0, [&](int j) {
-                    density_pair_fluid<DIM>(g, F, pi, j, wsum, rho, comp, a1x, a1y, a1z, a2, rho_e, comp_e);
-                    if (psi0) psi_pair(F.pos, vin, j, std::false_type{});
+                auto within = [&](const float4 *P, int j) {
+                    const float4 pj = __ldg(P + j);
+                    const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+                    return dx * dx + dy * dy + dz * dz < g.h2;
+                };
+                visit_candidates_within<DIM>(F.start, g, pi, code, shift_of<M>(st.f_shift), 0, [&](int j) {
+                    if (within(F.pos, j)) ff(j);
                 });
-                visit_candidates<DIM>(B.start, g, code, b_shift, 0, [&](int j) {
-                    density_pair_bound<DIM>(g, B, pi, j, wsum, rho, comp, a1x, a1y, a1z, rho_e, comp_e);
-                    if (psi0) psi_pair(B.pos, B.vadv, j, std::false_type{});
+                nfl = w.n;
+                visit_candidates_within<DIM>(B.start, g, pi, code, shift_of<M>(st.b_shift), 0, [&](int j) {
+                    if (within(B.pos, j)) fb(j);
                 });
+            }
+            w.finish();
+        }
+        const bool fits = w.n <= w.cap;
+        F.nbr_cnt[s] = fits ? ((unsigned int)nfl | ((unsigned int)(w.n - nfl) << 16)) : kNbrOverflow;
+        // phase 2: the arithmetic over the recorded pairs
+        DensAcc a = {};
+        if (fits) {
+            // a particle in the grid is its own candidate, at r = 0
+            if (s - c.f_slot < st.f_in) {
+                const float w0 = kw(0.f) * g.sig;
+                a.wsum = w0;
+                const float2 mv = F.mv[s];
+                acc2(a.rho, a.rho_e, __fmul_rn(w0, mv.x));
+                acc2(a.comp, a.comp_e, __fmul_rn(w0, mv.y));
+            }
+            if (psi0) {
+                const float4 vi = vin[s];
+                walk_blocks<1, false>(F.nbr, s, F.cap, 0, nfl, w.n,
+                    [&](int j) { density_list_pair<true, true>(g, pi, F.pos[j], F.mv[j], vi, vin[j], a); },
+                    [&](int j) { density_list_pair<false, true>(g, pi, B.pos[j], B.mv[j], vi, B.vadv[j], a); });
+            } else {
+                walk_blocks<1, false>(F.nbr, s, F.cap, 0, nfl, w.n,
+                    [&](int j) { density_list_pair<true, false>(g, pi, F.pos[j], F.mv[j], pi, pi, a); },
+                    [&](int j) { density_list_pair<false, false>(g, pi, B.pos[j], B.mv[j], pi, pi, a); });
             }
         }
-        F.nbr_cnt[s] = (nfl + nbo <= cap) ? ((unsigned int)nfl | ((unsigned int)nbo << 16)) : kNbrOverflow;
+        if (!fits || a.zeros) {
+            DensAcc e;  // (a itself stays in registers)
+            density_exact<DIM, M>(k, F, B, sc, s, psi0, e);
+            a = e;
+        }
         const float4 mp = F.mpsi[s];
-        float alpha = (a1x * a1x + a1y * a1y + a1z * a1z) / mp.x + a2;
+        float alpha = __fmaf_rn(a.a1z, a.a1z, __fmaf_rn(a.a1y, a.a1y, __fmul_rn(a.a1x, a.a1x))) / mp.x + a.a2;
         if (alpha < 1e-4f) alpha = 1e-4f;
         // the compensated sums rounded once; psi keeps the remainder as its low part
-        const float rho_f = __fadd_rn(rho, rho_e), comp_f = __fadd_rn(comp, comp_e);
+        const float rho_f = __fadd_rn(a.rho, a.rho_e), comp_f = __fadd_rn(a.comp, a.comp_e);
         const float psi = k.vfsph ? comp_f : rho_f;
-        const float psilo = k.vfsph ? __fsub_rn(comp_e, __fsub_rn(comp_f, comp)) : __fsub_rn(rho_e, __fsub_rn(rho_f, rho));
-        F.dens[s] = make_float4(wsum, rho_f, comp_f, a2);
-        F.a1[s] = make_float4(a1x, a1y, a1z, alpha);  // w: alpha again, for the write-back
+        const float psilo = k.vfsph ? __fsub_rn(a.comp_e, __fsub_rn(comp_f, a.comp))
+                                    : __fsub_rn(a.rho_e, __fsub_rn(rho_f, a.rho));
+        F.dens[s] = make_float4(a.wsum, rho_f, comp_f, a.a2);
+        F.a1[s] = make_float4(a.a1x, a.a1y, a.a1z, alpha);  // w: alpha again, for the write-back
         F.psilo[s] = psilo;
         F.mpsi[s] = make_float4(mp.x, psi, mp.z, alpha);
         // psi also rides in the current v_adv's unused w (the velocity sweeps carry
@@ -308,7 +323,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_density_fluid(KConst k, FluidBuf 
         F.vadv[(int64_t)st.cur * F.cap + s].w = psi;
         if (psi0) {
             // IPPE_adv_psi_init + IPPE_psi_adv_non_negative, as k_psi
-            float pa = ((psi - mp.z) + psilo) + pacc * k.sp[sc].dt;
+            float pa = ((psi - mp.z) + psilo) + a.pacc * k.sp[sc].dt;
             if (pa < 0.f) pa = 0.f;
             const float kap = pa / alpha;
             F.psiadv[s] = pa;
@@ -339,7 +354,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_density_fluid(KConst k, FluidBuf 
 
 // The boundary's own sums: SPH_prepare_attr (b,b)(b,f), SPH_prepare_alpha_2 (b,f),
 // SPH_prepare_alpha (sph.py:50-105 as called by main.py:190-197).
-template <int DIM, bool M>
+template <int DIM, bool M, bool R1>
 __global__ void __launch_bounds__(kBlock, 6) k_density_bound(KConst k, FluidBuf F, BoundBuf B) {
     pdl_entry();
     const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
@@ -364,8 +379,9 @@ __global__ void __launch_bounds__(kBlock, 6) k_density_bound(KConst k, FluidBuf 
             rho = bb.y;
             comp = bb.z;
         } else {
-            visit_candidates_within<DIM>(B.start, g, pi, code, shift_of<M>(st.b_shift), 0, [&](int j) {
-                const float4 pj = B.pos[j];
+            // (B.pos is not written here: the read-only path, as in the fluid sweep)
+            auto bb_pair = [&](int j) {
+                const float4 pj = __ldg(&B.pos[j]);
                 const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
                 const float r2 = dx * dx + dy * dy + dz * dz;
                 if (r2 < g.h2) {
@@ -377,11 +393,13 @@ __global__ void __launch_bounds__(kBlock, 6) k_density_bound(KConst k, FluidBuf 
                     rho += w * mv.x;
                     comp += w * mv.y;
                 }
-            });
+            };
+            if (R1) visit_hits_r1<DIM>(B.start, B.pos, g, pi, code, shift_of<M>(st.b_shift), bb_pair);
+            else visit_candidates_within<DIM>(B.start, g, pi, code, shift_of<M>(st.b_shift), 0, bb_pair);
             B.bb[s] = make_float4(wsum, rho, comp, 0.f);
         }
-        visit_candidates_within<DIM>(F.start, g, pi, code, shift_of<M>(st.f_shift), 0, [&](int j) {
-            const float4 pj = F.pos[j];
+        auto bf_pair = [&](int j) {
+            const float4 pj = __ldg(&F.pos[j]);
             const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
             const float r2 = dx * dx + dy * dy + dz * dz;
             if (r2 < g.h2) {
@@ -398,7 +416,9 @@ __global__ void __launch_bounds__(kBlock, 6) k_density_bound(KConst k, FluidBuf 
                     a2 += __fdividef(wg * wg * pj.w * pj.w, mv.x);
                 }
             }
-        });
+        };
+        if (R1) visit_hits_r1<DIM>(F.start, F.pos, g, pi, code, shift_of<M>(st.f_shift), bf_pair);
+        else visit_candidates_within<DIM>(F.start, g, pi, code, shift_of<M>(st.f_shift), 0, bf_pair);
     }
     const float m = B.mv[s].x;
     float alpha = 0.f / m + a2;
@@ -497,7 +517,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_psi(KConst k, FluidBuf F, BoundBu
             if (L || (r2 < g.h2 && r2 > 0.f)) {
                 if (!L) vj = V[j];
                 float r;
-                const float ri = L ? pair_rinv_pos(r2, r) : pair_rinv(r2, r);
+                const float ri = pair_rinv(r2, r);
                 const float f = kwg(r * g.inv_h) * g.sig_h * ri * pj.w;
                 acc += f * (dx * (vi.x - vj.x) + dy * (vi.y - vj.y) + dz * (vi.z - vj.z));
             }
@@ -580,7 +600,7 @@ __global__ void __launch_bounds__(kBlock) k_vel(KConst k, FluidBuf F, BoundBuf B
                 const float r2 = dx * dx + dy * dy + dz * dz;
                 if (L || (r2 < g.h2 && r2 > 0.f)) {
                     float r;
-                    const float ri = L ? pair_rinv_pos(r2, r) : pair_rinv(r2, r);
+                    const float ri = pair_rinv(r2, r);
                     const float f = qj.w * (kwg(r * g.inv_h) * g.sig_h * ri);
                     sx = valid ? sx + f * dx : sx;
                     sy = valid ? sy + f * dy : sy;
@@ -662,7 +682,7 @@ __global__ void __launch_bounds__(kBlock) k_normal(KConst k, FluidBuf F, BoundBu
                 if (L || (r2 < g.h2 && r2 > 0.f)) {
                     if (!L) psij = F.mpsi[j].y;
                     float r;
-                    const float ri = L ? pair_rinv_pos(r2, r) : pair_rinv(r2, r);
+                    const float ri = pair_rinv(r2, r);
                     const float f = -__fdividef(pj.w, psij) * (kwg(r * g.inv_h) * g.sig_h) * ri;
                     nx += f * dx;
                     ny += f * dy;
@@ -778,7 +798,7 @@ __global__ void __launch_bounds__(kBlock, M ? 1 : 5) k_advect(KConst k, FluidBuf
                     const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
                     const float r2 = dx * dx + dy * dy + dz * dz;
                     float r;
-                    const float ri = pair_rinv_pos(r2, r);
+                    const float ri = pair_rinv(r2, r);
                     const float wg = kwg(r * g.inv_h) * g.sig_h;
                     const float adx = (vi.x - vj.x) * dx + (vi.y - vj.y) * dy + (vi.z - vj.z) * dz;
                     // the two quotients by __fdividef (within 2 ulp, far inside the
@@ -841,6 +861,17 @@ __global__ void __launch_bounds__(kBlock, M ? 1 : 5) k_advect(KConst k, FluidBuf
     if (MULTI) { constexpr bool M = true; __VA_ARGS__; }                   \
     else { constexpr bool M = false; __VA_ARGS__; }
 
+template <bool M, bool R1>
+static void launch_density_r1(tsph_ctx &c, cudaStream_t st, cudaStream_t sd) {
+    if (c.k.dim == 3) {
+        TSPH_LAUNCH((k_density_bound<3, M, R1>), blocks_for(c.B.cap), kBlock, sd, c.k, c.F, c.B);
+        TSPH_LAUNCH((k_density_fluid<3, M, R1>), blocks_for(c.F.cap), kBlock, st, c.k, c.F, c.B, c.S.partials);
+    } else {
+        TSPH_LAUNCH((k_density_bound<2, M, R1>), blocks_for(c.B.cap), kBlock, sd, c.k, c.F, c.B);
+        TSPH_LAUNCH((k_density_fluid<2, M, R1>), blocks_for(c.F.cap), kBlock, st, c.k, c.F, c.B, c.S.partials);
+    }
+}
+
 // The boundary particles' own sums run on the side stream beside the fluid
 // sweep: neither writes what the other reads.
 void launch_density(tsph_ctx &c, cudaStream_t st) {
@@ -848,13 +879,8 @@ void launch_density(tsph_ctx &c, cudaStream_t st) {
     cudaStream_t sd = c.side ? c.side : st;
     fork_side(c, st);
     TSPH_M_DISPATCH(c.n_scenes > 1,
-        if (c.k.dim == 3) {
-            TSPH_LAUNCH((k_density_bound<3, M>), blocks_for(c.B.cap), kBlock, sd, c.k, c.F, c.B);
-            TSPH_LAUNCH((k_density_fluid<3, M>), blocks_for(c.F.cap), kBlock, st, c.k, c.F, c.B, c.S.partials);
-        } else {
-            TSPH_LAUNCH((k_density_bound<2, M>), blocks_for(c.B.cap), kBlock, sd, c.k, c.F, c.B);
-            TSPH_LAUNCH((k_density_fluid<2, M>), blocks_for(c.F.cap), kBlock, st, c.k, c.F, c.B, c.S.partials);
-        })
+        if (c.scan_r1) launch_density_r1<M, true>(c, st, sd);
+        else launch_density_r1<M, false>(c, st, sd);)
     join_side(c, st);
 }
 
