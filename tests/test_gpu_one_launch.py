@@ -1,0 +1,104 @@
+"""The one-launch substep against the separate kernels, bit for bit (needs a GPU).
+
+With the solver loops on the device, one-scene contexts up to a size run a substep as
+one cooperative kernel; with host-driven loops the same particle code runs as
+separate kernels.  Both add every sum in the same order, so after three
+substeps every field and every scalar must be equal -- at sizes around the
+warp and the 256-slot block, with capacities beyond the particle count,
+particles outside the grid, and no boundary.
+"""
+import numpy as np
+import pytest
+import torch
+
+from tests.test_gpu_grid_edges import _cloud, _need_cuda, _scene
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("pos", "vel", "vel_adv", "acce_adv", "alpha_1", "mass", "rest_density", "volume_frac", "W", "sph_density",
+          "sph_compression", "psi_adv", "alpha", "alpha_2", "flag", "neighb_cell_seq", "neighb_in_cell_seq",
+          "neighb_cell_structured_seq")
+SCALARS = ("dt", "time_count", "compression", "kinetic_energy", "potential_energy", "div_iter", "incom_iter",
+           "fbm_passes", "general_flag", "status", "fluid_in_grid", "bound_in_grid", "steps", "total_div_iter",
+           "total_incom_iter", "total_fbm_passes", "max_dens_compression")
+
+
+def _solver(dim, n, nb, two, use_graph):
+    from tichi_sph_gb300 import Fluid, Solver, sph_config
+    cfg_d, scen, span = _scene(dim, 6)
+    scen["sim_env"]["gravity"] = [0.0, -9.81, 0.0][:dim]
+    if two:
+        cfg_d.update(solver_type="VFSPH", solver_surface_tension_gamma=0.07, solver_fbm_convection_term=50.0)
+        scen["sim_env"].update(phase_num=2, phase_rest_density=[1000, 500],
+                               phase_color_hex=["0x6F7DBC", "0xFA8012"])
+    cfg = sph_config.Config(cfg_d, scen)
+    rng = np.random.default_rng(31 * n + nb)
+    sets = []
+    for uid, m in enumerate((n, nb)):
+        o = Fluid(m + 300, cfg, uid, device="cuda")
+        o.part_num[None] = m
+        o.pos[:m] = torch.as_tensor(_cloud(rng, m, dim, span), device="cuda")
+        if uid == 0:
+            o.vel[:m] = torch.as_tensor(rng.normal(0, 0.3, (m, dim)).astype(np.float32), device="cuda")
+        vf = rng.uniform(0, 1, m).astype(np.float32) if two else np.ones(m, np.float32)
+        vf[::2] = 1.0
+        vf = np.stack([vf, 1 - vf], 1) if two else vf[:, None]
+        o.volume_frac[:m] = torch.as_tensor(vf, device="cuda")
+        o.rest_volume[:m] = float(cfg.part_size[dim])
+        o.update_mass_all()
+        sets.append(o)
+    return Solver(cfg, sets[0], sets[1], fbm=two, use_graph=use_graph)
+
+
+@pytest.mark.parametrize("dim,n,nb,two", [(2, 1, 0, False), (2, 33, 40, False), (2, 257, 0, True),
+                                          (2, 700, 90, True), (3, 31, 1, False), (3, 256, 257, False),
+                                          (3, 900, 300, True), (3, 5000, 700, False)])
+def test_one_launch_equals_separate_kernels(dim, n, nb, two):
+    _need_cuda()
+    runs = []
+    for use_graph in (True, False):
+        s = _solver(dim, n, nb, two, use_graph)
+        stats = []
+        for _ in range(3):
+            s.substep()
+            stats.append(s.stats())
+        assert (stats[-1]["launches_per_step"] == 1) == use_graph
+        runs.append((s, stats))
+    (a, sa), (b, sb) = runs
+    for x, y in zip(sa, sb):
+        for k in SCALARS:
+            assert x[k] == y[k] or (x[k] != x[k] and y[k] != y[k]), k
+    for oa, ob in ((a.fluid, b.fluid), (a.bound, b.bound)):
+        for f in FIELDS:
+            x, y = getattr(oa, f), getattr(ob, f)
+            assert torch.equal(torch.nan_to_num(x.double()), torch.nan_to_num(y.double())), f
+    a.close()
+    b.close()
+
+
+def test_recorded_substep_equals_plain_one():
+    _need_cuda()
+    import ctypes as C
+
+    from tichi_sph_gb300 import _native
+    outs = []
+    for use_graph in (True, False):
+        s = _solver(3, 900, 300, False, use_graph)
+        tape = C.c_void_p()
+        _native.check(s._lib.tsph_tape_create(s.ctx, 2, 100, C.byref(tape)), "tape")
+        f, b = s._sets()
+        gmu = torch.zeros(1, dtype=torch.float64, device="cuda")
+        gx, gv = torch.ones(900, 3, device="cuda"), torch.ones(900, 3, device="cuda")
+        for slot in range(2):
+            _native.check(s._lib.tsph_substep_record(s.ctx, f, b, tape, slot, None), "record")
+        ptr = lambda t, c=C.c_float: C.cast(t.data_ptr(), C.POINTER(c))  # noqa: E731
+        torch.cuda.synchronize()
+        rc = s._lib.tsph_substep_adjoint(s.ctx, tape, 0, ptr(gx), ptr(gv), ptr(gx), ptr(gv), ptr(gmu, C.c_double),
+                                         None)
+        torch.cuda.synchronize()
+        outs.append((rc, gx, gv, gmu, s.fluid.pos.clone()))
+        s._lib.tsph_tape_destroy(tape)
+        s.close()
+    assert outs[0][0] == outs[1][0]
+    for x, y in zip(outs[0][1:], outs[1][1:]):
+        assert torch.equal(x, y)

@@ -37,7 +37,7 @@
 #include <new>
 
 #include "ctx.h"
-#include "tape.h"
+#include "tape.cuh"
 
 namespace tsph {
 
@@ -67,70 +67,18 @@ __global__ void k_tape_begin(TapeArrays a, int slot) {
 }
 
 __global__ void __launch_bounds__(kBlock) k_tape_state(KConst k, FluidBuf F, BoundBuf B, TapeArrays a) {
-    const int slot = *a.dslot;
-    const SceneConst &c = k.s0;
-    const SceneStep &st = k.ss[0];
-    TapeMeta &m = a.meta[slot];
     const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (s < c.f_n) {
-        const int64_t o = slot * a.cap + s;
-        a.perm[o] = F.perm[s];
-        a.pos[o] = F.pos[s];
-        a.mpsi[o] = F.mpsi[s];
-        a.a1[o] = F.a1[s];
-        a.a2[o] = F.dens[s].w;
-        a.rho0[o] = F.rho0[s];
-        if (a.vf0) a.vf0[o] = F.vf[s];
-        const unsigned int pc = F.nbr_cnt[s];
-        a.cnt[o] = pc;
-        if (pc == kNbrOverflow) {
-            atomicOr(&m.status, TSPH_TAPE_LIST_OVERFLOW);
-        } else {
-            const int nb4 = ((int)(pc & 0xffffu) + (int)(pc >> 16) + 3) >> 2;
-            const int4 *src = reinterpret_cast<const int4 *>(F.nbr) + s;
-            int4 *dst = reinterpret_cast<int4 *>(a.nbr + (int64_t)slot * a.nbr_max * a.cap) + s;
-            for (int b = 0; b < nb4; ++b) dst[(int64_t)b * a.cap] = src[(int64_t)b * F.cap];
-        }
-    }
-    if (s < c.b_n) {
-        const int64_t o = slot * a.bcap + s;
-        a.bpos[o] = B.pos[s];
-        a.bvel[o] = B.vadv[s];
-        if (B.kappa[s] != 0.f) atomicOr(&m.status, TSPH_TAPE_BOUND_PSI);
-    }
-    if (s == 0) {
-        m.n = (int32_t)c.f_n;
-        m.nb = (int32_t)c.b_n;
-        m.f_in = st.f_in;
-        m.dt = k.sp[0].dt;
-        m.mu = c.mu;
-        if (st.f_in != c.f_n) atomicOr(&m.status, TSPH_TAPE_OUTSIDE_GRID);
-    }
+    tape_state_fluid_item(k, F, a, *a.dslot, s);
+    tape_state_bound_item(k, B, a, *a.dslot, s);
 }
 
-// The iterate u^k read by the psi sweep and the kappa it wrote (between the two
-// sweeps of iteration k = st.iter).
 __global__ void __launch_bounds__(kBlock) k_tape_iter(KConst k, FluidBuf F, int kind, TapeArrays a) {
     const SceneStep &st = k.ss[0];
-    if (!st.cond) return;
-    const int slot = *a.dslot;
-    const int it = st.iter;
-    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (it >= a.max_iters) {
-        if (s == 0) atomicOr(&a.meta[slot].status, TSPH_TAPE_ITER_OVERFLOW);
-        return;
-    }
-    if (s >= k.s0.f_n) return;
-    const int64_t o = (((int64_t)slot * 2 + kind) * a.max_iters + it) * a.cap + s;
-    a.u[o] = F.vadv[st.cur * F.cap + s];
-    a.kap[o] = F.kappa[s];
+    if (st.cond) tape_iter_item(k, F, a, *a.dslot, kind, st.iter, st.cur, blockIdx.x * (int64_t)kBlock + threadIdx.x);
 }
 
 __global__ void __launch_bounds__(kBlock) k_tape_vmid(KConst k, FluidBuf F, TapeArrays a) {
-    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (s >= k.s0.f_n) return;
-    a.vmid[*a.dslot * a.cap + s] = F.vel[s];
-    if (a.nrm) a.nrm[*a.dslot * a.cap + s] = F.normal[s];
+    tape_vmid_item(k, F, a, *a.dslot, blockIdx.x * (int64_t)kBlock + threadIdx.x);
 }
 
 // The fluid grid's cell starts of the recorded substep (surface tension on: its
@@ -140,11 +88,7 @@ __global__ void __launch_bounds__(kBlock) k_tape_start(FluidBuf F, TapeArrays a)
     if (i < a.nstart) a.start[(int64_t)(*a.dslot) * a.nstart + i] = F.start[i];
 }
 
-__global__ void k_tape_end(KConst k, TapeArrays a) {
-    TapeMeta &m = a.meta[*a.dslot];
-    m.kd = k.ss[0].div_iter;
-    m.kp = k.ss[0].incom_iter;
-}
+__global__ void k_tape_end(KConst k, TapeArrays a) { tape_end_item(k, a, *a.dslot); }
 
 __global__ void __launch_bounds__(kBlock) k_density_out(KConst k, FluidBuf F, float *out) {
     const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;

@@ -175,6 +175,8 @@ int enqueue_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b, cudaStream_t
     if (c.rec_tape) launch_tape_end(c, st);
     launch_unsort(c, f, b, st);
     c.launches_per_step = c.launches;
+    c.launches_per_iter = 2;
+    c.launches_per_pass = 1;
     return TSPH_OK;
 }
 
@@ -236,6 +238,19 @@ int run_step(tsph_ctx *c, const tsph_set *f, const tsph_set *b, void *stream, bo
     int rc = bind_sets(c, f, b);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
+    if (c->use_graph && small_step_fits(*c, *f, *b)) {
+        const cudaError_t e = launch_small_step(*c, *f, *b, with_cfl, st);
+        if (e == cudaSuccess) {
+            c->launches_per_step = 1;
+            c->launches_per_iter = c->launches_per_pass = 0;
+            c->stepped++;
+            return TSPH_OK;
+        }
+        // this process may not use every SM at once: separate launches from here on
+        if (e != cudaErrorCooperativeLaunchTooLarge) return fail_cuda(e, "the one-launch step");
+        (void)cudaGetLastError();
+        c->sms = 0;
+    }
     if (!c->use_graph) {
         rc = enqueue_step(*c, *f, *b, st, with_cfl, false);
         if (rc) return rc;
@@ -351,6 +366,8 @@ int create_impl(const tsph_params *ps, int S, const int64_t *fn, const int64_t *
     c.cap_b = capb;
     c.tpp = 1;
     c.use_graph = 1;
+    c.launches_per_iter = 2;
+    c.launches_per_pass = 1;
 
     std::vector<SceneConst> sc(S);
     long long cbase = 0, fslot = 0, bslot = 0, fuser = 0, buser = 0, ublk = 0;
@@ -467,6 +484,16 @@ int create_impl(const tsph_params *ps, int S, const int64_t *fn, const int64_t *
     const int64_t nscan = (nn + 4095) / 4096 + 1;
     c.S.scan_len = 2 * nscan;
     c.S.scan_blocks = A.get<int>(c.S.scan_len);
+    int dev = 0, coop = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    if (coop && S == 1) cudaDeviceGetAttribute(&c.sms, cudaDevAttrMultiProcessorCount, dev);
+    if (c.sms) {
+        c.X.sums = A.get<double>(2 * (fcap / 32));
+        c.X.vmax = A.get<float>(c.sms);
+        c.X.totals = A.get<int>(2 * c.sms);
+        c.X.bar = A.get<unsigned int>(kBarWords);
+    }
     SceneConst *d_sc = A.get<SceneConst>(S);
     k.sp = A.get<ScenePersist>(S);
     k.ss = A.get<SceneStep>(S);
@@ -550,8 +577,8 @@ void fill_stats(const tsph_ctx *c, int s, tsph_stats *out) {
     out->total_fbm_passes = d.total_fbm_passes;
     out->max_dens_compression = d.max_dens_compression;
     out->launches_per_step = c->launches_per_step;
-    out->launches_per_iter = 2;
-    out->launches_per_pass = 1;
+    out->launches_per_iter = c->launches_per_iter;
+    out->launches_per_pass = c->launches_per_pass;
 }
 
 }  // namespace
@@ -827,6 +854,8 @@ int tsph_read_scene_stats(tsph_ctx *c, int first, int count, tsph_stats *out, vo
     TSPH_CK(cudaMemcpyAsync(c->host_ss, c->k.ss, sizeof(SceneStep) * c->n_scenes, cudaMemcpyDeviceToHost, st));
     TSPH_CK(cudaMemcpyAsync(c->host_sp, c->k.sp, sizeof(ScenePersist) * c->n_scenes, cudaMemcpyDeviceToHost, st));
     TSPH_CK(cudaStreamSynchronize(st));
+    if (c->host_ss[0].status & kStGaveUp)
+        return fail(TSPH_ERR_CUDA, "the step gave up at a grid barrier: a block did not arrive");
     for (int i = 0; i < count; ++i) fill_stats(c, first + i, out + i);
     return TSPH_OK;
 }

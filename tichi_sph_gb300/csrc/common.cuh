@@ -229,6 +229,20 @@ struct BoundBuf {
     float4 *bb;
 };
 
+// Scratch of the one-launch step (small.cuh): per-warp sums, per-block maxima and
+// cell totals, the grid barrier's words (each in a line of its own).
+enum { kBarCount = 0, kBarGaveUp = 32, kBarLeft = 64, kBarWords = 96 };
+constexpr int kSmallSums = 512;  // block sums held in shared memory at a time
+struct SmallScratch {
+    double *sums;
+    float *vmax;
+    int *totals;
+    unsigned int *bar;
+};
+
+// Step status bit (internal): the one-launch step gave up at a grid barrier.
+constexpr int kStGaveUp = 1 << 30;
+
 struct Scratch {
     double *partials;        // per-block FP64 partial sums
     int64_t partials_len;
@@ -289,6 +303,14 @@ __device__ __forceinline__ long long cell_code(float4 p, const Geo &g, bool &ok)
     return code;
 }
 
+// A load of data that an earlier launch wrote (NC: through the read-only path), or
+// that this launch may have written before a grid-wide barrier (plain).
+template <bool NC, class T>
+__device__ __forceinline__ T ld_ro(const T *p) {
+    if (NC) return __ldg(p);
+    return *p;
+}
+
 // Visits every candidate the reference's template loop visits (sph.py:52-60):
 // for each row offset (dy, dz) the x-adjacent codes [rc - R, rc + R] clipped to
 // the scene's valid range (0, node_num) form one contiguous range of sorted
@@ -296,8 +318,8 @@ __device__ __forceinline__ long long cell_code(float4 p, const Geo &g, bool &ok)
 // next row exactly like dim_encode without bounds checks.  `shift` maps a scan
 // position of the grid to a sorted slot.  Lane q of a TPP-lane group visits only
 // j = beg + q, beg + q + TPP, ...
-template <int DIM, int TPP = 1, class F>
-__device__ __forceinline__ void visit_candidates(const int *__restrict__ start, const Geo &g, long long code,
+template <int DIM, int TPP = 1, bool NC = true, class F>
+__device__ __forceinline__ void visit_candidates(const int *start, const Geo &g, long long code,
                                                  long long shift, int q, F &&f) {
     const int R = g.R;
     const int zr = (DIM == 3) ? R : 0;
@@ -308,8 +330,8 @@ __device__ __forceinline__ void visit_candidates(const int *__restrict__ start, 
             if (lo < 1) lo = 1;
             if (hi > g.node_num - 1) hi = g.node_num - 1;
             if (lo > hi) continue;
-            const int beg = (int)(__ldg(start + g.cbase + lo) + shift);
-            const int end = (int)(__ldg(start + g.cbase + hi + 1) + shift);
+            const int beg = (int)(ld_ro<NC>(start + g.cbase + lo) + shift);
+            const int end = (int)(ld_ro<NC>(start + g.cbase + hi + 1) + shift);
             for (int j = beg + q; j < end; j += TPP) f(j);
         }
     }
@@ -354,8 +376,8 @@ __device__ __forceinline__ void visit_candidates_lean(const int *__restrict__ st
 // of distance from lb, for the particle and for the candidate's own cell), so
 // the margin on h^2 grows with it too.  Without row_trim (a row could alias
 // another) the margin is infinite: every candidate is visited.
-template <int DIM, int TPP, class F>
-__device__ __forceinline__ void visit_within_any(const int *__restrict__ start, const Geo &g, float4 p,
+template <int DIM, int TPP, bool NC, class F>
+__device__ __forceinline__ void visit_within_any(const int *start, const Geo &g, float4 p,
                                                  long long code, long long shift, int q, F &&f) {
     const int R = g.R;
     const int zr = (DIM == 3) ? R : 0;
@@ -387,8 +409,8 @@ __device__ __forceinline__ void visit_within_any(const int *__restrict__ start, 
             if (lo < 1) lo = 1;
             if (hi > g.node_num - 1) hi = g.node_num - 1;
             if (lo > hi) continue;
-            const int beg = (int)(__ldg(start + g.cbase + lo) + shift);
-            const int end = (int)(__ldg(start + g.cbase + hi + 1) + shift);
+            const int beg = (int)(ld_ro<NC>(start + g.cbase + lo) + shift);
+            const int end = (int)(ld_ro<NC>(start + g.cbase + hi + 1) + shift);
             for (int j = beg + q; j < end; j += TPP) f(j);
         }
     }
@@ -397,8 +419,8 @@ __device__ __forceinline__ void visit_within_any(const int *__restrict__ start, 
 // The scan for the template radius 1: the face distances (fy h,
 // (1 - fy) h and their x and z counterparts; the general form adds an exact
 // 0.f) and the end-cell squares are computed once per particle, not per row.
-template <int DIM, int TPP, class F>
-__device__ __forceinline__ void visit_within_r1(const int *__restrict__ start, const Geo &g, float4 p,
+template <int DIM, int TPP, bool NC, class F>
+__device__ __forceinline__ void visit_within_r1(const int *start, const Geo &g, float4 p,
                                                 long long code, long long shift, int q, F &&f) {
     const int zr = (DIM == 3) ? 1 : 0;
     const float qx = __fdiv_rn(p.x - g.lb[0], g.h);
@@ -423,8 +445,8 @@ __device__ __forceinline__ void visit_within_r1(const int *__restrict__ start, c
             if (lo < 1) lo = 1;
             if (hi > g.node_num - 1) hi = g.node_num - 1;
             if (lo > hi) continue;
-            const int beg = (int)(__ldg(start + g.cbase + lo) + shift);
-            const int end = (int)(__ldg(start + g.cbase + hi + 1) + shift);
+            const int beg = (int)(ld_ro<NC>(start + g.cbase + lo) + shift);
+            const int end = (int)(ld_ro<NC>(start + g.cbase + hi + 1) + shift);
             for (int j = beg + q; j < end; j += TPP) f(j);
         }
     }
@@ -432,11 +454,11 @@ __device__ __forceinline__ void visit_within_r1(const int *__restrict__ start, c
 
 // The template radius r = 1 (the reference's configurations) in its own form,
 // any other radius read at run time; the same candidates.
-template <int DIM, int TPP = 1, class F>
-__device__ __forceinline__ void visit_candidates_within(const int *__restrict__ start, const Geo &g, float4 p,
+template <int DIM, int TPP = 1, bool NC = true, class F>
+__device__ __forceinline__ void visit_candidates_within(const int *start, const Geo &g, float4 p,
                                                         long long code, long long shift, int q, F &&f) {
-    if (g.R == 1) visit_within_r1<DIM, TPP>(start, g, p, code, shift, q, f);
-    else visit_within_any<DIM, TPP>(start, g, p, code, shift, q, f);
+    if (g.R == 1) visit_within_r1<DIM, TPP, NC>(start, g, p, code, shift, q, f);
+    else visit_within_any<DIM, TPP, NC>(start, g, p, code, shift, q, f);
 }
 
 // The radius-1 scan in two phases per template row: test every candidate of the
@@ -449,10 +471,10 @@ __device__ __forceinline__ void visit_candidates_within(const int *__restrict__ 
 // per-hit work runs about 7 times per row and warp instead of on most of the
 // row's 18 candidates (some lane of a warp hits nearly every candidate).
 // Takes row_trim scenes whose codes stay within 32 bits over the template's
-// reach (tsph_ctx::scan_r1): a row then never aliases another.  `pos` is read
-// through the read-only path and up to kScanPad entries past the row.
-template <int DIM, class F>
-__device__ __forceinline__ void visit_hits_r1(const int *__restrict__ start, const float4 *__restrict__ pos,
+// reach (tsph_ctx::scan_r1): a row then never aliases another.  `pos` is read up
+// to kScanPad entries past the row.
+template <int DIM, bool NC, class F>
+__device__ __forceinline__ void visit_hits_r1(const int *start, const float4 *pos,
                                               const Geo &g, float4 p, long long code64, long long shift, F &&f) {
     const int zr = (DIM == 3) ? 1 : 0;
     const int nx = (int)g.nx, nxny = DIM == 3 ? (int)g.nxny : 0, nn = (int)g.node_num;
@@ -488,8 +510,8 @@ __device__ __forceinline__ void visit_hits_r1(const int *__restrict__ start, con
         const int hi = min((t & 4u) ? rc : rc + 1, nn - 1);
         beg = end = 0;
         if (!(t & 1u) && lo <= hi) {
-            beg = (int)(__ldg(st + lo) + shift);
-            end = (int)(__ldg(st + hi + 1) + shift);
+            beg = (int)(ld_ro<NC>(st + lo) + shift);
+            end = (int)(ld_ro<NC>(st + hi + 1) + shift);
         }
     };
     int dy = -1, dz = -zr, beg, end;
@@ -511,7 +533,7 @@ __device__ __forceinline__ void visit_hits_r1(const int *__restrict__ start, con
             for (int k = 0; k < n; k += 4) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const float4 pj = __ldg(P + k + e);
+                    const float4 pj = ld_ro<NC>(P + k + e);
                     const float dx = p.x - pj.x, dy_ = p.y - pj.y, dz_ = p.z - pj.z;
                     const float r2 = dx * dx + dy_ * dy_ + dz_ * dz_;
                     // r2 < h2 exactly when the rounded difference is negative
@@ -667,21 +689,30 @@ __device__ __forceinline__ int4 ld_list(const int4 *p) {
     return r;
 }
 
+// The list was written by an earlier launch; by the calling thread; by this launch
+// before a grid-wide barrier (it then stays in L1 like any other data).
+enum ListLoad { kListNc, kListOwn, kListPlain };
+template <int LD>
+__device__ __forceinline__ int4 ld_block(const int4 *p) {
+    if (LD == kListNc) return ld_list_nc(p);
+    if (LD == kListOwn) return ld_list(p);
+    return *p;
+}
+
 // Walks the blocked neighbour list of sorted particle s for lane q of a TPP-lane
 // group: blocks b = q, q + TPP, ... of four entries; entries t < nfl are fluid
 // neighbours (ff), nfl <= t < ntot boundary ones (fb).  The next block's int4 is
 // loaded before the current block is processed, and the four callbacks of a
 // block only accumulate into registers, so their gathers can all be in flight
-// together.  NC = false: the list was written by the calling kernel (plain
-// loads instead of the read-only path).
-template <int TPP, bool NC = true, class FF, class FB>
+// together.  LD: how the list is loaded (kListNc, kListOwn, kListPlain).
+template <int TPP, int LD = kListNc, class FF, class FB>
 __device__ __forceinline__ void walk_blocks(const int *__restrict__ nbr, int64_t s, int64_t cap, int q,
                                             int nfl, int ntot, FF &&ff, FB &&fb) {
     const int4 *L4 = reinterpret_cast<const int4 *>(nbr) + s;
     const int nblk = (ntot + 3) >> 2;
     int b = q;
     if (b >= nblk) return;
-    auto ld = [&](int64_t i) { return NC ? ld_list_nc(L4 + i) : ld_list(L4 + i); };
+    auto ld = [&](int64_t i) { return ld_block<LD>(L4 + i); };
     int4 cur = ld((int64_t)b * cap);
     while (b < nblk) {
         const int bn = b + TPP;
@@ -706,18 +737,18 @@ __device__ __forceinline__ void walk_blocks(const int *__restrict__ nbr, int64_t
 // block's first entry in range, so the block's gathers carry no branch and can
 // all be issued before the first one is used.  Per lane, the valid entries come
 // in the same order as in walk_blocks.
-template <int TPP, class Fn>
+template <int TPP, int LD, class Fn>
 __device__ __forceinline__ void walk_range_pred(const int4 *__restrict__ L4, int64_t cap, int q, int lo, int hi,
                                                 Fn &&f) {
     if (lo >= hi) return;
     const int b0 = lo >> 2, b1 = (hi + 3) >> 2;
     int b = b0 + ((q - b0) & (TPP - 1));
     if (b >= b1) return;
-    int4 cur = ld_list_nc(L4 + (int64_t)b * cap);
+    int4 cur = ld_block<LD>(L4 + (int64_t)b * cap);
     while (b < b1) {
         const int bn = b + TPP;
         int4 nxt = cur;
-        if (bn < b1) nxt = ld_list_nc(L4 + (int64_t)bn * cap);
+        if (bn < b1) nxt = ld_block<LD>(L4 + (int64_t)bn * cap);
         const int t0 = b << 2;
         const int first = lo > t0 ? lo - t0 : 0;  // first in-range entry (0..3)
         const int jf = first == 0 ? cur.x : first == 1 ? cur.y : first == 2 ? cur.z : cur.w;
@@ -733,12 +764,12 @@ __device__ __forceinline__ void walk_range_pred(const int4 *__restrict__ L4, int
     }
 }
 
-template <int TPP, class FF, class FB>
+template <int TPP, int LD, class FF, class FB>
 __device__ __forceinline__ void walk_blocks_pred(const int *__restrict__ nbr, int64_t s, int64_t cap, int q,
                                                  int nfl, int ntot, FF &&ff, FB &&fb) {
     const int4 *L4 = reinterpret_cast<const int4 *>(nbr) + s;
-    walk_range_pred<TPP>(L4, cap, q, 0, nfl, ff);
-    walk_range_pred<TPP>(L4, cap, q, nfl, ntot, fb);
+    walk_range_pred<TPP, LD>(L4, cap, q, 0, nfl, ff);
+    walk_range_pred<TPP, LD>(L4, cap, q, nfl, ntot, fb);
 }
 
 // Neighbours of sorted fluid particle s for lane q of a TPP-lane particle group:
@@ -746,7 +777,7 @@ __device__ __forceinline__ void walk_blocks_pred(const int *__restrict__ nbr, in
 // candidate scan of the template cells.  Both visit the pairs the density sweep
 // selected; the callbacks keep their own 0 < r < h test, which is what selects
 // the pairs on the scanning path.
-template <int DIM, bool BOUND, int TPP, bool M, class FF, class FB>
+template <int DIM, bool BOUND, int TPP, bool M, bool NC = true, class FF, class FB>
 __device__ __forceinline__ void for_each_neighbor_tpp(const SceneConst &c, const SceneStep &st, int R,
                                                       const FluidBuf &F, const BoundBuf &B, int64_t s, int q,
                                                       float4 pi, FF &&ff, FB &&fb) {
@@ -757,11 +788,11 @@ __device__ __forceinline__ void for_each_neighbor_tpp(const SceneConst &c, const
         const int nfl = (int)(pc & 0xffffu), nbo = (int)(pc >> 16);
         if constexpr (std::is_invocable_v<FF &, int, std::true_type, bool>) {
             // callbacks that take a valid flag: branch-free four-entry blocks
-            walk_blocks_pred<TPP>(F.nbr, s, F.cap, q, nfl, BOUND ? nfl + nbo : nfl,
+            walk_blocks_pred<TPP, NC ? kListNc : kListPlain>(F.nbr, s, F.cap, q, nfl, BOUND ? nfl + nbo : nfl,
                                   [&](int j, bool v) { ff(j, std::true_type{}, v); },
                                   [&](int j, bool v) { fb(j, std::true_type{}, v); });
         } else {
-            walk_blocks<TPP>(F.nbr, s, F.cap, q, nfl, BOUND ? nfl + nbo : nfl,
+            walk_blocks<TPP, NC ? kListNc : kListPlain>(F.nbr, s, F.cap, q, nfl, BOUND ? nfl + nbo : nfl,
                              [&](int j) { ff(j, std::true_type{}); }, [&](int j) { fb(j, std::true_type{}); });
         }
         return;
@@ -781,8 +812,8 @@ __device__ __forceinline__ void for_each_neighbor_tpp(const SceneConst &c, const
         bool ok;
         const long long code = cell_code<DIM>(pi, g, ok);
         if (ok) {
-            visit_candidates<DIM, TPP>(F.start, g, code, 0, q, ffs);
-            if (BOUND) visit_candidates<DIM, TPP>(B.start, g, code, 0, q, fbs);
+            visit_candidates<DIM, TPP, NC>(F.start, g, code, 0, q, ffs);
+            if (BOUND) visit_candidates<DIM, TPP, NC>(B.start, g, code, 0, q, fbs);
         }
     } else {
         // batched instances: the scene's geometry is re-read from the scene table

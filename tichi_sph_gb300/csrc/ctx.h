@@ -13,6 +13,8 @@ struct tsph_ctx {
     tsph::FluidBuf F;
     tsph::BoundBuf B;
     tsph::Scratch S;
+    tsph::SmallScratch X;     // of the one-launch step
+    int sms;                  // SMs of the device; 0: no cooperative launches
     tsph::SceneConst *host_sc;  // host copy of the scene table (pinned)
     tsph::SceneStep *host_ss;   // pinned mirrors for host-loop mode and stats
     tsph::ScenePersist *host_sp;
@@ -32,6 +34,8 @@ struct tsph_ctx {
     tsph_tape *rec_tape;      // non-null while a recorded step is enqueued
     int launches;             // kernel launches enqueued (counted by the launchers)
     int launches_per_step;    // top-level kernels of the last enqueued step
+    int launches_per_iter;    // kernels of a solver iteration of the last enqueued step
+    int launches_per_pass;    // kernels of a volume-fraction pass of the last enqueued step
     int tpp;                  // threads per particle of the list sweeps (1, 2, 4, 8)
     // second stream for the boundary set's share of a phase (fork_side / join_side)
     cudaStream_t side;
@@ -112,6 +116,11 @@ void launch_tape_vmid(tsph_ctx &c, cudaStream_t st);
 void launch_tape_end(tsph_ctx &c, cudaStream_t st);
 int tape_begin(tsph_tape &t, int slot, cudaStream_t st);
 void launch_density_out(tsph_ctx &c, float *out, cudaStream_t st);
+
+// small.cu
+// Whether the step runs as one launch (launch_small_step) for these sets.
+bool small_step_fits(const tsph_ctx &c, const tsph_set &f, const tsph_set &b);
+cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b, bool with_cfl, cudaStream_t st);
 
 // fbm.cu
 void launch_fbm_begin(tsph_ctx &c, cudaGraphConditionalHandle h, int use_cond, cudaStream_t st);

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include "ctx.h"
+#include "fbm.cuh"
 
 namespace tsph {
 
@@ -43,48 +44,13 @@ __global__ void k_fbm_begin(KConst k, cudaGraphConditionalHandle h, int use_cond
     }
 }
 
-// First loop of SPH_FBM_convect, sph.py:331-345.
 template <int DIM, int P>
 __global__ void __launch_bounds__(kBlock) k_fbm_drift(KConst k, FluidBuf F) {
     pdl_entry();
     const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
     const int sc = k.f_chunk_scene[(blockIdx.x * (int64_t)kBlock) / kChunk];
     const SceneConst &c = k.sc[sc];
-    if (s - c.f_slot >= c.f_n) return;
-    const float dt = k.sp[sc].dt;
-    const float4 va = F.vadv[k.ss[sc].cur * F.cap + s];
-    const float4 v = F.vel[s];
-    const float ax = (va.x - v.x) / dt, ay = (va.y - v.y) / dt, az = (va.z - v.z) / dt;
-    const float rho0 = F.rho0[s];
-    float vf[P];
-    float zeta = 0.f;
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-        vf[q] = F.vf[q * F.cap + s];
-        zeta += vf[q] * (c.rho_phase[q] - rho0) / c.rho_phase[q];
-    }
-    const float gz = DIM == 3 ? c.g[2] : 0.f;
-    const float fx = (ax - zeta * c.g[0]) / (1.f - zeta);
-    const float fy = (ay - zeta * c.g[1]) / (1.f - zeta);
-    const float fz = (az - zeta * gz) / (1.f - zeta);
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-        const float cq = vf[q] * (c.rho_phase[q] - rho0);
-        float dx = cq * (c.g[0] - fx), dy = cq * (c.g[1] - fy), dz = cq * (gz - fz);
-        const float w = vf[q] * c.rho_phase[q];
-        if (w > 1e-6f) {
-            dx /= w; dy /= w; dz /= w;
-        } else {
-            dx *= 0.f; dy *= 0.f; dz *= 0.f;
-        }
-        dx += fx - ax; dy += fy - ay; dz += fz - az;
-        // w: the phase's volume fraction, which no pass changes (the passes
-        // read a neighbour's drift and volume fraction in one load)
-        F.drift[s * P + q] = make_float4(dx * dt, dy * dt, dz * dt, vf[q]);
-    }
-    F.acc[s] = make_float4(ax, ay, az, 0.f);
-    F.facc[s] = make_float4(fx, fy, fz, 0.f);
-    F.zeta[s] = zeta;
+    if (s - c.f_slot < c.f_n) fbm_drift_item<DIM, P>(k, F, sc, c, k.ss[sc].cur, s);
 }
 
 // One pass: SPH_FBM_clean_tmp + pair loop of SPH_FBM_convect + SPH_FBM_diffuse +
@@ -106,62 +72,7 @@ __global__ void __launch_bounds__(kBlock, P <= 2 ? 5 : 1) k_fbm_pass(KConst k, F
     __syncthreads();
     const int pass = st.fbm_pass + 1;
     if (running && s - c.f_slot < c.f_n) {
-        const int fp = F.flagpass[s];
-        float tmp[P];
-        float vfi[P];
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-            tmp[q] = 0.f;
-            vfi[q] = F.vf[q * F.cap + s];
-        }
-        if (fp == 0) {
-            Geo g;
-            g.load(c, k.R);
-            const float dt = k.sp[sc].dt;
-            const float4 pi = F.pos[s];
-            float4 ui[P];
-#pragma unroll
-            for (int q = 0; q < P; ++q) ui[q] = F.drift[s * P + q];
-            const float cc = c.fbm_c * dt, cd = dt * c.fbm_D, eps = 0.01f * g.h2;
-            for_each_neighbor_tpp<DIM, false, 1, true>(c, st, k.R, F, B, s, 0, pi,
-                [&](int j, auto) {
-                    const float4 pj = F.pos[j];
-                    const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-                    const float r2 = dx * dx + dy * dy + dz * dz;
-                    if (!(r2 < g.h2 && r2 > 0.f)) return;
-                    const int fj = F.flagpass[j];
-                    if (fj != 0 && fj != pass) return;
-                    // pair geometry from rsqrt and a fast quotient (as the other
-                    // sweeps; within a few ulp)
-                    float r;
-                    const float ri = pair_rinv(r2, r);
-                    const float wg = kwg(r * g.inv_h) * g.sig_h;
-                    const float Vj = k.vfsph ? pj.w : F.mv[j].y;  // VFSPH: X = rest volume
-                    const float gx = dx * ri * wg, gy = dy * ri * wg, gz = dz * ri * wg;
-                    const float dif = __fdividef(cd * Vj * r * wg, r2 + eps);
-#pragma unroll
-                    for (int q = 0; q < P; ++q) {
-                        const float4 uj = F.drift[(int64_t)j * P + q];
-                        const float vfj = uj.w;
-                        const float fx = vfi[q] * ui[q].x + vfj * uj.x;
-                        const float fy = vfi[q] * ui[q].y + vfj * uj.y;
-                        const float fz = vfi[q] * ui[q].z + vfj * uj.z;
-                        tmp[q] -= cc * Vj * (fx * gx + fy * gy + fz * gz);
-                        tmp[q] += (vfi[q] - vfj) * dif;
-                    }
-                },
-                [&](int, auto) {});
-        }
-        bool neg = false;
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-            F.vftmp[q * F.cap + s] = tmp[q];
-            if (vfi[q] + tmp[q] < 0.f) neg = true;
-        }
-        if (neg) {
-            if (fp == 0) F.flagpass[s] = pass;
-            any_neg = 1;
-        }
+        if (fbm_pass_item<DIM, P, true, true>(k, F, B, sc, c, st, pass, s)) any_neg = 1;
     }
     __syncthreads();
     if (running) {

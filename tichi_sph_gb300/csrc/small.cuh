@@ -1,0 +1,490 @@
+// One-launch substep of a small scene: every phase of the step inside one
+// cooperative kernel, grid-wide barriers between them.
+//
+// A scene of a few thousand particles fills a fraction of the GPU, and its
+// substep as separate launches is a chain of about thirty kernels of 2 to 10 us
+// (plus the while nodes of the solver loops): launch gaps, tail reductions and
+// cold starts, not work.  Here a phase costs its own latency and one barrier
+// (about 2 us with one block per SM), and the solver loops' tests are made by
+// every block from the same sums.  The per-particle arithmetic and the order of
+// every sum are those of the separate kernels, so the results are the same bit
+// for bit (sweeps.cuh, grid.cuh, fbm.cuh, tape.cuh hold the particle code).
+//
+// Which scenes take it: see small_step_fits.
+#pragma once
+
+#include "ctx.h"
+#include "fbm.cuh"
+#include "grid.cuh"
+#include "sweeps.cuh"
+#include "tape.cuh"
+
+namespace tsph {
+
+// Kernel arguments beside the context's own structures.
+struct SmallArgs {
+    tsph_set f, b;
+    SmallScratch x;
+    TapeArrays tape;
+    int record, with_cfl, st_on;
+};
+
+// A poll of the barrier's counter takes about half a microsecond: the limit is
+// a few seconds, after which the step is given up and its status says so.
+constexpr unsigned int kSpinLimit = 1u << 23;
+
+// Barrier over the grid's blocks (all resident: a cooperative launch).  The
+// counter only grows within a launch; the launch's last block to leave sets it
+// back.  False: a block did not arrive within the limit; every block then leaves.
+struct GridBarrier {
+    unsigned int *bar;  // words kBarCount, kBarGaveUp, kBarLeft
+    unsigned int target;
+    static __device__ __forceinline__ unsigned int acquire(const unsigned int *p) {
+        unsigned int v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ bool sync() {
+        __shared__ int ok;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            target += gridDim.x;
+            // release / acquire at GPU scope, with the block's two barriers around
+            // them, order everything before against everything after
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar + kBarCount) : "memory");
+            bool all = true;
+            unsigned int n = 0;
+            while (acquire(bar + kBarCount) < target) {
+                if ((++n & 1023u) != 0) continue;
+                if (n > kSpinLimit) atomicExch(bar + kBarGaveUp, 1u);
+                if (acquire(bar + kBarGaveUp)) {
+                    all = false;
+                    break;
+                }
+            }
+            ok = all;
+        }
+        __syncthreads();
+        return ok != 0;
+    }
+};
+
+// The block's share of n items, in whole warps: contiguous runs of 32.
+struct WarpShare {
+    int64_t first, last;  // warps [first, last) of the items, before the end is cut off
+    __device__ __forceinline__ WarpShare(int64_t n) {
+        const int64_t nw = (n + 31) >> 5;
+        const int64_t per = (nw + gridDim.x - 1) / gridDim.x;
+        first = blockIdx.x * per;
+        last = first + per < nw ? first + per : nw;
+        if (first > last) first = last;
+    }
+    __device__ __forceinline__ int64_t count() const { return last - first; }
+};
+
+// Runs ff(i, warp) over the fluid's nf items and fb(i) over the boundary's nb in
+// the block's warps (every lane of a warp calls, i may be past the end).
+template <class FF, class FB>
+__device__ __forceinline__ void for_items(int64_t nf, int64_t nb, FF &&ff, FB &&fb) {
+    const WarpShare f(nf), b(nb);
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int64_t total = f.count() + b.count();
+    for (int64_t w = threadIdx.x >> 5; w < total; w += warps) {
+        if (w < f.count()) ff((f.first + w) * 32 + lane, f.first + w);
+        else fb((b.first + w - f.count()) * 32 + lane);
+    }
+}
+
+// Inclusive scan over the block; total in every thread.
+__device__ __forceinline__ int small_block_scan(int v, int *sh, int &total) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    __syncthreads();
+    if (lane == 31) sh[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        int u = lane < warps ? sh[lane] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, u, o);
+            if (lane >= o) u += y;
+        }
+        sh[lane] = u;
+    }
+    __syncthreads();
+    total = sh[31];
+    return x + (w > 0 ? sh[w - 1] : 0);
+}
+
+// Sum of per-warp sums in the order the separate kernels add them: the eight warps
+// of a 256-slot block one after another, block sums by lanes 32 apart, then the
+// lanes' tree.  All threads of the block call; the result is in thread 0.
+__device__ __forceinline__ double small_psi_sum(const double *warp_sums, int64_t slots, double *sh) {
+    const int64_t nblk = slots / kBlock;
+    const int lane = threadIdx.x & 31;
+    double acc = 0.0;
+    for (int64_t b0 = 0; b0 < nblk; b0 += kSmallSums) {
+        const int m = (int)(nblk - b0 < kSmallSums ? nblk - b0 : kSmallSums);
+        __syncthreads();
+        for (int i = threadIdx.x; i < m; i += blockDim.x) {
+            const double *p = warp_sums + (b0 + i) * (kBlock / 32);
+            double s = 0.0;
+#pragma unroll
+            for (int q = 0; q < kBlock / 32; ++q) s += __ldcg(p + q);
+            sh[i] = s;
+        }
+        __syncthreads();
+        if (threadIdx.x < 32)
+            for (int i = lane; i < m; i += 32) acc += sh[i];
+    }
+    if (threadIdx.x < 32) acc = warp_sum(acc);
+    return acc;
+}
+
+// The tree of block_sum over a 256-thread block's eight warp sums.
+__device__ __forceinline__ double small_block_tree(const double *p) {
+    double v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __ldcg(p + i);
+    return ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
+}
+
+// P: phases of the volume-fraction update, 0 without it.
+template <int DIM, bool ST, int P>
+struct SmallStep {
+    const KConst &k;
+    const FluidBuf &F;
+    const BoundBuf &B;
+    const SmallArgs &a;
+    GridBarrier bar;
+    double *sh_d;
+    int *sh_i;
+    int64_t ns;  // the fluid's slots in whole blocks of the separate kernels
+    int cur;  // the current v_adv buffer: the same in every thread of the grid
+
+    __device__ __forceinline__ SceneStep &st() const { return k.ss[0]; }
+    __device__ __forceinline__ bool first_block() const { return blockIdx.x == 0; }
+    __device__ __forceinline__ bool last_block() const { return blockIdx.x == gridDim.x - 1; }
+
+    // Zeroes the step's counters; with the CFL condition on, the block's largest |v|.
+    __device__ __forceinline__ void begin() {
+        const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+        for (int64_t i = tid; i < k.total_nodes; i += nt) {
+            F.count[i] = 0;
+            B.count[i] = 0;
+        }
+        if (tid < (int64_t)(sizeof(SceneStep) / 4)) reinterpret_cast<int *>(&st())[tid] = 0;
+        if (!a.with_cfl) return;
+        float m = 0.f;
+        for (int64_t i = tid; i < a.f.n; i += nt) {
+            float s = 0.f;
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+                const float v = a.f.vel[i * DIM + d];
+                s += v * v;
+            }
+            const float vn = sqrtf(s);
+            if (vn > 1e-4f) m = fmaxf(m, vn);  // NaN norms fail the test, as in the reference
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        float *sh = reinterpret_cast<float *>(sh_i);
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmaxf(m, sh[w]);
+            a.x.vmax[blockIdx.x] = m;
+        }
+    }
+
+    // cfl_condition from the blocks' maxima (first block; k_cfl's arithmetic).
+    __device__ __forceinline__ void time_step() {
+        if (!a.with_cfl || !first_block() || threadIdx.x >= 32) return;
+        float vm = 0.f;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += 32) vm = fmaxf(vm, __ldcg(a.x.vmax + i));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, o));
+        if (threadIdx.x != 0) return;
+        const SceneConst &c = k.s0;
+        float dt = __fdiv_rn(c.part_size, (float)c.cs);
+        if (vm > 1e-4f) dt = fminf(dt, __fmul_rn(__fdiv_rn(c.part_size, vm), c.cfl));
+        k.sp[0].dt = dt;
+        k.sp[0].time_count += (double)dt;
+    }
+
+    // The block's cells [lo, hi) of the two grids' counts.
+    __device__ __forceinline__ void cell_range(int64_t &lo, int64_t &hi) const {
+        const int64_t per = (k.total_nodes + gridDim.x - 1) / gridDim.x;
+        lo = blockIdx.x * per < k.total_nodes ? blockIdx.x * per : k.total_nodes;
+        hi = lo + per < k.total_nodes ? lo + per : k.total_nodes;
+    }
+    __device__ __forceinline__ void count_totals() {
+        int64_t lo, hi;
+        cell_range(lo, hi);
+        for (int g = 0; g < 2; ++g) {
+            const int *count = g ? B.count : F.count;
+            int s = 0, total;
+            for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) s += __ldcg(count + i);
+            small_block_scan(s, sh_i, total);
+            if (threadIdx.x == 0) a.x.totals[2 * blockIdx.x + g] = total;
+        }
+    }
+    __device__ __forceinline__ void scan_cells() {
+        int64_t lo, hi;
+        cell_range(lo, hi);
+        for (int g = 0; g < 2; ++g) {
+            const int *count = g ? B.count : F.count;
+            int *start = g ? B.start : F.start;
+            int before = 0, total;
+            for (int i = threadIdx.x; i < (int)blockIdx.x; i += blockDim.x) before += __ldcg(a.x.totals + 2 * i + g);
+            small_block_scan(before, sh_i, total);
+            int run = total;  // particles in the cells before this block's
+            for (int64_t i0 = lo; i0 < hi; i0 += blockDim.x) {
+                const int64_t i = i0 + threadIdx.x;
+                const int v = i < hi ? __ldcg(count + i) : 0;
+                const int incl = small_block_scan(v, sh_i, total);
+                if (i < hi) start[i] = run + incl - v;
+                run += total;
+            }
+            if (last_block() && threadIdx.x == 0) {
+                start[k.total_nodes] = run;
+                if (g) st().b_in = run;
+                else st().f_in = run;
+            }
+        }
+    }
+
+    // The warp's share of the scene's psi_sum.
+    __device__ __forceinline__ void put_warp_sum(double v, int64_t warp) {
+        v = warp_sum(v);
+        if ((threadIdx.x & 31) == 0) a.x.sums[warp] = v;
+    }
+
+    // One pressure solve (k_solve_begin, k_psi, k_vel); psi_done: the first psi sweep
+    // has run.  Every block makes the loop test from the compression that the
+    // last block derives while the others update velocities.
+    __device__ __forceinline__ bool solve(int kind, bool psi_done) {
+        const SceneConst &c = k.s0;
+        const double tol = kind == kSolveDiv ? (double)c.div_tol : (double)c.comp_tol;
+        const int slot = a.record ? *a.tape.dslot : 0;
+        int it = 0;
+        bool cond = 0 < c.iter_min || *(volatile double *)&k.sp[0].compression > tol;
+        while (cond) {
+            if (!psi_done) {
+                for_items(ns, 0, [&](int64_t s, int64_t w) {
+                    const Lanes<1> ln;
+                    put_warp_sum(psi_item<DIM, 1, false, false>(k, F, B, 0, c, st(), cur, ln, s, s < c.f_n), w);
+                }, [](int64_t) {});
+                if (!bar.sync()) return false;
+            }
+            psi_done = false;
+            for_items(ns, 0, [&](int64_t s, int64_t) {
+                const Lanes<1> ln;
+                if (a.record) tape_iter_item(k, F, a.tape, slot, kind, it, cur, s);
+                vel_item<DIM, 1, false, false>(k, F, B, 0, c, st(), cur, ln, s, s < c.f_n);
+            }, [](int64_t) {});
+            ++it;
+            const bool capped = it > c.iter_max;
+            if (last_block()) {
+                const double sum = small_psi_sum(a.x.sums, ns, sh_d);
+                if (threadIdx.x == 0) {
+                    st().psi_sum = sum;
+                    k.sp[0].compression = sum / (double)c.f_n;
+                    if (kind == kSolveDiv) st().div_iter = it;
+                    else st().incom_iter = it;
+                    if (capped) atomicOr(&st().status, kind == kSolveDiv ? TSPH_ST_DIV_ITER_CAP : TSPH_ST_DENS_ITER_CAP);
+                }
+            }
+            if (!bar.sync()) return false;
+            cur = 1 - cur;
+            cond = !capped && (it < c.iter_min || *(volatile double *)&k.sp[0].compression > tol);
+        }
+        return true;
+    }
+
+    // The volume-fraction update (k_fbm_drift, k_fbm_begin, k_fbm_pass).
+    __device__ __forceinline__ bool mixture() {
+        const SceneConst &c = k.s0;
+        for_items(c.f_n, 0, [&](int64_t s, int64_t) {
+            if (s >= c.f_n) return;
+            F.flagpass[s] = 0;
+            fbm_drift_item<DIM, P ? P : 1>(k, F, 0, c, cur, s);
+        }, [](int64_t) {});
+        if (!bar.sync()) return false;
+        int pass = 0;
+        bool flagged;
+        do {
+            ++pass;
+            for_items(c.f_n, 0, [&](int64_t s, int64_t) {
+                const bool neg = s < c.f_n && fbm_pass_item<DIM, P ? P : 1, false, false>(k, F, B, 0, c, st(), pass, s);
+                if (__any_sync(0xffffffffu, neg) && (threadIdx.x & 31) == 0) atomicMax(&st().general_flag, pass);
+            }, [](int64_t) {});
+            if (!bar.sync()) return false;
+            // (a block that is ahead may have raised it to the next pass already)
+            flagged = *(volatile int32_t *)&st().general_flag >= pass;
+        } while (flagged && pass < c.fbm_max_passes);
+        if (first_block() && threadIdx.x == 0) {
+            st().fbm_passes = pass;
+            st().gflag_out = flagged ? 1 : 0;
+            if (flagged) atomicOr(&st().status, TSPH_ST_FBM_PASS_CAP);
+        }
+        return true;
+    }
+
+    __device__ __forceinline__ bool run() {
+        const SceneConst &c = k.s0;
+        begin();
+        if (!bar.sync()) return false;
+        time_step();
+        for_items(a.f.n, a.b.n,
+                  [&](int64_t i, int64_t) { if (i < a.f.n) encode_item<DIM>(k, a.f, 0, F.count, F.slot, i); },
+                  [&](int64_t i) { if (i < a.b.n) encode_item<DIM>(k, a.b, 1, B.count, B.slot, i); });
+        if (!bar.sync()) return false;
+        count_totals();
+        if (!bar.sync()) return false;
+        scan_cells();
+        if (!bar.sync()) return false;
+        for_items(a.f.n, a.b.n,
+            [&](int64_t i, int64_t) {
+                if (i < a.f.n) scatter_item(k, 0, a.f.neighb_cell_seq, F.slot, F.start, F.perm_u, i);
+            },
+            [&](int64_t i) {
+                if (i < a.b.n) scatter_item(k, 1, a.b.neighb_cell_seq, B.slot, B.start, B.perm_u, i);
+            });
+        if (!bar.sync()) return false;
+        for_items(a.f.n, a.b.n,
+                  [&](int64_t u, int64_t) { if (u < a.f.n) gather_fluid_item<DIM>(k, a.f, F, c, st(), u); },
+                  [&](int64_t u) { if (u < a.b.n) gather_bound_item<DIM>(k, a.b, B, c, 0, u); });
+        if (!bar.sync()) return false;
+        const bool psi0 = density_does_psi(c, *(volatile double *)&k.sp[0].compression);
+        const int slot = a.record ? *a.tape.dslot : 0;
+        for_items(ns, a.b.n,
+            [&](int64_t s, int64_t w) {
+                double v = 0.0;
+                if (s < c.f_n) v = density_fluid_item<DIM, false, true, false>(k, F, B, 0, c, st(), 0, psi0, s);
+                put_warp_sum(v, w);
+                if (a.record) tape_state_fluid_item(k, F, a.tape, slot, s);
+            },
+            [&](int64_t s) {
+                if (s >= c.b_n) return;
+                density_bound_item<DIM, false, true, false>(k, F, B, c, st(), k.sp[0], s);
+                if (a.record) tape_state_bound_item(k, B, a.tape, slot, s);
+            });
+        if (ST && a.record && a.tape.start) {
+            const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+            for (int64_t i = tid; i < a.tape.nstart; i += (int64_t)gridDim.x * blockDim.x)
+                a.tape.start[(int64_t)slot * a.tape.nstart + i] = F.start[i];
+        }
+        if (!bar.sync()) return false;
+        cur = 0;
+        if (!solve(kSolveDiv, psi0)) return false;
+        if (ST) {
+            for_items(ns, 0, [&](int64_t s, int64_t) {
+                const Lanes<1> ln;
+                normal_item<DIM, 1, false, false>(k, F, B, c, st(), ln, s, s < c.f_n);
+            }, [](int64_t) {});
+            if (!bar.sync()) return false;
+        }
+        for_items(ns, 0, [&](int64_t s, int64_t) {
+            const Lanes<1> ln;
+            advect_item<DIM, ST, 1, false, false>(k, F, B, 0, c, st(), cur, ln, s, s < c.f_n, 1.f, 1.f);
+            if (a.record) tape_vmid_item(k, F, a.tape, slot, s);
+        }, [](int64_t) {});
+        if (!bar.sync()) return false;
+        cur = 1 - cur;
+        if (!solve(kSolveDens, false)) return false;
+        if (P && !mixture()) return false;
+        double *en = a.x.sums;  // the solves' sums are done with
+        for_items(ns, a.b.n,
+            [&](int64_t pid, int64_t w) {
+                double ke = 0.0, pe = 0.0;
+                if (pid < c.f_n)
+                    update_fluid_item<DIM>(k, a.f, F, 0, c, st(), cur, B.start, P ? 1 : 0, a.st_on, pid, ke, pe);
+                ke = warp_sum(ke);
+                pe = warp_sum(pe);
+                if ((threadIdx.x & 31) == 0) {
+                    en[w] = ke;
+                    en[ns / 32 + w] = pe;
+                }
+            },
+            [&](int64_t pid) { if (pid < a.b.n) update_bound_item<DIM>(k, a.b, B, F.start, pid); });
+        if (first_block() && threadIdx.x == 0) {
+            st().cur = cur;
+            if (a.record) tape_end_item(k, a.tape, slot);
+        }
+        return true;
+    }
+
+    // The last block to leave: the energies, the running totals, the barrier's reset.
+    __device__ __forceinline__ void leave(bool done) {
+        if (!last_block_done(a.x.bar + kBarLeft, gridDim.x)) return;
+        double ke = 0.0, pe = 0.0;
+        for (int64_t i = threadIdx.x; i < ns / kBlock && threadIdx.x < kBlock; i += kBlock) {
+            ke += small_block_tree(a.x.sums + i * (kBlock / 32));
+            pe += small_block_tree(a.x.sums + ns / 32 + i * (kBlock / 32));
+        }
+        ke = small_sum256(ke);
+        pe = small_sum256(pe);
+        if (threadIdx.x != 0) return;
+        if (done && !__ldcg(a.x.bar + kBarGaveUp)) {
+            st().kinetic_energy = ke;
+            st().potential_energy = pe;
+            step_totals(k.sp[0], st());
+        } else {
+            atomicOr(&st().status, kStGaveUp);
+        }
+        a.x.bar[kBarCount] = a.x.bar[kBarGaveUp] = a.x.bar[kBarLeft] = 0;
+    }
+    // block_sum<256> over the first 256 threads.
+    __device__ __forceinline__ double small_sum256(double v) {
+        v = warp_sum(v);
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0 && threadIdx.x < kBlock) sh_d[threadIdx.x >> 5] = v;
+        __syncthreads();
+        double r = 0.0;
+        if (threadIdx.x < 32) {
+            r = threadIdx.x < kBlock / 32 ? sh_d[threadIdx.x] : 0.0;
+            r = warp_sum(r);
+        }
+        return r;
+    }
+};
+
+// One block per SM; 64 registers let the largest block have 1,024 threads.
+template <int DIM, bool ST, int P>
+__global__ void __launch_bounds__(1024, 1) k_small_step(const __grid_constant__ KConst k,
+                                                        const __grid_constant__ FluidBuf F,
+                                                        const __grid_constant__ BoundBuf B,
+                                                        const __grid_constant__ SmallArgs a) {
+    __shared__ double sh_d[kSmallSums];
+    __shared__ int sh_i[33];
+    SmallStep<DIM, ST, P> step{k, F, B, a, {a.x.bar, 0u}, sh_d, sh_i, (a.f.n + kBlock - 1) / kBlock * kBlock, 0};
+    const bool done = step.run();
+    step.leave(done);
+}
+
+template <int DIM>
+cudaError_t launch_small_dim(tsph_ctx &c, const SmallArgs &a, int threads, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(c.sms);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const bool fbm = c.p.fbm_enabled != 0;
+    if (c.st_on)
+        return fbm ? cudaLaunchKernelEx(&cfg, k_small_step<DIM, true, 2>, c.k, c.F, c.B, a)
+                   : cudaLaunchKernelEx(&cfg, k_small_step<DIM, true, 0>, c.k, c.F, c.B, a);
+    return fbm ? cudaLaunchKernelEx(&cfg, k_small_step<DIM, false, 2>, c.k, c.F, c.B, a)
+               : cudaLaunchKernelEx(&cfg, k_small_step<DIM, false, 0>, c.k, c.F, c.B, a);
+}
+
+}  // namespace tsph
