@@ -554,6 +554,31 @@ __device__ __forceinline__ void visit_hits_r1(const int *start, const float4 *po
     }
 }
 
+// Whether no particle of the grid lies in any template cell of the calling lanes'
+// codes (their common range per row, so "false" may be for another lane's sake).
+// Takes the scenes of visit_hits_r1, whose rows it may spare: one pair of cell
+// starts per row and warp.  Most fluid particles have no wall near them and most
+// of a wall no fluid; walking nine empty rows per particle cost the fluid sweep
+// 24 us of 405 at 1M particles.
+template <int DIM, bool NC>
+__device__ __forceinline__ bool rows_empty_r1(const int *start, const Geo &g, long long code64) {
+    const unsigned int lanes = __activemask();
+    const int nx = (int)g.nx, nxny = DIM == 3 ? (int)g.nxny : 0, nn = (int)g.node_num;
+    // (a code out of reach of the grid clamps to one that is, too)
+    const long long reach = nxny + nx + 1;
+    const int code = (int)(code64 < -reach ? -reach : code64 > nn + reach ? nn + reach : code64);
+    const int first = __reduce_min_sync(lanes, code), last = __reduce_max_sync(lanes, code);
+    const int *st = start + g.cbase;
+    bool any = false;
+    constexpr int rows = DIM == 3 ? 9 : 3;
+    for (int r = __popc(lanes & ((1u << (threadIdx.x & 31)) - 1u)); r < rows; r += __popc(lanes)) {
+        const int off = (r % 3 - 1) * nx + (DIM == 3 ? (r / 3 - 1) * nxny : 0);
+        const int lo = max(first + off - 1, 1), hi = min(last + off + 1, nn - 1);
+        if (lo <= hi) any |= ld_ro<NC>(st + hi + 1) != ld_ro<NC>(st + lo);
+    }
+    return !__any_sync(lanes, any);
+}
+
 // entries past the end of a position array that visit_hits_r1 may read
 constexpr int kScanPad = 4;
 

@@ -216,7 +216,8 @@ __device__ __forceinline__ double density_fluid_item(const KConst &k, const Flui
         if (R1) {
             visit_hits_r1<DIM, NC>(F.start, F.pos, g, pi, code, shift_of<M>(st.f_shift), ff);
             nfl = w.n;
-            visit_hits_r1<DIM, NC>(B.start, B.pos, g, pi, code, shift_of<M>(st.b_shift), fb);
+            if (!rows_empty_r1<DIM, NC>(B.start, g, code))
+                visit_hits_r1<DIM, NC>(B.start, B.pos, g, pi, code, shift_of<M>(st.b_shift), fb);
         } else {
             auto within = [&](const float4 *P, int j) {
                 const float4 pj = ld_ro<NC>(P + j);
@@ -350,8 +351,10 @@ __device__ __forceinline__ void density_bound_item(const KConst &k, const FluidB
                 }
             }
         };
-        if (R1) visit_hits_r1<DIM, NC>(F.start, F.pos, g, pi, code, shift_of<M>(st.f_shift), bf_pair);
-        else visit_candidates_within<DIM, 1, NC>(F.start, g, pi, code, shift_of<M>(st.f_shift), 0, bf_pair);
+        if (R1) {
+            if (!rows_empty_r1<DIM, NC>(F.start, g, code))
+                visit_hits_r1<DIM, NC>(F.start, F.pos, g, pi, code, shift_of<M>(st.f_shift), bf_pair);
+        } else visit_candidates_within<DIM, 1, NC>(F.start, g, pi, code, shift_of<M>(st.f_shift), 0, bf_pair);
     }
     const float m = B.mv[s].x;
     float alpha = 0.f / m + a2;
