@@ -19,7 +19,7 @@ constexpr int64_t kSmallWarpsPerSm = 512;
 
 bool small_step_fits(const tsph_ctx &c, const tsph_set &f, const tsph_set &b) {
     if (c.n_scenes != 1 || c.batch || !c.sms || !c.scan_r1 || c.tpp != 1 || f.n < 1) return false;
-    if (c.p.wcsph_enabled || (c.p.fbm_enabled && c.k.P != 2)) return false;
+    if (c.p.fbm_enabled && c.k.P != 2) return false;
     return (f.n + 31) / 32 + (b.n + 31) / 32 <= kSmallWarpsPerSm * c.sms;
 }
 
@@ -30,6 +30,7 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
     a.x = c.X;
     a.with_cfl = with_cfl ? 1 : 0;
     a.st_on = c.st_on;
+    a.wc = c.p.wcsph_enabled;
     if (c.rec_tape) {
         a.tape = c.rec_tape->a;
         a.record = 1;

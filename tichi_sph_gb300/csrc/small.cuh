@@ -18,6 +18,7 @@
 #include "grid.cuh"
 #include "sweeps.cuh"
 #include "tape.cuh"
+#include "wcsph.cuh"
 
 namespace tsph {
 
@@ -26,7 +27,7 @@ struct SmallArgs {
     tsph_set f, b;
     SmallScratch x;
     TapeArrays tape;
-    int record, with_cfl, st_on;
+    int record, with_cfl, st_on, wc;
 };
 
 // A poll of the barrier's counter takes about half a microsecond: the limit is
@@ -307,6 +308,18 @@ struct SmallStep {
         return true;
     }
 
+    // The weakly compressible pressure block (k_wc_pressure, k_wc_acce).
+    __device__ __forceinline__ bool weakly_compressible() {
+        const SceneConst &c = k.s0;
+        for_items(c.f_n, c.b_n, [&](int64_t s, int64_t) { if (s < c.f_n) wc_pressure_fluid_item(F, c, s); },
+                  [&](int64_t s) { if (s < c.b_n) wc_pressure_bound_item(B, a.b.pressure, s); });
+        if (!bar.sync()) return false;
+        for_items(c.f_n, 0, [&](int64_t s, int64_t) {
+            if (s < c.f_n) wc_acce_item<DIM, false, false>(k, F, B, 0, c, st(), cur, s);
+        }, [](int64_t) {});
+        return bar.sync();
+    }
+
     // The volume-fraction update (k_fbm_drift, k_fbm_begin, k_fbm_pass).
     __device__ __forceinline__ bool mixture() {
         const SceneConst &c = k.s0;
@@ -398,6 +411,7 @@ struct SmallStep {
         if (!bar.sync()) return false;
         cur = 1 - cur;
         if (!solve(kSolveDens, false)) return false;
+        if (a.wc && !weakly_compressible()) return false;
         if (P && !mixture()) return false;
         double *en = a.x.sums;  // the solves' sums are done with
         for_items(ns, a.b.n,

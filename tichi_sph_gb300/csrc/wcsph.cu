@@ -15,17 +15,11 @@
 #include <cuda_runtime.h>
 
 #include "ctx.h"
+#include "wcsph.cuh"
 
 namespace tsph {
 
 namespace {
-
-// (rho / rho0)^7 by squaring, as an integer power.
-__device__ __forceinline__ float pow7(float r) {
-    const float r2 = r * r;
-    const float r4 = r2 * r2;
-    return r4 * r2 * r;
-}
 
 template <bool M>
 __global__ void __launch_bounds__(kBlock) k_wc_pressure(KConst k, FluidBuf F, BoundBuf B, const float *bpress) {
@@ -33,20 +27,11 @@ __global__ void __launch_bounds__(kBlock) k_wc_pressure(KConst k, FluidBuf F, Bo
     const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
     if (s < F.cap) {
         const SceneConst &c = scene<M>(k, f_block_scene<M>(k, s - (s % kChunk)));
-        if (s - c.f_slot < c.f_n) {
-            const float rho = F.dens[s].y, rho0 = F.rho0[s];
-            float p = (rho0 * (float)(c.cs * c.cs)) / (float)c.wc_gamma * (pow7(rho / rho0) - 1.f);
-            if (p < 0.f) p = 0.f;
-            F.wcp[s] = make_float2(p, p / (rho * rho));
-        }
+        if (s - c.f_slot < c.f_n) wc_pressure_fluid_item(F, c, s);
     }
     if (s < B.cap) {
         const SceneConst &c = scene<M>(k, b_block_scene<M>(k, s - (s % kChunk)));
-        if (s - c.b_slot < c.b_n) {
-            const float p = bpress ? bpress[B.perm[s]] : 0.f;
-            const float rho = B.dens[s].y;
-            B.wcp2[s] = p / (rho * rho);
-        }
+        if (s - c.b_slot < c.b_n) wc_pressure_bound_item(B, bpress, s);
     }
 }
 
@@ -56,76 +41,68 @@ __global__ void __launch_bounds__(kBlock) k_wc_acce(KConst k, FluidBuf F, BoundB
     const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
     const int sc = f_block_scene<M>(k, blockIdx.x * (int64_t)kBlock);
     const SceneConst &c = scene<M>(k, sc);
-    if (s - c.f_slot >= c.f_n) return;
-    const SceneStep &st = k.ss[sc];
-    const float h2 = c.h2, inv_h = c.inv_h, sig_h = c.sig_h;
-    const float4 pi = F.pos[s];
-    const float pri = F.wcp[s].y;
-    float ax = 0.f, ay = 0.f, az = 0.f;
-    auto term = [&](float4 pj, float prj, float mj) {
-        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 < h2 && r2 > 0.f) {
-            float r;
-            const float ri = pair_rinv(r2, r);  // rsqrt pair geometry, as the other sweeps
-            const float f = -(pri + prj) * mj * (kwg(r * inv_h) * sig_h) * ri;
-            ax += f * dx;
-            ay += f * dy;
-            az += f * dz;
-        }
-    };
-    for_each_neighbor_tpp<DIM, true, 1, M>(c, st, k.R, F, B, s, 0, pi,
-        [&](int j, auto) { term(F.pos[j], F.wcp[j].y, F.mv[j].x); },
-        [&](int j, auto) { term(B.pos[j], B.wcp2[j], B.mv[j].x); });
-    const float4 a0 = F.acc[s];
-    const float4 a = make_float4(a0.x + ax, a0.y + ay, a0.z + az, 0.f);
-    F.acc[s] = a;
-    const float dt = k.sp[sc].dt;
-    const float4 v = F.vel[s];
-    F.vadv[st.cur * F.cap + s] = make_float4(v.x + a.x * dt, v.y + a.y * dt, v.z + a.z * dt, 0.f);
+    if (s - c.f_slot < c.f_n) wc_acce_item<DIM, M, true>(k, F, B, sc, c, k.ss[sc], k.ss[sc].cur, s);
 }
 
-// map_velocity over the nodes of a regular grid (C order), one thread per node.
+// What the velocity map reads of a particle, in sorted order: the caller's
+// current position with X / psi, and velocity.  A velocity that is not finite
+// makes X / psi NaN, so that the map need not read velocities beyond h, where
+// W = 0, to give the NaN that 0 times it is.
 template <int DIM>
+__device__ __forceinline__ void map_record(const KConst &k, const tsph_set &U, int64_t pid, float4 &p, float4 &v) {
+    const bool vf = k.vfsph != 0;
+    const float X = vf ? U.rest_volume[pid] : U.mass[pid];
+    const float psi = vf ? U.sph_compression[pid] : U.sph_density[pid];
+    const float *x = U.pos + pid * DIM, *u = U.vel + pid * DIM;
+    v = make_float4(u[0], u[1], DIM == 3 ? u[2] : 0.f, 0.f);
+    const bool fin = isfinite(v.x) && isfinite(v.y) && isfinite(v.z);
+    p = make_float4(x[0], x[1], DIM == 3 ? x[2] : 0.f, fin ? X / psi : __int_as_float(0x7fffffff));
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kBlock) k_map_pack(KConst k, FluidBuf F, tsph_set U) {
+    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    if (s < k.s0.f_n) map_record<DIM>(k, U, F.perm[s], F.pk[s], F.facc[s]);
+}
+
+// map_velocity over the nodes of a regular grid, one thread per node, x fastest
+// (the nodes of a warp then lie along a row of cells and share candidates; out
+// is in C order).  PACKED: the particles' records are in F.pk and F.facc, which
+// hold nothing between steps, one 16-byte load per candidate and the velocity
+// only within h; otherwise (a step composed call by call is under way) they are
+// made per candidate from the caller's arrays.  Bound by the candidate loads:
+// 190k nodes over 97k particles took 167 us with nine scattered loads per
+// candidate and z fastest, and takes 57 us in both launches.
+template <int DIM, bool PACKED>
 __global__ void __launch_bounds__(kBlock) k_map_velocity(KConst k, FluidBuf F, tsph_set U, float lb0, float lb1,
                                                          float lb2, float dist, int n0, int n1, int n2,
                                                          float *out) {
-    pdl_entry();
-    const int64_t I = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    const int64_t t = blockIdx.x * (int64_t)kBlock + threadIdx.x;
     const int64_t total = (int64_t)n0 * n1 * (DIM == 3 ? n2 : 1);
-    if (I >= total) return;
+    if (t >= total) return;
     const SceneConst &c = k.s0;
-    int idx[3];
-    int64_t r = I;
-    if (DIM == 3) {
-        idx[2] = (int)(r % n2);
-        r /= n2;
-    } else {
-        idx[2] = 0;
-    }
-    idx[1] = (int)(r % n1);
-    idx[0] = (int)(r / n1);
-    const float4 gp = make_float4(lb0 + (float)idx[0] * dist, lb1 + (float)idx[1] * dist,
-                                  DIM == 3 ? lb2 + (float)idx[2] * dist : 0.f, 0.f);
+    const int i0 = (int)(t % n0), i1 = (int)(t / n0 % n1), i2 = DIM == 3 ? (int)(t / n0 / n1) : 0;
+    const int64_t I = ((int64_t)i0 * n1 + i1) * (DIM == 3 ? n2 : 1) + i2;
+    const float4 gp = make_float4(lb0 + (float)i0 * dist, lb1 + (float)i1 * dist,
+                                  DIM == 3 ? lb2 + (float)i2 * dist : 0.f, 0.f);
     Geo g;
     g.load(c, k.R);
     bool ok;
     const long long code = cell_code<DIM>(gp, g, ok);
-    const bool vf = k.vfsph != 0;
     float vx = 0.f, vy = 0.f, vz = 0.f;
     if (ok) {
         visit_candidates<DIM>(F.start, g, code, 0, 0, [&](int j) {
-            const int64_t pid = F.perm[j];
-            const float *p = U.pos + pid * DIM;
-            const float dx = gp.x - p[0], dy = gp.y - p[1], dz = DIM == 3 ? gp.z - p[2] : 0.f;
-            const float w = kw(sqrtf(dx * dx + dy * dy + dz * dz) * g.inv_h) * g.sig;
-            const float X = vf ? U.rest_volume[pid] : U.mass[pid];
-            const float psi = vf ? U.sph_compression[pid] : U.sph_density[pid];
-            const float f = X / psi * w;
-            const float *v = U.vel + pid * DIM;
-            vx += f * v[0];
-            vy += f * v[1];
-            if (DIM == 3) vz += f * v[2];
+            float4 p, v;
+            if (PACKED) p = F.pk[j];
+            else map_record<DIM>(k, U, F.perm[j], p, v);
+            const float dx = gp.x - p.x, dy = gp.y - p.y, dz = DIM == 3 ? gp.z - p.z : 0.f;
+            const float q = sqrtf(dx * dx + dy * dy + dz * dz) * g.inv_h;
+            if (q >= 1.f && isfinite(p.w)) return;  // W = 0
+            const float f = p.w * (kw(q) * g.sig);
+            if (PACKED) v = F.facc[j];
+            vx += f * v.x;
+            vy += f * v.y;
+            if (DIM == 3) vz += f * v.z;
         });
     }
     out[I * DIM] = vx;
@@ -150,6 +127,21 @@ void launch_wc(tsph_ctx &c, const tsph_set &b, cudaStream_t st) {
 }
 
 void set_last_error_text(const char *msg);
+
+template <int DIM>
+static void launch_map(tsph_ctx &c, const tsph_set &f, const float *lb, float dist, const int32_t *shape,
+                       int64_t total, float *out, cudaStream_t st) {
+    const int nb = blocks_for(total), n2 = DIM == 3 ? shape[2] : 1;
+    const float lb2 = DIM == 3 ? lb[2] : 0.f;
+    if (c.kl_phase == 0 && c.k.s0.f_n > 0) {
+        k_map_pack<DIM><<<blocks_for(c.k.s0.f_n), kBlock, 0, st>>>(c.k, c.F, f);
+        k_map_velocity<DIM, true>
+            <<<nb, kBlock, 0, st>>>(c.k, c.F, f, lb[0], lb[1], lb2, dist, shape[0], shape[1], n2, out);
+    } else {
+        k_map_velocity<DIM, false>
+            <<<nb, kBlock, 0, st>>>(c.k, c.F, f, lb[0], lb[1], lb2, dist, shape[0], shape[1], n2, out);
+    }
+}
 
 }  // namespace tsph
 
@@ -183,13 +175,8 @@ extern "C" int tsph_map_velocity(tsph_ctx *c, const tsph_set *f, const float *lb
         return TSPH_ERR_INVALID;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    const int nb = blocks_for(total);
-    if (dim == 3)
-        k_map_velocity<3><<<nb, kBlock, 0, st>>>(c->k, c->F, *f, lb[0], lb[1], lb[2], dist, shape[0], shape[1],
-                                                 shape[2], grid_vel);
-    else
-        k_map_velocity<2><<<nb, kBlock, 0, st>>>(c->k, c->F, *f, lb[0], lb[1], 0.f, dist, shape[0], shape[1], 1,
-                                                 grid_vel);
+    if (dim == 3) launch_map<3>(*c, *f, lb, dist, shape, total, grid_vel, st);
+    else launch_map<2>(*c, *f, lb, dist, shape, total, grid_vel, st);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_last_error_text(cudaGetErrorString(e));
