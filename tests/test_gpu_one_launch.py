@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 import torch
 
-from tests.test_gpu_grid_edges import _cloud, _need_cuda, _scene
+from tests.test_gpu_grid_edges import H, _cloud, _need_cuda, _scene
 
 pytestmark = pytest.mark.gpu
 
@@ -23,10 +23,15 @@ SCALARS = ("dt", "time_count", "compression", "kinetic_energy", "potential_energ
            "total_incom_iter", "total_fbm_passes", "max_dens_compression")
 
 
-def _solver(dim, n, nb, two, use_graph):
+def _solver(dim, n, nb, two, use_graph, gamma=0.0, inside=False):
     from tichi_sph_gb300 import Fluid, Solver, sph_config
     cfg_d, scen, span = _scene(dim, 6)
     scen["sim_env"]["gravity"] = [0.0, -9.81, 0.0][:dim]
+    if gamma:
+        cfg_d["solver_surface_tension_gamma"] = gamma
+    if inside:  # room for the lists: about 3 (2D) or 4 (3D) particles a cell
+        span = [3 * H + H * (n / (3 if dim == 2 else 4)) ** (1.0 / dim)] * dim
+        scen["sim_env"]["sim_space_rt"] = span
     if two:
         cfg_d.update(solver_type="VFSPH", solver_surface_tension_gamma=0.07, solver_fbm_convection_term=50.0)
         scen["sim_env"].update(phase_num=2, phase_rest_density=[1000, 500],
@@ -37,7 +42,11 @@ def _solver(dim, n, nb, two, use_graph):
     for uid, m in enumerate((n, nb)):
         o = Fluid(m + 300, cfg, uid, device="cuda")
         o.part_num[None] = m
-        o.pos[:m] = torch.as_tensor(_cloud(rng, m, dim, span), device="cuda")
+        pos = _cloud(rng, m, dim, span)
+        if inside:  # off cell 0 too, which is no valid cell
+            pos = np.clip(pos, 0.25 * H, np.asarray(span, np.float32) - 0.25 * H) + np.float32(0.0)
+            pos[:, 0] = np.maximum(pos[:, 0], np.float32(1.25 * H))
+        o.pos[:m] = torch.as_tensor(pos, device="cuda")
         if uid == 0:
             o.vel[:m] = torch.as_tensor(rng.normal(0, 0.3, (m, dim)).astype(np.float32), device="cuda")
         vf = rng.uniform(0, 1, m).astype(np.float32) if two else np.ones(m, np.float32)
@@ -76,19 +85,28 @@ def test_one_launch_equals_separate_kernels(dim, n, nb, two):
     b.close()
 
 
-def test_recorded_substep_equals_plain_one():
+@pytest.mark.parametrize("dim,n,nb,gamma", [(2, 1, 0, 0.0), (2, 700, 90, 0.0), (3, 33, 5, 0.0), (3, 900, 300, 0.07),
+                                            (3, 25000, 400, 0.0), (3, 45000, 0, 0.0)])
+def test_recorded_substep_and_its_reverse(dim, n, nb, gamma):
+    """Recorded in one launch, reversed in one (with eight, four or one lanes per
+    particle as the size has it), against separate kernels.  The forward is
+    bitwise the same; the reverse adds a particle's up to 64 pair terms in
+    another order, within 64 x 2^-24 = 4e-6 of the terms' size a sweep: 1e-4 of
+    the largest gradient over the seven or more sweeps."""
     _need_cuda()
     import ctypes as C
 
     from tichi_sph_gb300 import _native
     outs = []
     for use_graph in (True, False):
-        s = _solver(3, 900, 300, False, use_graph)
+        s = _solver(dim, n, nb, False, use_graph, gamma=gamma, inside=True)
         tape = C.c_void_p()
-        _native.check(s._lib.tsph_tape_create(s.ctx, 2, 100, C.byref(tape)), "tape")
+        _native.check(s._lib.tsph_tape_create(s.ctx, 2, 110, C.byref(tape)), "tape")
         f, b = s._sets()
         gmu = torch.zeros(1, dtype=torch.float64, device="cuda")
-        gx, gv = torch.ones(900, 3, device="cuda"), torch.ones(900, 3, device="cuda")
+        gen = torch.Generator("cuda").manual_seed(1)
+        gx = torch.randn(n, dim, generator=gen, device="cuda")
+        gv = torch.randn(n, dim, generator=gen, device="cuda") * 1e-3
         for slot in range(2):
             _native.check(s._lib.tsph_substep_record(s.ctx, f, b, tape, slot, None), "record")
         ptr = lambda t, c=C.c_float: C.cast(t.data_ptr(), C.POINTER(c))  # noqa: E731
@@ -96,9 +114,11 @@ def test_recorded_substep_equals_plain_one():
         rc = s._lib.tsph_substep_adjoint(s.ctx, tape, 0, ptr(gx), ptr(gv), ptr(gx), ptr(gv), ptr(gmu, C.c_double),
                                          None)
         torch.cuda.synchronize()
-        outs.append((rc, gx, gv, gmu, s.fluid.pos.clone()))
+        outs.append((rc, s.fluid.pos.clone(), gx, gv, gmu))
         s._lib.tsph_tape_destroy(tape)
         s.close()
-    assert outs[0][0] == outs[1][0]
-    for x, y in zip(outs[0][1:], outs[1][1:]):
-        assert torch.equal(x, y)
+    (rc0, p0, *g0), (rc1, p1, *g1) = outs
+    assert rc0 == rc1 == 0, _native.lib().tsph_last_error()
+    assert torch.equal(p0, p1)
+    for x, y in zip(g0, g1):
+        assert float((x - y).abs().max()) <= 1e-4 * max(float(y.abs().max()), 1e-30)

@@ -32,11 +32,13 @@
 // checked there against torch.autograd and central finite differences.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <new>
 
 #include "ctx.h"
+#include "coop.cuh"
 #include "tape.cuh"
 
 namespace tsph {
@@ -134,50 +136,75 @@ struct Pair {
     __device__ __forceinline__ float dot(float ax, float ay, float az) const { return x * ax + y * ay + z * az; }
 };
 
-template <class FF, class FB>
-__device__ __forceinline__ void for_pairs(const SlotView &v, int64_t s, FF &&ff, FB &&fb) {
-    const unsigned int pc = v.cnt[s];
+// The recorded pairs of the particle at slot s, or of none for s beyond the last;
+// its TPP lanes (ln) share them, a block of four entries each in turn.
+template <int TPP, class FF, class FB>
+__device__ __forceinline__ void for_pairs(const SlotView &v, const Lanes<TPP> &ln, int64_t s, FF &&ff, FB &&fb) {
+    const unsigned int pc = s < v.n ? v.cnt[s] : 0u;
     const int nfl = (int)(pc & 0xffffu), nbo = (int)(pc >> 16);
-    walk_blocks<1>(v.nbr, s, v.cap, 0, nfl, nfl + nbo, ff, fb);
+    walk_blocks<TPP>(v.nbr, s, v.cap, ln.q, nfl, nfl + nbo, ff, fb);
+}
+
+// Working arrays of the reverse pass, in the slot's sorted order.
+struct Lam {
+    float4 *u, *u2;   // adjoint of the velocity (two buffers: the viscosity sweep); w: rest density
+    float4 *x;        // of the position
+    float4 *beta;     // lam_u / (dt m); w: kappa of the iteration to reverse next
+    float4 *us;       // the iterate u^k; w: lam_s
+    float4 *a1;       // of alpha's two sums
+    float4 *n;        // of the surface normals
+    float *psi, *alpha;
+};
+
+// Kappa of iteration `it` of a solve (it >= 0).
+__device__ __forceinline__ const float *kappa_of(const SlotView &v, int kind, int it) {
+    return v.kap + ((int64_t)kind * v.max_iters + it) * v.cap;
+}
+
+// lam_u of a particle as the next kappa sweep gathers it, with its kappa (it < 0:
+// no sweep follows).
+__device__ __forceinline__ void put_beta(const SlotView &v, const Lam &l, int kind, int it, float m, float4 lu,
+                                         int64_t s) {
+    if (it < 0) return;
+    const float inv = 1.f / (v.dt * m);
+    l.beta[s] = make_float4(lu.x * inv, lu.y * inv, lu.z * inv, kappa_of(v, kind, it)[s]);
 }
 
 template <int DIM>
-__global__ void __launch_bounds__(kBlock) k_adj_in(SlotView v, const float *__restrict__ gx, const float *__restrict__ gv,
-                                                   float4 *lx, float4 *lu, float *lpsi, float *lalpha) {
-    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (s >= v.n) return;
+__device__ __forceinline__ void adj_in_item(const SlotView &v, const Lam &l, const float *gx, const float *gv, int kp,
+                                            int64_t s) {
     const int64_t b = (int64_t)v.perm[s] * DIM;
     const float x0 = gx[b], x1 = gx[b + 1], x2 = DIM == 3 ? gx[b + 2] : 0.f;
     const float v0 = gv[b], v1 = gv[b + 1], v2 = DIM == 3 ? gv[b + 2] : 0.f;
-    lx[s] = make_float4(x0, x1, x2, 0.f);
+    l.x[s] = make_float4(x0, x1, x2, 0.f);
     // x' = x + v' dt: the step's velocity output also moved the positions
-    lu[s] = make_float4(v0 + v.dt * x0, v1 + v.dt * x1, v2 + v.dt * x2, 0.f);
-    lpsi[s] = 0.f;
-    lalpha[s] = 0.f;
+    const float4 lu = make_float4(v0 + v.dt * x0, v1 + v.dt * x1, v2 + v.dt * x2, v.rho0[s]);
+    l.u[s] = lu;
+    put_beta(v, l, kSolveDens, kp - 1, v.pos[s].w, lu, s);
+    l.psi[s] = 0.f;
+    l.alpha[s] = 0.f;
 }
 
-__global__ void __launch_bounds__(kBlock) k_adj_kappa(SlotView v, int kind, int it, const float4 *__restrict__ lu,
-                                                      float *ls, float4 *lx, float *lpsi, float *lalpha) {
-    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (s >= v.n) return;
-    const float *kap = v.kap + ((int64_t)kind * v.max_iters + it) * v.cap;
-    const float4 pi = v.pos[s];
+// Reverse of the velocity update of iteration `it`.
+template <int TPP>
+__device__ __forceinline__ void adj_kappa_item(const SlotView &v, const Lam &l, const Lanes<TPP> &ln, int kind,
+                                               int it, int64_t s) {
+    const int64_t i = s < v.n ? s : 0;  // (lanes past the end compute and drop)
+    const float4 pi = v.pos[i];
     const float mi = pi.w;
-    const float ki = kap[s];
-    const float4 lui = lu[s];
-    const float inv = 1.f / (v.dt * mi);
-    const float bx = lui.x * inv, by = lui.y * inv, bz = lui.z * inv;
+    const float4 bi = l.beta[i];
+    const float ki = bi.w;
+    const float bx = bi.x, by = bi.y, bz = bi.z;
     float lk = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
-    for_pairs(v, s,
+    for_pairs(v, ln, s,
         [&](int j) {
             const float4 pj = v.pos[j];
             const Pair P(v, pi, pj);
-            const float4 luj = lu[j];
-            const float invj = 1.f / (v.dt * pj.w);
-            const float dx = bx - luj.x * invj, dy = by - luj.y * invj, dz = bz - luj.z * invj;
+            const float4 bj = l.beta[j];
+            const float dx = bx - bj.x, dy = by - bj.y, dz = bz - bj.z;
             const float rd = P.dot(dx, dy, dz);
             lk -= pj.w * P.g * rd;
-            const float cK = ki * pj.w + kap[j] * mi;
+            const float cK = ki * pj.w + bj.w * mi;
             gx -= cK * (P.g * dx + P.G2 * rd * P.x);
             gy -= cK * (P.g * dy + P.G2 * rd * P.y);
             gz -= cK * (P.g * dz + P.G2 * rd * P.z);
@@ -192,24 +219,30 @@ __global__ void __launch_bounds__(kBlock) k_adj_kappa(SlotView v, int kind, int 
             gy -= cK * (P.g * by + P.G2 * rd * P.y);
             gz -= cK * (P.g * bz + P.G2 * rd * P.z);
         });
+    lk = ln.sum(lk);
+    gx = ln.sum(gx);
+    gy = ln.sum(gy);
+    gz = ln.sum(gz);
+    if (s >= v.n || ln.q != 0) return;
     const float alpha = v.mpsi[s].w;
     const float lsi = ki > 0.f ? lk / alpha : 0.f;
-    lalpha[s] -= lk * ki / alpha;
-    lpsi[s] += lsi;
-    ls[s] = lsi;
-    const float4 o = lx[s];
-    lx[s] = make_float4(o.x + gx, o.y + gy, o.z + gz, 0.f);
+    l.alpha[s] -= lk * ki / alpha;
+    l.psi[s] += lsi;
+    const float4 u = v.u[((int64_t)kind * v.max_iters + it) * v.cap + s];
+    l.us[s] = make_float4(u.x, u.y, u.z, lsi);
+    const float4 o = l.x[s];
+    l.x[s] = make_float4(o.x + gx, o.y + gy, o.z + gz, 0.f);
 }
 
-__global__ void __launch_bounds__(kBlock) k_adj_vel(SlotView v, int kind, int it, const float *__restrict__ ls,
-                                                    float4 *lu, float4 *lx) {
-    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (s >= v.n) return;
-    const float4 *u = v.u + ((int64_t)kind * v.max_iters + it) * v.cap;
-    const float4 pi = v.pos[s];
+// Reverse of the divergence of iteration `it`.
+template <int TPP>
+__device__ __forceinline__ void adj_vel_item(const SlotView &v, const Lam &l, const Lanes<TPP> &ln, int kind, int it,
+                                             int64_t s) {
+    const int64_t i = s < v.n ? s : 0;  // (lanes past the end compute and drop)
+    const float4 pi = v.pos[i];
     const float mi = pi.w;
-    const float4 ui = u[s];
-    const float lsi = ls[s];
+    const float4 ui = l.us[i];
+    const float lsi = ui.w;
     float ax = 0.f, ay = 0.f, az = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
     auto term = [&](const Pair &P, float cS, float4 uj) {
         ax += cS * P.g * P.x;
@@ -221,88 +254,96 @@ __global__ void __launch_bounds__(kBlock) k_adj_vel(SlotView v, int kind, int it
         gy += cS * (P.g * dy + P.G2 * rd * P.y);
         gz += cS * (P.g * dz + P.G2 * rd * P.z);
     };
-    for_pairs(v, s,
+    for_pairs(v, ln, s,
         [&](int j) {
             const float4 pj = v.pos[j];
-            term(Pair(v, pi, pj), lsi * pj.w + ls[j] * mi, u[j]);
+            const float4 uj = l.us[j];
+            term(Pair(v, pi, pj), lsi * pj.w + uj.w * mi, uj);
         },
         [&](int b) {
             const float4 pb = v.bpos[b];
             term(Pair(v, pi, pb), lsi * pb.w, v.bvel[b]);
         });
-    const float4 l = lu[s];
-    lu[s] = make_float4(l.x + v.dt * ax, l.y + v.dt * ay, l.z + v.dt * az, 0.f);
-    const float4 o = lx[s];
-    lx[s] = make_float4(o.x + v.dt * gx, o.y + v.dt * gy, o.z + v.dt * gz, 0.f);
+    ax = ln.sum(ax);
+    ay = ln.sum(ay);
+    az = ln.sum(az);
+    gx = ln.sum(gx);
+    gy = ln.sum(gy);
+    gz = ln.sum(gz);
+    if (s >= v.n || ln.q != 0) return;
+    const float4 lu = l.u[s];
+    const float4 nu = make_float4(lu.x + v.dt * ax, lu.y + v.dt * ay, lu.z + v.dt * az, lu.w);
+    l.u[s] = nu;
+    put_beta(v, l, kind, it - 1, mi, nu, s);
+    const float4 o = l.x[s];
+    l.x[s] = make_float4(o.x + v.dt * gx, o.y + v.dt * gy, o.z + v.dt * gz, 0.f);
 }
 
 // Reverse of u0 = v + dt (g + mu V): lam_v = lam_u0 + (dV/dv)^T lam_a with
 // lam_a = dt lam_u0; also lam_x, lam_psi and dL/dmu = sum_i lam_a_i . V_i.
-template <int DIM>
-__global__ void __launch_bounds__(kBlock) k_adj_visc(SlotView v, const float4 *__restrict__ lu, float4 *lu2,
-                                                     float4 *lx, float *lpsi, double *partials, unsigned int *ticket,
-                                                     double *gmu) {
-    __shared__ double sh[kBlock / 32];
-    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    double contrib = 0.0;
-    if (s < v.n) {
-        const float lap = 2.f * (2.f + DIM);
-        const float4 pi = v.pos[s];
-        const float mi = pi.w;
-        const float4 lui = lu[s];
-        const float lax = v.dt * lui.x, lay = v.dt * lui.y, laz = v.dt * lui.z;
-        const float psii = v.mpsi[s].y, r0i = v.rho0[s];
-        const float4 vi = v.vmid[s];
-        float avx = 0.f, avy = 0.f, avz = 0.f, gx = 0.f, gy = 0.f, gz = 0.f, lp = 0.f;
-        float Vx = 0.f, Vy = 0.f, Vz = 0.f;
-        for_pairs(v, s,
-            [&](int j) {
-                const float4 pj = v.pos[j];
-                const Pair P(v, pi, pj);
-                const float den = v.eps + P.r2;
-                const float phi = P.g / den;
-                const float dphi = P.G2 / den - 2.f * P.g / (den * den);
-                const float4 vj = v.vmid[j];
-                const float psij = v.mpsi[j].y, r0j = v.rho0[j];
-                const float4 luj = lu[j];
-                const float ljx = v.dt * luj.x, ljy = v.dt * luj.y, ljz = v.dt * luj.z;
-                const float wx = vi.x - vj.x, wy = vi.y - vj.y, wz = vi.z - vj.z;
-                const float vr = P.dot(wx, wy, wz);
-                const float ci = v.mu * lap * pj.w / (r0i * psij);
-                const float cj = v.mu * lap * mi / (r0j * psii);
-                const float rli = P.dot(lax, lay, laz), rlj = P.dot(ljx, ljy, ljz);
-                const float fv = (ci * rli - cj * rlj) * phi;
-                avx += fv * P.x;
-                avy += fv * P.y;
-                avz += fv * P.z;
-                lp += cj * phi * vr * rlj / psii;
-                const float ti = vr * rli * dphi, tj = vr * rlj * dphi;
-                gx += ci * (phi * (rli * wx + vr * lax) + ti * P.x) - cj * (phi * (rlj * wx + vr * ljx) + tj * P.x);
-                gy += ci * (phi * (rli * wy + vr * lay) + ti * P.y) - cj * (phi * (rlj * wy + vr * ljy) + tj * P.y);
-                gz += ci * (phi * (rli * wz + vr * laz) + ti * P.z) - cj * (phi * (rlj * wz + vr * ljz) + tj * P.z);
-                const float fV = lap * (pj.w / psij) * phi * vr;
-                Vx += fV * P.x;
-                Vy += fV * P.y;
-                Vz += fV * P.z;
-            },
-            [&](int) {});
-        lu2[s] = make_float4(lui.x + avx, lui.y + avy, lui.z + avz, 0.f);
-        const float4 o = lx[s];
-        lx[s] = make_float4(o.x + gx, o.y + gy, o.z + gz, 0.f);
-        lpsi[s] += lp;
-        contrib = (double)((lax * Vx + lay * Vy + laz * Vz) / r0i);
-    }
-    const double bs = block_sum<kBlock>(contrib, sh);
-    if (threadIdx.x == 0) partials[blockIdx.x] = bs;
-    if (last_block_done(ticket, gridDim.x)) {
-        double a = 0.0;
-        for (int i = threadIdx.x; i < (int)gridDim.x; i += kBlock) a += __ldcg(partials + i);
-        a = block_sum<kBlock>(a, sh);
-        if (threadIdx.x == 0) {
-            *gmu += a;
-            *ticket = 0;
-        }
-    }
+// Returns the particle's share of dL/dmu.
+template <int DIM, int TPP>
+__device__ __forceinline__ double adj_visc_item(const SlotView &v, const Lam &l, const Lanes<TPP> &ln, int kd,
+                                                int64_t s) {
+    const int64_t i = s < v.n ? s : 0;  // (lanes past the end compute and drop)
+    const float lap = 2.f * (2.f + DIM);
+    const float4 pi = v.pos[i];
+    const float mi = pi.w;
+    const float4 lui = l.u[i];
+    const float lax = v.dt * lui.x, lay = v.dt * lui.y, laz = v.dt * lui.z;
+    const float4 vi = v.vmid[i];  // w: psi
+    const float psii = vi.w, r0i = lui.w;
+    float avx = 0.f, avy = 0.f, avz = 0.f, gx = 0.f, gy = 0.f, gz = 0.f, lp = 0.f;
+    float Vx = 0.f, Vy = 0.f, Vz = 0.f;
+    for_pairs(v, ln, s,
+        [&](int j) {
+            const float4 pj = v.pos[j];
+            const Pair P(v, pi, pj);
+            const float den = v.eps + P.r2;
+            const float phi = P.g / den;
+            const float dphi = P.G2 / den - 2.f * P.g / (den * den);
+            const float4 vj = v.vmid[j];
+            const float4 luj = l.u[j];
+            const float psij = vj.w, r0j = luj.w;
+            const float ljx = v.dt * luj.x, ljy = v.dt * luj.y, ljz = v.dt * luj.z;
+            const float wx = vi.x - vj.x, wy = vi.y - vj.y, wz = vi.z - vj.z;
+            const float vr = P.dot(wx, wy, wz);
+            const float ci = v.mu * lap * pj.w / (r0i * psij);
+            const float cj = v.mu * lap * mi / (r0j * psii);
+            const float rli = P.dot(lax, lay, laz), rlj = P.dot(ljx, ljy, ljz);
+            const float fv = (ci * rli - cj * rlj) * phi;
+            avx += fv * P.x;
+            avy += fv * P.y;
+            avz += fv * P.z;
+            lp += cj * phi * vr * rlj / psii;
+            const float ti = vr * rli * dphi, tj = vr * rlj * dphi;
+            gx += ci * (phi * (rli * wx + vr * lax) + ti * P.x) - cj * (phi * (rlj * wx + vr * ljx) + tj * P.x);
+            gy += ci * (phi * (rli * wy + vr * lay) + ti * P.y) - cj * (phi * (rlj * wy + vr * ljy) + tj * P.y);
+            gz += ci * (phi * (rli * wz + vr * laz) + ti * P.z) - cj * (phi * (rlj * wz + vr * ljz) + tj * P.z);
+            const float fV = lap * (pj.w / psij) * phi * vr;
+            Vx += fV * P.x;
+            Vy += fV * P.y;
+            Vz += fV * P.z;
+        },
+        [&](int) {});
+    avx = ln.sum(avx);
+    avy = ln.sum(avy);
+    avz = ln.sum(avz);
+    gx = ln.sum(gx);
+    gy = ln.sum(gy);
+    gz = ln.sum(gz);
+    lp = ln.sum(lp);
+    Vx = ln.sum(Vx);
+    Vy = ln.sum(Vy);
+    Vz = ln.sum(Vz);
+    if (s >= v.n || ln.q != 0) return 0.0;
+    const float4 nu = make_float4(lui.x + avx, lui.y + avy, lui.z + avz, lui.w);
+    l.u2[s] = nu;
+    put_beta(v, l, kSolveDiv, kd - 1, mi, nu, s);
+    const float4 o = l.x[s];
+    l.x[s] = make_float4(o.x + gx, o.y + gy, o.z + gz, 0.f);
+    l.psi[s] += lp;
+    return (double)((lax * Vx + lay * Vy + laz * Vz) / r0i);
 }
 
 // Surface tension, first reverse sweep, over the template candidates the
@@ -313,23 +354,21 @@ __global__ void __launch_bounds__(kBlock) k_adj_visc(SlotView v, const float4 *_
 //   lam_x_i   += sum_j (k_ij D_C(lam_a_i) - k_ji D_C(lam_a_j)), k_ij = -gamma m_j c_ij,
 // D_C(w) = (C/r) w + ((C' - C/r) / r^2)(r_ij.w) r_ij.  Pairs count only where
 // both particles' phase-0 volume fraction exceeds 0.99, as in the forward.
-template <int DIM>
-__global__ void __launch_bounds__(kBlock) k_adj_st1(SlotView v, const float4 *__restrict__ lu, float4 *ln,
-                                                    float4 *lx, float *lpsi) {
-    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (s >= v.n) return;
-    const float4 pi = v.pos[s];
-    const float4 mpi = v.mpsi[s];
+template <int DIM, int TPP>
+__device__ __forceinline__ void adj_st1_item(const SlotView &v, const Lam &l, const Lanes<TPP> &ln, int64_t s) {
+    const int64_t i = s < v.n ? s : 0;  // (lanes past the end compute and drop)
+    const float4 pi = v.pos[i];
+    const float4 mpi = v.mpsi[i];
     const float mi = mpi.x, psii = mpi.y, r0i = mpi.z;
-    const float4 ni = v.nrm[s];
-    const float4 lui = lu[s];
+    const float4 ni = v.nrm[i];
+    const float4 lui = l.u[i];
     const float lax = v.dt * lui.x, lay = v.dt * lui.y, laz = v.dt * lui.z;
     const float gam = v.gamma;
     float nx = 0.f, ny = 0.f, nz = 0.f, lp = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
     bool ok;
     const long long code = cell_code<DIM>(pi, v.geo, ok);
-    if (ok && v.vf0[s] > 0.99f) {
-        visit_candidates<DIM>(v.start, v.geo, code, 0, 0, [&](int j) {
+    if (s < v.n && ok && v.vf0[i] > 0.99f) {
+        visit_candidates<DIM, TPP>(v.start, v.geo, code, 0, ln.q, [&](int j) {
             const float4 pj = v.pos[j];
             const float x = pi.x - pj.x, y = pi.y - pj.y, z = pi.z - pj.z;
             const float r2 = x * x + y * y + z * z;
@@ -342,7 +381,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_st1(SlotView v, const float4 *__
             const float4 mpj = v.mpsi[j];
             const float mj = mpj.x, psij = mpj.y, r0j = mpj.z;
             const float4 nj = v.nrm[j];
-            const float4 luj = lu[j];
+            const float4 luj = l.u[j];
             const float ljx = v.dt * luj.x, ljy = v.dt * luj.y, ljz = v.dt * luj.z;
             const float sum = psii + psij;
             const float cij = 2.f * r0i / sum, cji = 2.f * r0j / sum;
@@ -360,10 +399,18 @@ __global__ void __launch_bounds__(kBlock) k_adj_st1(SlotView v, const float4 *__
             gz += kij * (gC * laz + G2C * rli * z) - kji * (gC * ljz + G2C * rlj * z);
         });
     }
-    ln[s] = make_float4(nx, ny, nz, 0.f);
-    const float4 o = lx[s];
-    lx[s] = make_float4(o.x + gx, o.y + gy, o.z + gz, 0.f);
-    lpsi[s] += lp;
+    nx = ln.sum(nx);
+    ny = ln.sum(ny);
+    nz = ln.sum(nz);
+    gx = ln.sum(gx);
+    gy = ln.sum(gy);
+    gz = ln.sum(gz);
+    lp = ln.sum(lp);
+    if (s >= v.n || ln.q != 0) return;
+    l.n[s] = make_float4(nx, ny, nz, 0.f);
+    const float4 o = l.x[s];
+    l.x[s] = make_float4(o.x + gx, o.y + gy, o.z + gz, 0.f);
+    l.psi[s] += lp;
 }
 
 // Surface tension, second reverse sweep: the normals n_i = h sum_j -(X_j /
@@ -371,21 +418,20 @@ __global__ void __launch_bounds__(kBlock) k_adj_st1(SlotView v, const float4 *__
 //   lam_x_i   += h sum_j ((X_i / psi_i) D(lam_n_j) - (X_j / psi_j) D(lam_n_i)),
 //   lam_psi_i -= h (X_i / psi_i^2) sum_j g_ij r_ij.lam_n_j,
 // D(w) = g w + G2 (r_ij.w) r_ij.
-__global__ void __launch_bounds__(kBlock) k_adj_st2(SlotView v, const float4 *__restrict__ ln, float4 *lx,
-                                                    float *lpsi) {
-    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (s >= v.n) return;
-    const float4 pi = v.pos[s];
-    const float psii = v.mpsi[s].y;
+template <int TPP>
+__device__ __forceinline__ void adj_st2_item(const SlotView &v, const Lam &l, const Lanes<TPP> &ln, int64_t s) {
+    const int64_t i = s < v.n ? s : 0;  // (lanes past the end compute and drop)
+    const float4 pi = v.pos[i];
+    const float psii = v.mpsi[i].y;
     const float ai = pi.w / psii;
-    const float4 ni = ln[s];
+    const float4 ni = l.n[i];
     float gx = 0.f, gy = 0.f, gz = 0.f, lp = 0.f;
-    for_pairs(v, s,
+    for_pairs(v, ln, s,
         [&](int j) {
             const float4 pj = v.pos[j];
             const Pair P(v, pi, pj);
             const float aj = pj.w / v.mpsi[j].y;
-            const float4 nj = ln[j];
+            const float4 nj = l.n[j];
             const float rj = P.dot(nj.x, nj.y, nj.z), rI = P.dot(ni.x, ni.y, ni.z);
             gx += ai * (P.g * nj.x + P.G2 * rj * P.x) - aj * (P.g * ni.x + P.G2 * rI * P.x);
             gy += ai * (P.g * nj.y + P.G2 * rj * P.y) - aj * (P.g * ni.y + P.G2 * rI * P.y);
@@ -393,42 +439,44 @@ __global__ void __launch_bounds__(kBlock) k_adj_st2(SlotView v, const float4 *__
             lp += P.g * rj;
         },
         [&](int) {});
-    const float4 o = lx[s];
-    lx[s] = make_float4(o.x + v.h * gx, o.y + v.h * gy, o.z + v.h * gz, 0.f);
-    lpsi[s] -= v.h * ai / psii * lp;
+    gx = ln.sum(gx);
+    gy = ln.sum(gy);
+    gz = ln.sum(gz);
+    lp = ln.sum(lp);
+    if (s >= v.n || ln.q != 0) return;
+    const float4 o = l.x[s];
+    l.x[s] = make_float4(o.x + v.h * gx, o.y + v.h * gy, o.z + v.h * gz, 0.f);
+    l.psi[s] -= v.h * ai / psii * lp;
 }
 
 // lam of alpha's two sums: (lam_alpha1 xyz, lam_alpha2) where alpha was not clamped.
-__global__ void __launch_bounds__(kBlock) k_adj_alpha_prep(SlotView v, const float *__restrict__ lalpha, float4 *la1) {
-    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (s >= v.n) return;
+__device__ __forceinline__ void adj_alpha_item(const SlotView &v, const Lam &l, int64_t s) {
     const float4 a1 = v.a1[s];
     const float m = v.mpsi[s].x;
     const float raw = (a1.x * a1.x + a1.y * a1.y + a1.z * a1.z) / m + v.a2[s];
     const bool on = !(raw < 1e-4f);
-    const float la = on ? lalpha[s] : 0.f;
+    const float la = on ? l.alpha[s] : 0.f;
     const float f = la * 2.f / m;
-    la1[s] = make_float4(f * a1.x, f * a1.y, f * a1.z, la);
+    l.a1[s] = make_float4(f * a1.x, f * a1.y, f * a1.z, la);
 }
 
 // Reverse of rho_i = sum_j m_j W_ij, alpha1_i = sum_j X_j g r_ij and
 // alpha2_i = sum_j (X_j^2 / m_j) W'(r)^2 (X = m for DFSPH): position terms only.
-__global__ void __launch_bounds__(kBlock) k_adj_density(SlotView v, const float *__restrict__ lpsi,
-                                                        const float4 *__restrict__ la1, float4 *lx) {
-    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (s >= v.n) return;
-    const float4 pi = v.pos[s];
+template <int TPP>
+__device__ __forceinline__ void adj_density_item(const SlotView &v, const Lam &l, const Lanes<TPP> &ln, int64_t s) {
+    const int64_t i = s < v.n ? s : 0;  // (lanes past the end compute and drop)
+    const float4 pi = v.pos[i];
     const float mi = pi.w;
-    const float lpi = lpsi[s];
-    const float4 ai = la1[s];
+    const float lpi = l.psi[i];
+    const float4 ai = l.a1[i];
     float gx = 0.f, gy = 0.f, gz = 0.f;
-    for_pairs(v, s,
+    for_pairs(v, ln, s,
         [&](int j) {
             const float4 pj = v.pos[j];
             const Pair P(v, pi, pj);
-            const float4 aj = la1[j];
+            const float4 aj = l.a1[j];
             const float ri = P.dot(ai.x, ai.y, ai.z), rj = P.dot(aj.x, aj.y, aj.z);
-            const float cR = (lpi * pj.w + lpsi[j] * mi) * P.g + (ai.w * pj.w + aj.w * mi) * 2.f * P.g * P.W2;
+            const float cR = (lpi * pj.w + l.psi[j] * mi) * P.g + (ai.w * pj.w + aj.w * mi) * 2.f * P.g * P.W2;
             const float cA = P.G2 * (pj.w * ri - mi * rj);
             gx += cR * P.x + P.g * (pj.w * ai.x - mi * aj.x) + cA * P.x;
             gy += cR * P.y + P.g * (pj.w * ai.y - mi * aj.y) + cA * P.y;
@@ -443,16 +491,17 @@ __global__ void __launch_bounds__(kBlock) k_adj_density(SlotView v, const float 
             gy += c * P.y + pb.w * P.g * ai.y;
             gz += c * P.z + pb.w * P.g * ai.z;
         });
-    const float4 o = lx[s];
-    lx[s] = make_float4(o.x + gx, o.y + gy, o.z + gz, 0.f);
+    gx = ln.sum(gx);
+    gy = ln.sum(gy);
+    gz = ln.sum(gz);
+    if (s >= v.n || ln.q != 0) return;
+    const float4 o = l.x[s];
+    l.x[s] = make_float4(o.x + gx, o.y + gy, o.z + gz, 0.f);
 }
 
 template <int DIM>
-__global__ void __launch_bounds__(kBlock) k_adj_out(SlotView v, const float4 *__restrict__ lx,
-                                                    const float4 *__restrict__ lu, float *gx, float *gv,
-                                                    int accumulate) {
-    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (s >= v.n) return;
+__device__ __forceinline__ void adj_out_item(const SlotView &v, const float4 *lx, const float4 *lu, float *gx,
+                                             float *gv, int accumulate, int64_t s) {
     const int64_t b = (int64_t)v.perm[s] * DIM;
     const float4 x = lx[s];
     const float xv[3] = {x.x, x.y, x.z};
@@ -466,13 +515,162 @@ __global__ void __launch_bounds__(kBlock) k_adj_out(SlotView v, const float4 *__
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_adj_in_density(SlotView v, const float *__restrict__ grho, float *lpsi,
-                                                           float4 *la1, float4 *lx) {
+// ----------------------------------------------------------------------------- one kernel a sweep
+// The sweeps as separate launches, where the cooperative kernel is not taken.
+template <int DIM>
+__global__ void __launch_bounds__(kBlock) k_adj_in(SlotView v, Lam l, const float *__restrict__ gx,
+                                                   const float *__restrict__ gv, int kp) {
+    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    if (s < v.n) adj_in_item<DIM>(v, l, gx, gv, kp, s);
+}
+
+__global__ void __launch_bounds__(kBlock) k_adj_kappa(SlotView v, Lam l, int kind, int it) {
+    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    adj_kappa_item<1>(v, l, Lanes<1>(), kind, it, s);
+}
+
+__global__ void __launch_bounds__(kBlock) k_adj_vel(SlotView v, Lam l, int kind, int it) {
+    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    adj_vel_item<1>(v, l, Lanes<1>(), kind, it, s);
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kBlock) k_adj_visc(SlotView v, Lam l, int kd, double *partials,
+                                                     unsigned int *ticket, double *gmu) {
+    __shared__ double sh[kBlock / 32];
+    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    const double contrib = adj_visc_item<DIM, 1>(v, l, Lanes<1>(), kd, s);
+    const double bs = block_sum<kBlock>(contrib, sh);
+    if (threadIdx.x == 0) partials[blockIdx.x] = bs;
+    if (last_block_done(ticket, gridDim.x)) {
+        double a = 0.0;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += kBlock) a += __ldcg(partials + i);
+        a = block_sum<kBlock>(a, sh);
+        if (threadIdx.x == 0) {
+            *gmu += a;
+            *ticket = 0;
+        }
+    }
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kBlock) k_adj_st1(SlotView v, Lam l) {
+    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    adj_st1_item<DIM, 1>(v, l, Lanes<1>(), s);
+}
+
+__global__ void __launch_bounds__(kBlock) k_adj_st2(SlotView v, Lam l) {
+    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    adj_st2_item<1>(v, l, Lanes<1>(), s);
+}
+
+__global__ void __launch_bounds__(kBlock) k_adj_alpha(SlotView v, Lam l) {
+    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    if (s < v.n) adj_alpha_item(v, l, s);
+}
+
+__global__ void __launch_bounds__(kBlock) k_adj_density(SlotView v, Lam l) {
+    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    adj_density_item<1>(v, l, Lanes<1>(), s);
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kBlock) k_adj_out(SlotView v, const float4 *__restrict__ lx,
+                                                    const float4 *__restrict__ lu, float *gx, float *gv,
+                                                    int accumulate) {
+    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    if (s < v.n) adj_out_item<DIM>(v, lx, lu, gx, gv, accumulate, s);
+}
+
+// ----------------------------------------------------------------------------- one launch a substep
+struct AdjArgs {
+    const float *gx_out, *gv_out;
+    float *gx_in, *gv_in;
+    double *gmu, *sums;  // sums: 32 per block, one per warp
+    unsigned int *bar;
+    int kd, kp;
+};
+
+// The reverse of a substep in one cooperative launch: fourteen or more sweeps of a
+// few microseconds each are otherwise as many launches.  A block's particles
+// in runs of 32 as elsewhere; with TPP lanes per particle a run takes TPP warps.
+template <int DIM, int TPP>
+__global__ void __launch_bounds__(1024, 1) k_adj_step(const __grid_constant__ SlotView v,
+                                                      const __grid_constant__ Lam lam,
+                                                      const __grid_constant__ AdjArgs a) {
+    __shared__ double sh[kBlock / 32];
+    GridBarrier bar{a.bar, 0u};
+    Lam l = lam;
+    // item(slot) for every lane of the particles' lane groups; all lanes of a warp call
+    auto sweep = [&](auto &&item) {
+        const WarpShare w(v.n);
+        const Lanes<TPP> ln;
+        for (int64_t i = threadIdx.x >> 5; i < w.count() * TPP; i += blockDim.x >> 5)
+            item(ln, (w.first * TPP + i) * ln.PPW + ln.p);
+    };
+    auto own = [&](const Lanes<TPP> &ln, int64_t s) { return s < v.n && ln.q == 0; };
+    auto solve = [&](int kind, int iters) {
+        for (int it = iters - 1; it >= 0; --it) {
+            sweep([&](const Lanes<TPP> &ln, int64_t s) { adj_kappa_item<TPP>(v, l, ln, kind, it, s); });
+            if (!bar.sync()) return false;
+            sweep([&](const Lanes<TPP> &ln, int64_t s) {
+                adj_vel_item<TPP>(v, l, ln, kind, it, s);
+                // lam_alpha is complete after the last kappa sweep
+                if (kind == kSolveDiv && it == 0 && own(ln, s)) adj_alpha_item(v, l, s);
+            });
+            if (!bar.sync()) return false;
+        }
+        return true;
+    };
+    auto run = [&]() {
+        sweep([&](const Lanes<TPP> &ln, int64_t s) {
+            if (own(ln, s)) adj_in_item<DIM>(v, l, a.gx_out, a.gv_out, a.kp, s);
+        });
+        if (!bar.sync() || !solve(kSolveDens, a.kp)) return false;
+        double g = 0.0;  // this lane's particles' share of dL/dmu
+        sweep([&](const Lanes<TPP> &ln, int64_t s) {
+            g += adj_visc_item<DIM, TPP>(v, l, ln, a.kd, s);
+            // the surface tension's reverse reads the same lam_a = dt lam_u
+            if (v.gamma != 0.f) adj_st1_item<DIM, TPP>(v, l, ln, s);
+            if (a.kd == 0 && own(ln, s)) adj_alpha_item(v, l, s);
+        });
+        g = warp_sum(g);
+        if ((threadIdx.x & 31) == 0) a.sums[blockIdx.x * 32 + (threadIdx.x >> 5)] = g;
+        if (!bar.sync()) return false;
+        if (v.gamma != 0.f) {
+            sweep([&](const Lanes<TPP> &ln, int64_t s) { adj_st2_item<TPP>(v, l, ln, s); });
+            if (a.kd == 0 && !bar.sync()) return false;
+        }
+        float4 *u = l.u;
+        l.u = l.u2;
+        l.u2 = u;
+        if (!solve(kSolveDiv, a.kd)) return false;
+        sweep([&](const Lanes<TPP> &ln, int64_t s) {
+            adj_density_item<TPP>(v, l, ln, s);
+            if (own(ln, s)) adj_out_item<DIM>(v, l.x, l.u, a.gx_in, a.gv_in, 0, s);
+        });
+        return true;
+    };
+    // (a barrier given up leaves the gradients unfinished: dL/dmu becomes NaN)
+    const bool done = run();
+    if (!last_block_done(a.bar + kBarLeft, gridDim.x)) return;
+    // dL/dmu: the warps' sums, in a fixed order
+    double g = 0.0;
+    const int warps = blockDim.x >> 5;
+    for (int i = threadIdx.x; i < (int)gridDim.x * warps && threadIdx.x < kBlock; i += kBlock)
+        g += __ldcg(a.sums + i / warps * 32 + i % warps);
+    g = coop_sum256(g, sh);
+    if (threadIdx.x != 0) return;
+    *a.gmu += done ? g : __longlong_as_double(0x7ff8000000000000ll);
+    a.bar[kBarCount] = a.bar[kBarGaveUp] = a.bar[kBarLeft] = 0;
+}
+
+__global__ void __launch_bounds__(kBlock) k_adj_in_density(SlotView v, Lam l, const float *__restrict__ grho) {
     const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
     if (s >= v.n) return;
-    lpsi[s] = grho[v.perm[s]];
-    la1[s] = make_float4(0.f, 0.f, 0.f, 0.f);
-    lx[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+    l.psi[s] = grho[v.perm[s]];
+    l.a1[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+    l.x[s] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 int fail_text(int code, const char *msg) {
@@ -528,6 +726,25 @@ SlotView slot_view(const tsph_tape &t, int slot) {
     g.R = t.ctx->k.R;
     g.row_trim = c.row_trim;
     return v;
+}
+
+Lam lam_of(const tsph_tape &t) {
+    return {t.lam_u, t.lam_u2, t.lam_x, t.lam_beta, t.lam_us, t.lam_a1, t.lam_n, t.lam_psi, t.lam_alpha};
+}
+
+// Up to this many warps of particles per SM a substep is reversed in one launch
+// (the forward step's rule, small_step_fits).
+constexpr int64_t kAdjWarpsPerSm = 512;
+
+// Eight lanes per particle while the SMs' 32 warps hold them all, then four, then
+// one: the sweeps of a small scene are chains of list blocks and their gathers,
+// one after another in a lane (a rollout of 2,028 particles: 5.1 ms, 6.5 with one lane).
+template <int DIM>
+cudaError_t launch_adj_step(tsph_ctx &c, const SlotView &v, const Lam &l, const AdjArgs &a, cudaStream_t st) {
+    const int64_t warps = ((int64_t)v.n + 31) / 32, runs = (warps + c.sms - 1) / c.sms;
+    if (runs * 8 <= 32) return launch_coop(k_adj_step<DIM, 8>, c.sms, coop_threads(runs * 8 * c.sms, c.sms), st, v, l, a);
+    if (runs * 4 <= 32) return launch_coop(k_adj_step<DIM, 4>, c.sms, coop_threads(runs * 4 * c.sms, c.sms), st, v, l, a);
+    return launch_coop(k_adj_step<DIM, 1>, c.sms, coop_threads(warps, c.sms), st, v, l, a);
 }
 
 // Host copy of every slot's metadata (one synchronisation per recording).
@@ -647,10 +864,12 @@ int tsph_tape_create(tsph_ctx *c, int slots, int max_iters, tsph_tape **out) {
     t->lam_u2 = (float4 *)get(N * sizeof(float4));
     t->lam_x = (float4 *)get(N * sizeof(float4));
     t->lam_a1 = (float4 *)get(N * sizeof(float4));
-    t->lam_s = (float *)get(N * sizeof(float));
+    t->lam_beta = (float4 *)get(N * sizeof(float4));
+    t->lam_us = (float4 *)get(N * sizeof(float4));
     t->lam_psi = (float *)get(N * sizeof(float));
     t->lam_alpha = (float *)get(N * sizeof(float));
-    t->partials = (double *)get((N / kBlock + 2) * sizeof(double));
+    t->partials = (double *)get(std::max(N / kBlock + 2, (size_t)c->sms * 32) * sizeof(double));
+    t->bar = (unsigned int *)get(kBarWords * sizeof(unsigned int));
     t->ticket = (unsigned int *)get(sizeof(unsigned int));
     if (c->st_on) {
         a.nstart = c->k.total_nodes + 1;
@@ -693,33 +912,39 @@ int tsph_substep_adjoint(tsph_ctx *c, tsph_tape *t, int slot, const float *gx_ou
         return fail_text(TSPH_ERR_STATE, "tape slot ran more iterations than it holds");
     const SlotView v = slot_view(*t, slot);
     const int nb = blocks_for(v.n);
-    const int dim = c->k.dim;
-    float4 *lu = t->lam_u, *lu2 = t->lam_u2;
-    if (dim == 3) k_adj_in<3><<<nb, kBlock, 0, st>>>(v, gx_out, gv_out, t->lam_x, lu, t->lam_psi, t->lam_alpha);
-    else k_adj_in<2><<<nb, kBlock, 0, st>>>(v, gx_out, gv_out, t->lam_x, lu, t->lam_psi, t->lam_alpha);
-    for (int it = m.kp - 1; it >= 0; --it) {
-        k_adj_kappa<<<nb, kBlock, 0, st>>>(v, kSolveDens, it, lu, t->lam_s, t->lam_x, t->lam_psi, t->lam_alpha);
-        k_adj_vel<<<nb, kBlock, 0, st>>>(v, kSolveDens, it, t->lam_s, lu, t->lam_x);
+    Lam l = lam_of(*t);
+    if (c->use_graph && c->sms && ((int64_t)v.n + 31) / 32 <= kAdjWarpsPerSm * c->sms) {
+        const AdjArgs a = {gx_out, gv_out, gx_in, gv_in, gmu, t->partials, t->bar, m.kd, m.kp};
+        const cudaError_t e = c->k.dim == 3 ? launch_adj_step<3>(*c, v, l, a, st) : launch_adj_step<2>(*c, v, l, a, st);
+        if (e == cudaSuccess) return TSPH_OK;
+        // this process may not use every SM at once: separate launches
+        if (e != cudaErrorCooperativeLaunchTooLarge) return fail_text(TSPH_ERR_CUDA, cudaGetErrorString(e));
+        (void)cudaGetLastError();
     }
-    if (dim == 3) k_adj_visc<3><<<nb, kBlock, 0, st>>>(v, lu, lu2, t->lam_x, t->lam_psi, t->partials, t->ticket, gmu);
-    else k_adj_visc<2><<<nb, kBlock, 0, st>>>(v, lu, lu2, t->lam_x, t->lam_psi, t->partials, t->ticket, gmu);
+    auto solve = [&](int kind, int iters) {
+        for (int it = iters - 1; it >= 0; --it) {
+            k_adj_kappa<<<nb, kBlock, 0, st>>>(v, l, kind, it);
+            k_adj_vel<<<nb, kBlock, 0, st>>>(v, l, kind, it);
+        }
+    };
+    const bool d3 = c->k.dim == 3;
+    if (d3) k_adj_in<3><<<nb, kBlock, 0, st>>>(v, l, gx_out, gv_out, m.kp);
+    else k_adj_in<2><<<nb, kBlock, 0, st>>>(v, l, gx_out, gv_out, m.kp);
+    solve(kSolveDens, m.kp);
+    if (d3) k_adj_visc<3><<<nb, kBlock, 0, st>>>(v, l, m.kd, t->partials, t->ticket, gmu);
+    else k_adj_visc<2><<<nb, kBlock, 0, st>>>(v, l, m.kd, t->partials, t->ticket, gmu);
     if (v.gamma != 0.f) {
         // the surface tension's reverse reads the same lam_a = dt lam_u as k_adj_visc
-        if (dim == 3) k_adj_st1<3><<<nb, kBlock, 0, st>>>(v, lu, t->lam_n, t->lam_x, t->lam_psi);
-        else k_adj_st1<2><<<nb, kBlock, 0, st>>>(v, lu, t->lam_n, t->lam_x, t->lam_psi);
-        k_adj_st2<<<nb, kBlock, 0, st>>>(v, t->lam_n, t->lam_x, t->lam_psi);
+        if (d3) k_adj_st1<3><<<nb, kBlock, 0, st>>>(v, l);
+        else k_adj_st1<2><<<nb, kBlock, 0, st>>>(v, l);
+        k_adj_st2<<<nb, kBlock, 0, st>>>(v, l);
     }
-    float4 *tmp = lu;
-    lu = lu2;
-    lu2 = tmp;
-    for (int it = m.kd - 1; it >= 0; --it) {
-        k_adj_kappa<<<nb, kBlock, 0, st>>>(v, kSolveDiv, it, lu, t->lam_s, t->lam_x, t->lam_psi, t->lam_alpha);
-        k_adj_vel<<<nb, kBlock, 0, st>>>(v, kSolveDiv, it, t->lam_s, lu, t->lam_x);
-    }
-    k_adj_alpha_prep<<<nb, kBlock, 0, st>>>(v, t->lam_alpha, t->lam_a1);
-    k_adj_density<<<nb, kBlock, 0, st>>>(v, t->lam_psi, t->lam_a1, t->lam_x);
-    if (dim == 3) k_adj_out<3><<<nb, kBlock, 0, st>>>(v, t->lam_x, lu, gx_in, gv_in, 0);
-    else k_adj_out<2><<<nb, kBlock, 0, st>>>(v, t->lam_x, lu, gx_in, gv_in, 0);
+    std::swap(l.u, l.u2);
+    solve(kSolveDiv, m.kd);
+    k_adj_alpha<<<nb, kBlock, 0, st>>>(v, l);
+    k_adj_density<<<nb, kBlock, 0, st>>>(v, l);
+    if (d3) k_adj_out<3><<<nb, kBlock, 0, st>>>(v, l.x, l.u, gx_in, gv_in, 0);
+    else k_adj_out<2><<<nb, kBlock, 0, st>>>(v, l.x, l.u, gx_in, gv_in, 0);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TSPH_OK : fail_text(TSPH_ERR_CUDA, cudaGetErrorString(e));
 }
@@ -735,10 +960,11 @@ int tsph_density_adjoint(tsph_ctx *c, tsph_tape *t, int slot, const float *grho,
     if (rc) return rc;
     const SlotView v = slot_view(*t, slot);
     const int nb = blocks_for(v.n);
-    k_adj_in_density<<<nb, kBlock, 0, st>>>(v, grho, t->lam_psi, t->lam_a1, t->lam_x);
-    k_adj_density<<<nb, kBlock, 0, st>>>(v, t->lam_psi, t->lam_a1, t->lam_x);
-    if (c->k.dim == 3) k_adj_out<3><<<nb, kBlock, 0, st>>>(v, t->lam_x, nullptr, gx, nullptr, 1);
-    else k_adj_out<2><<<nb, kBlock, 0, st>>>(v, t->lam_x, nullptr, gx, nullptr, 1);
+    const Lam l = lam_of(*t);
+    k_adj_in_density<<<nb, kBlock, 0, st>>>(v, l, grho);
+    k_adj_density<<<nb, kBlock, 0, st>>>(v, l);
+    if (c->k.dim == 3) k_adj_out<3><<<nb, kBlock, 0, st>>>(v, l.x, nullptr, gx, nullptr, 1);
+    else k_adj_out<2><<<nb, kBlock, 0, st>>>(v, l.x, nullptr, gx, nullptr, 1);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? TSPH_OK : fail_text(TSPH_ERR_CUDA, cudaGetErrorString(e));
 }

@@ -234,22 +234,40 @@ int bind_sets(tsph_ctx *c, const tsph_set *f, const tsph_set *b) {
     return TSPH_OK;
 }
 
+// The step (or, with density_out, its first part) as one cooperative launch, where
+// the sets take it (`taken`).
+int small_step(tsph_ctx *c, const tsph_set *f, const tsph_set *b, bool with_cfl, float *density_out, cudaStream_t st,
+               bool &taken) {
+    taken = small_step_fits(*c, *f, *b);
+    if (!taken) return TSPH_OK;
+    const cudaError_t e = launch_small_step(*c, *f, *b, with_cfl, density_out, st);
+    if (e == cudaSuccess) return TSPH_OK;
+    // this process may not use every SM at once: separate launches from here on
+    if (e != cudaErrorCooperativeLaunchTooLarge) return fail_cuda(e, "the one-launch step");
+    (void)cudaGetLastError();
+    c->sms = 0;
+    taken = false;
+    return TSPH_OK;
+}
+
 int run_step(tsph_ctx *c, const tsph_set *f, const tsph_set *b, void *stream, bool with_cfl) {
     int rc = bind_sets(c, f, b);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    if (c->use_graph && small_step_fits(*c, *f, *b)) {
-        const cudaError_t e = launch_small_step(*c, *f, *b, with_cfl, st);
-        if (e == cudaSuccess) {
+    if (c->use_graph) {
+        bool taken;
+        rc = small_step(c, f, b, with_cfl, nullptr, st, taken);
+        if (rc) return rc;
+        if (taken) {
             c->launches_per_step = 1;
             c->launches_per_iter = c->launches_per_pass = 0;
             c->stepped++;
             return TSPH_OK;
         }
-        // this process may not use every SM at once: separate launches from here on
-        if (e != cudaErrorCooperativeLaunchTooLarge) return fail_cuda(e, "the one-launch step");
-        (void)cudaGetLastError();
-        c->sms = 0;
+    }
+    if (c->rec_tape) {
+        rc = tape_begin(*c->rec_tape, c->rec_slot, st);
+        if (rc) return rc;
     }
     if (!c->use_graph) {
         rc = enqueue_step(*c, *f, *b, st, with_cfl, false);
@@ -926,10 +944,10 @@ int tsph_set_state(tsph_ctx *c, double time_count, float dt, double compression,
 int tsph_substep_record(tsph_ctx *c, const tsph_set *f, const tsph_set *b, tsph_tape *t, int slot, void *stream) {
     if (!c || !t || t->ctx != c) return fail(TSPH_ERR_INVALID, "tape does not belong to this context");
     if (slot < 0 || slot >= t->a.slots) return fail(TSPH_ERR_INVALID, "tape slot out of range");
-    int rc = tape_begin(*t, slot, (cudaStream_t)stream);
-    if (rc) return rc;
+    t->host_valid = 0;
     c->rec_tape = t;
-    rc = run_step(c, f, b, stream, true);
+    c->rec_slot = slot;
+    const int rc = run_step(c, f, b, stream, true);
     c->rec_tape = nullptr;
     return rc;
 }
@@ -942,9 +960,16 @@ int tsph_density_record(tsph_ctx *c, const tsph_set *f, const tsph_set *b, tsph_
     int rc = bind_sets(c, f, b);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    rc = tape_begin(*t, slot, st);
-    if (rc) return rc;
+    t->host_valid = 0;
     c->rec_tape = t;
+    c->rec_slot = slot;
+    bool taken = false;
+    if (c->use_graph) rc = small_step(c, f, b, false, out, st, taken);
+    if (!rc && !taken) rc = tape_begin(*t, slot, st);
+    if (rc || taken) {
+        c->rec_tape = nullptr;
+        return rc;
+    }
     launch_step_begin(*c, st);
     launch_grid_build(*c, *f, *b, st);
     launch_density(*c, st);

@@ -32,6 +32,7 @@ struct tsph_ctx {
     cudaGraphExec_t exec[2];
     unsigned long long graph_key[2][4];
     tsph_tape *rec_tape;      // non-null while a recorded step is enqueued
+    int rec_slot;             // its tape slot
     int launches;             // kernel launches enqueued (counted by the launchers)
     int launches_per_step;    // top-level kernels of the last enqueued step
     int launches_per_iter;    // kernels of a solver iteration of the last enqueued step
@@ -120,7 +121,9 @@ void launch_density_out(tsph_ctx &c, float *out, cudaStream_t st);
 // small.cu
 // Whether the step runs as one launch (launch_small_step) for these sets.
 bool small_step_fits(const tsph_ctx &c, const tsph_set &f, const tsph_set &b);
-cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b, bool with_cfl, cudaStream_t st);
+// density_out: not null to stop after the density sweep and write the densities there.
+cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b, bool with_cfl, float *density_out,
+                              cudaStream_t st);
 
 // fbm.cu
 void launch_fbm_begin(tsph_ctx &c, cudaGraphConditionalHandle h, int use_cond, cudaStream_t st);

@@ -23,7 +23,8 @@ bool small_step_fits(const tsph_ctx &c, const tsph_set &f, const tsph_set &b) {
     return (f.n + 31) / 32 + (b.n + 31) / 32 <= kSmallWarpsPerSm * c.sms;
 }
 
-cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b, bool with_cfl, cudaStream_t st) {
+cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b, bool with_cfl, float *density_out,
+                              cudaStream_t st) {
     SmallArgs a = {};
     a.f = f;
     a.b = b;
@@ -31,14 +32,13 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
     a.with_cfl = with_cfl ? 1 : 0;
     a.st_on = c.st_on;
     a.wc = c.p.wcsph_enabled;
+    a.density_out = density_out;
     if (c.rec_tape) {
         a.tape = c.rec_tape->a;
         a.record = 1;
+        a.slot = c.rec_slot;
     }
-    // enough warps per block for one pass over the particles: 8, 16 or 32 (fewer
-    // warps meet sooner at a barrier: 5k particles 136 us a substep with 8, 145 with 32)
-    const int64_t warps = ((f.n + 31) / 32 + (b.n + 31) / 32 + c.sms - 1) / c.sms;
-    const int threads = warps <= 8 ? 256 : warps <= 16 ? 512 : 1024;
+    const int threads = coop_threads((f.n + 31) / 32 + (b.n + 31) / 32, c.sms);
     return c.k.dim == 3 ? launch_small_dim<3>(c, a, threads, st) : launch_small_dim<2>(c, a, threads, st);
 }
 

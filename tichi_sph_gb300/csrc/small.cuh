@@ -13,7 +13,7 @@
 // Which scenes take it: see small_step_fits.
 #pragma once
 
-#include "ctx.h"
+#include "coop.cuh"
 #include "fbm.cuh"
 #include "grid.cuh"
 #include "sweeps.cuh"
@@ -27,74 +27,10 @@ struct SmallArgs {
     tsph_set f, b;
     SmallScratch x;
     TapeArrays tape;
+    float *density_out;  // not null: only the grid and the densities (in the caller's order), no step
+    int slot;            // of the tape
     int record, with_cfl, st_on, wc;
 };
-
-// A poll of the barrier's counter takes about half a microsecond: the limit is
-// a few seconds, after which the step is given up and its status says so.
-constexpr unsigned int kSpinLimit = 1u << 23;
-
-// Barrier over the grid's blocks (all resident: a cooperative launch).  The
-// counter only grows within a launch; the launch's last block to leave sets it
-// back.  False: a block did not arrive within the limit; every block then leaves.
-struct GridBarrier {
-    unsigned int *bar;  // words kBarCount, kBarGaveUp, kBarLeft
-    unsigned int target;
-    static __device__ __forceinline__ unsigned int acquire(const unsigned int *p) {
-        unsigned int v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-        return v;
-    }
-    __device__ __forceinline__ bool sync() {
-        __shared__ int ok;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            target += gridDim.x;
-            // release / acquire at GPU scope, with the block's two barriers around
-            // them, order everything before against everything after
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar + kBarCount) : "memory");
-            bool all = true;
-            unsigned int n = 0;
-            while (acquire(bar + kBarCount) < target) {
-                if ((++n & 1023u) != 0) continue;
-                if (n > kSpinLimit) atomicExch(bar + kBarGaveUp, 1u);
-                if (acquire(bar + kBarGaveUp)) {
-                    all = false;
-                    break;
-                }
-            }
-            ok = all;
-        }
-        __syncthreads();
-        return ok != 0;
-    }
-};
-
-// The block's share of n items, in whole warps: contiguous runs of 32.
-struct WarpShare {
-    int64_t first, last;  // warps [first, last) of the items, before the end is cut off
-    __device__ __forceinline__ WarpShare(int64_t n) {
-        const int64_t nw = (n + 31) >> 5;
-        const int64_t per = (nw + gridDim.x - 1) / gridDim.x;
-        first = blockIdx.x * per;
-        last = first + per < nw ? first + per : nw;
-        if (first > last) first = last;
-    }
-    __device__ __forceinline__ int64_t count() const { return last - first; }
-};
-
-// Runs ff(i, warp) over the fluid's nf items and fb(i) over the boundary's nb in
-// the block's warps (every lane of a warp calls, i may be past the end).
-template <class FF, class FB>
-__device__ __forceinline__ void for_items(int64_t nf, int64_t nb, FF &&ff, FB &&fb) {
-    const WarpShare f(nf), b(nb);
-    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    const int64_t total = f.count() + b.count();
-    for (int64_t w = threadIdx.x >> 5; w < total; w += warps) {
-        if (w < f.count()) ff((f.first + w) * 32 + lane, f.first + w);
-        else fb((b.first + w - f.count()) * 32 + lane);
-    }
-}
 
 // Inclusive scan over the block; total in every thread.
 __device__ __forceinline__ int small_block_scan(int v, int *sh, int &total) {
@@ -147,14 +83,6 @@ __device__ __forceinline__ double small_psi_sum(const double *warp_sums, int64_t
     return acc;
 }
 
-// The tree of block_sum over a 256-thread block's eight warp sums.
-__device__ __forceinline__ double small_block_tree(const double *p) {
-    double v[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __ldcg(p + i);
-    return ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
-}
-
 // P: phases of the volume-fraction update, 0 without it.
 template <int DIM, bool ST, int P>
 struct SmallStep {
@@ -180,6 +108,7 @@ struct SmallStep {
             B.count[i] = 0;
         }
         if (tid < (int64_t)(sizeof(SceneStep) / 4)) reinterpret_cast<int *>(&st())[tid] = 0;
+        if (a.record && tid == 0) a.tape.meta[a.slot] = TapeMeta{};
         if (!a.with_cfl) return;
         float m = 0.f;
         for (int64_t i = tid; i < a.f.n; i += nt) {
@@ -272,7 +201,7 @@ struct SmallStep {
     __device__ __forceinline__ bool solve(int kind, bool psi_done) {
         const SceneConst &c = k.s0;
         const double tol = kind == kSolveDiv ? (double)c.div_tol : (double)c.comp_tol;
-        const int slot = a.record ? *a.tape.dslot : 0;
+        const int slot = a.slot;
         int it = 0;
         bool cond = 0 < c.iter_min || *(volatile double *)&k.sp[0].compression > tol;
         while (cond) {
@@ -375,13 +304,14 @@ struct SmallStep {
                   [&](int64_t u) { if (u < a.b.n) gather_bound_item<DIM>(k, a.b, B, c, 0, u); });
         if (!bar.sync()) return false;
         const bool psi0 = density_does_psi(c, *(volatile double *)&k.sp[0].compression);
-        const int slot = a.record ? *a.tape.dslot : 0;
+        const int slot = a.slot;
         for_items(ns, a.b.n,
             [&](int64_t s, int64_t w) {
                 double v = 0.0;
                 if (s < c.f_n) v = density_fluid_item<DIM, false, true, false>(k, F, B, 0, c, st(), 0, psi0, s);
                 put_warp_sum(v, w);
                 if (a.record) tape_state_fluid_item(k, F, a.tape, slot, s);
+                if (a.density_out && s < c.f_n) a.density_out[F.perm[s]] = F.dens[s].y;
             },
             [&](int64_t s) {
                 if (s >= c.b_n) return;
@@ -393,6 +323,7 @@ struct SmallStep {
             for (int64_t i = tid; i < a.tape.nstart; i += (int64_t)gridDim.x * blockDim.x)
                 a.tape.start[(int64_t)slot * a.tape.nstart + i] = F.start[i];
         }
+        if (a.density_out) return true;
         if (!bar.sync()) return false;
         cur = 0;
         if (!solve(kSolveDiv, psi0)) return false;
@@ -438,34 +369,23 @@ struct SmallStep {
     __device__ __forceinline__ void leave(bool done) {
         if (!last_block_done(a.x.bar + kBarLeft, gridDim.x)) return;
         double ke = 0.0, pe = 0.0;
-        for (int64_t i = threadIdx.x; i < ns / kBlock && threadIdx.x < kBlock; i += kBlock) {
-            ke += small_block_tree(a.x.sums + i * (kBlock / 32));
-            pe += small_block_tree(a.x.sums + ns / 32 + i * (kBlock / 32));
+        for (int64_t i = threadIdx.x; !a.density_out && i < ns / kBlock && threadIdx.x < kBlock; i += kBlock) {
+            ke += coop_block_tree(a.x.sums + i * (kBlock / 32));
+            pe += coop_block_tree(a.x.sums + ns / 32 + i * (kBlock / 32));
         }
-        ke = small_sum256(ke);
-        pe = small_sum256(pe);
+        ke = coop_sum256(ke, sh_d);
+        pe = coop_sum256(pe, sh_d);
         if (threadIdx.x != 0) return;
         if (done && !__ldcg(a.x.bar + kBarGaveUp)) {
-            st().kinetic_energy = ke;
-            st().potential_energy = pe;
-            step_totals(k.sp[0], st());
+            if (!a.density_out) {
+                st().kinetic_energy = ke;
+                st().potential_energy = pe;
+                step_totals(k.sp[0], st());
+            }
         } else {
             atomicOr(&st().status, kStGaveUp);
         }
         a.x.bar[kBarCount] = a.x.bar[kBarGaveUp] = a.x.bar[kBarLeft] = 0;
-    }
-    // block_sum<256> over the first 256 threads.
-    __device__ __forceinline__ double small_sum256(double v) {
-        v = warp_sum(v);
-        __syncthreads();
-        if ((threadIdx.x & 31) == 0 && threadIdx.x < kBlock) sh_d[threadIdx.x >> 5] = v;
-        __syncthreads();
-        double r = 0.0;
-        if (threadIdx.x < 32) {
-            r = threadIdx.x < kBlock / 32 ? sh_d[threadIdx.x] : 0.0;
-            r = warp_sum(r);
-        }
-        return r;
     }
 };
 
@@ -484,21 +404,12 @@ __global__ void __launch_bounds__(1024, 1) k_small_step(const __grid_constant__ 
 
 template <int DIM>
 cudaError_t launch_small_dim(tsph_ctx &c, const SmallArgs &a, int threads, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(c.sms);
-    cfg.blockDim = dim3(threads);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
     const bool fbm = c.p.fbm_enabled != 0;
     if (c.st_on)
-        return fbm ? cudaLaunchKernelEx(&cfg, k_small_step<DIM, true, 2>, c.k, c.F, c.B, a)
-                   : cudaLaunchKernelEx(&cfg, k_small_step<DIM, true, 0>, c.k, c.F, c.B, a);
-    return fbm ? cudaLaunchKernelEx(&cfg, k_small_step<DIM, false, 2>, c.k, c.F, c.B, a)
-               : cudaLaunchKernelEx(&cfg, k_small_step<DIM, false, 0>, c.k, c.F, c.B, a);
+        return fbm ? launch_coop(k_small_step<DIM, true, 2>, c.sms, threads, st, c.k, c.F, c.B, a)
+                   : launch_coop(k_small_step<DIM, true, 0>, c.sms, threads, st, c.k, c.F, c.B, a);
+    return fbm ? launch_coop(k_small_step<DIM, false, 2>, c.sms, threads, st, c.k, c.F, c.B, a)
+               : launch_coop(k_small_step<DIM, false, 0>, c.sms, threads, st, c.k, c.F, c.B, a);
 }
 
 }  // namespace tsph

@@ -47,10 +47,11 @@ struct tsph_tape {
     tsph::TapeMeta *host_meta;  // pinned copy of every slot's metadata
     int host_valid;             // host_meta matches the device
     // reverse-pass scratch in sorted order (cap entries)
-    float4 *lam_u, *lam_u2, *lam_x, *lam_a1;
+    float4 *lam_u, *lam_u2, *lam_x, *lam_a1, *lam_beta, *lam_us;
     float4 *lam_n;  // adjoint of the surface normals (surface tension on)
-    float *lam_s, *lam_psi, *lam_alpha;
+    float *lam_psi, *lam_alpha;
     double *partials;
     unsigned int *ticket;
+    unsigned int *bar;  // words of the grid barrier (coop.cuh)
     std::vector<void *> allocs;
 };
