@@ -61,12 +61,14 @@ def _solver(dim, n, nb, two, use_graph, gamma=0.0, inside=False):
 
 @pytest.mark.parametrize("dim,n,nb,two", [(2, 1, 0, False), (2, 33, 40, False), (2, 257, 0, True),
                                           (2, 700, 90, True), (3, 31, 1, False), (3, 256, 257, False),
-                                          (3, 900, 300, True), (3, 5000, 700, False)])
+                                          (3, 900, 300, True), (3, 5000, 700, False), (2, 21000, 500, True),
+                                          (3, 25000, 900, False), (2, 60000, 0, False)])
 def test_one_launch_equals_separate_kernels(dim, n, nb, two):
+    # (above 19,456 particles four lanes of a warp share one, above 38,912 one has it)
     _need_cuda()
     runs = []
     for use_graph in (True, False):
-        s = _solver(dim, n, nb, two, use_graph)
+        s = _solver(dim, n, nb, two, use_graph, inside=n > 5000)
         stats = []
         for _ in range(3):
             s.substep()

@@ -451,7 +451,7 @@ int create_impl(const tsph_params *ps, int S, const int64_t *fn, const int64_t *
 
     FluidBuf &F = c.F;
     F.cap = fcap;
-    F.count = A.get<int>(nn);
+    F.count = A.get<int>(nn + 3);
     F.start = A.get<int>(nn + 1);
     F.slot = A.get<int>((long long)fus.size());
     F.inv = A.get<int>((long long)fus.size());
@@ -482,7 +482,7 @@ int create_impl(const tsph_params *ps, int S, const int64_t *fn, const int64_t *
     F.wcp = ps[0].wcsph_enabled ? A.get<float2>(fcap) : nullptr;
     BoundBuf &B = c.B;
     B.cap = bcap;
-    B.count = A.get<int>(nn);
+    B.count = A.get<int>(nn + 3);
     B.start = A.get<int>(nn + 1);
     B.slot = A.get<int>((long long)bus.size());
     B.inv = A.get<int>((long long)bus.size());
@@ -511,6 +511,7 @@ int create_impl(const tsph_params *ps, int S, const int64_t *fn, const int64_t *
         c.X.vmax = A.get<float>(c.sms);
         c.X.totals = A.get<int>(2 * c.sms);
         c.X.bar = A.get<unsigned int>(kBarWords);
+        c.counts_zero = 1;  // as allocated
     }
     SceneConst *d_sc = A.get<SceneConst>(S);
     k.sp = A.get<ScenePersist>(S);
@@ -872,8 +873,10 @@ int tsph_read_scene_stats(tsph_ctx *c, int first, int count, tsph_stats *out, vo
     TSPH_CK(cudaMemcpyAsync(c->host_ss, c->k.ss, sizeof(SceneStep) * c->n_scenes, cudaMemcpyDeviceToHost, st));
     TSPH_CK(cudaMemcpyAsync(c->host_sp, c->k.sp, sizeof(ScenePersist) * c->n_scenes, cudaMemcpyDeviceToHost, st));
     TSPH_CK(cudaStreamSynchronize(st));
-    if (c->host_ss[0].status & kStGaveUp)
+    if (c->host_ss[0].status & kStGaveUp) {
+        c->counts_zero = 0;
         return fail(TSPH_ERR_CUDA, "the step gave up at a grid barrier: a block did not arrive");
+    }
     for (int i = 0; i < count; ++i) fill_stats(c, first + i, out + i);
     return TSPH_OK;
 }

@@ -230,8 +230,9 @@ struct BoundBuf {
 };
 
 // Scratch of the one-launch step (small.cuh): per-warp sums, per-block maxima and
-// cell totals, the grid barrier's words (each in a line of its own).
-enum { kBarCount = 0, kBarGaveUp = 32, kBarLeft = 64, kBarWords = 96 };
+// cell totals, the grid barrier's words (each in a line of its own) and the encode's
+// counters (tails and status, until the step's scalars are set).
+enum { kBarCount = 0, kBarGaveUp = 32, kBarLeft = 64, kBarTailF = 96, kBarTailB = 97, kBarStatus = 98, kBarWords = 128 };
 constexpr int kSmallSums = 512;  // block sums held in shared memory at a time
 struct SmallScratch {
     double *sums;

@@ -48,15 +48,14 @@ struct GridBarrier {
     }
 };
 
-// The block's share of n items, in whole warps: contiguous runs of 32.
+// The block's share of n items: contiguous runs of 32, shares that differ by one
+// run at most.
 struct WarpShare {
-    int64_t first, last;  // warps [first, last) of the items, before the end is cut off
+    int64_t first, last;  // runs [first, last)
     __device__ __forceinline__ WarpShare(int64_t n) {
-        const int64_t nw = (n + 31) >> 5;
-        const int64_t per = (nw + gridDim.x - 1) / gridDim.x;
-        first = blockIdx.x * per;
-        last = first + per < nw ? first + per : nw;
-        if (first > last) first = last;
+        const unsigned int nw = (unsigned int)((n + 31) >> 5), per = nw / gridDim.x, more = nw % gridDim.x;
+        first = (int64_t)blockIdx.x * per + min(blockIdx.x, more);
+        last = first + per + (blockIdx.x < more ? 1 : 0);
     }
     __device__ __forceinline__ int64_t count() const { return last - first; }
 };

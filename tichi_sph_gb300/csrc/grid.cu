@@ -80,7 +80,10 @@ __global__ void __launch_bounds__(kBlock) k_encode(KConst k, tsph_set U, int bou
                                                    int *__restrict__ slot) {
     pdl_entry();
     const int64_t i = blockIdx.x * (int64_t)kBlock + threadIdx.x;
-    if (i < U.n) encode_item<DIM>(k, U, bound, count, slot, i);
+    if (i >= U.n) return;
+    const int sc = bound ? k.b_user_scene[i] : k.f_user_scene[i];
+    SceneStep &st = k.ss[sc];
+    encode_item<DIM>(k, U, sc, count, slot, bound ? &st.b_tail : &st.f_tail, &st.status, i);
 }
 
 // ----------------------------------------------------------------------------- scan
@@ -377,6 +380,7 @@ void launch_grid_build(tsph_ctx &c, const tsph_set &f, const tsph_set &b, cudaSt
     // the boundary set's encode, scatter and gather run on the side stream,
     // beside the fluid's; the scans cover both grids in one launch
     cudaStream_t sd = c.side ? c.side : st;
+    c.counts_zero = 0;
     c.launches += (f.n > 0) + (b.n > 0) + 2 + (f.n > 0) + (b.n > 0) + 2;
     fork_side(c, st);
     if (with_cfl) launch_cfl(c, f, sd);  // nothing before the first solve reads dt

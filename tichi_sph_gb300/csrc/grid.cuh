@@ -12,9 +12,8 @@ namespace tsph {
 // count in the scene's range of the global grid.  A particle without a valid
 // code gets a rank in its scene's tail.
 template <int DIM>
-__device__ __forceinline__ void encode_item(const KConst &k, const tsph_set &U, int bound, int *count, int *slot,
-                                            int64_t i) {
-    const int sc = bound ? k.b_user_scene[i] : k.f_user_scene[i];
+__device__ __forceinline__ void encode_item(const KConst &k, const tsph_set &U, int sc, int *count, int *slot, int *tail,
+                                            int *status, int64_t i) {
     Geo g;
     g.load(k.sc[sc], k.R);
     float4 p = make_float4(U.pos[i * DIM], U.pos[i * DIM + 1], DIM == 3 ? U.pos[i * DIM + 2] : 0.f, 0.f);
@@ -29,8 +28,8 @@ __device__ __forceinline__ void encode_item(const KConst &k, const tsph_set &U, 
     if (ok && code > 0 && code < g.node_num) {
         s = atomicAdd(count + g.cbase + code, 1);
     } else {
-        s = -1 - atomicAdd(bound ? &k.ss[sc].b_tail : &k.ss[sc].f_tail, 1);
-        atomicOr(&k.ss[sc].status, ok ? TSPH_ST_OUTSIDE_GRID : (TSPH_ST_NONFINITE_POS | TSPH_ST_OUTSIDE_GRID));
+        s = -1 - atomicAdd(tail, 1);
+        atomicOr(status, ok ? TSPH_ST_OUTSIDE_GRID : (TSPH_ST_NONFINITE_POS | TSPH_ST_OUTSIDE_GRID));
     }
     slot[i] = s;
 }

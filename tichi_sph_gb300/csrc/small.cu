@@ -1,10 +1,13 @@
-// The one-launch step of small scenes (small.cuh): its rule, its launch and the 3D
-// instances (small2.cu holds the 2D ones).
+// The one-launch step of small scenes (small.cuh): its rules and its launch.  The
+// small_*d_*.cu files hold the kernel's instances.
 #include "small.cuh"
 
 namespace tsph {
 
-extern template cudaError_t launch_small_dim<2>(tsph_ctx &, const SmallArgs &, int, cudaStream_t);
+#define TSPH_SMALL(D, L) extern template cudaError_t launch_small_lanes<D, L>(tsph_ctx &, const SmallArgs &, int, cudaStream_t);
+TSPH_SMALL(2, 1) TSPH_SMALL(2, 4) TSPH_SMALL(2, 8)
+TSPH_SMALL(3, 1) TSPH_SMALL(3, 4) TSPH_SMALL(3, 8)
+#undef TSPH_SMALL
 
 // One-scene contexts on the default settings (the solver loops on the device, one
 // thread per particle) whose options the kernel has, up to 512 warps of
@@ -38,8 +41,30 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
         a.record = 1;
         a.slot = c.rec_slot;
     }
-    const int threads = coop_threads((f.n + 31) / 32 + (b.n + 31) / 32, c.sms);
-    return c.k.dim == 3 ? launch_small_dim<3>(c, a, threads, st) : launch_small_dim<2>(c, a, threads, st);
+    // lanes per particle: as many as the block's 32 warps leave for its runs of 32
+    // (us a substep with one lane and with eight or four: 1.3k particles in 3D 166 /
+    // 93, 8k 155 / 95, 27k 177 / 143; in 2D, a third of the neighbours, 5k 132 / 122)
+    const int64_t runs = ((f.n + kBlock - 1) / kBlock * (kBlock / 32) + c.sms - 1) / c.sms;
+    const int lanes = runs * 8 <= 32 ? 8 : runs * 4 <= 32 ? 4 : 1;
+    const int64_t bruns = ((b.n + 31) / 32 + c.sms - 1) / c.sms;
+    const int threads = coop_threads((runs * lanes + bruns) * c.sms, c.sms);
+    // the kernel leaves zero counters behind, other grid builds do not; a captured
+    // launch must not rely on what came before it
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(st, &cap);
+    if (!c.counts_zero || cap != cudaStreamCaptureStatusNone) {
+        cudaError_t e = cudaMemsetAsync(c.F.count, 0, sizeof(int) * c.k.total_nodes, st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(c.B.count, 0, sizeof(int) * c.k.total_nodes, st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(c.X.bar + kBarTailF, 0, 4 * (kBarWords - kBarTailF), st);
+        if (e != cudaSuccess) return e;
+    }
+    c.counts_zero = 1;
+    const bool d3 = c.k.dim == 3;
+    switch (lanes) {
+        case 8: return d3 ? launch_small_lanes<3, 8>(c, a, threads, st) : launch_small_lanes<2, 8>(c, a, threads, st);
+        case 4: return d3 ? launch_small_lanes<3, 4>(c, a, threads, st) : launch_small_lanes<2, 4>(c, a, threads, st);
+        default: return d3 ? launch_small_lanes<3, 1>(c, a, threads, st) : launch_small_lanes<2, 1>(c, a, threads, st);
+    }
 }
 
 }  // namespace tsph

@@ -16,6 +16,7 @@
 #include "coop.cuh"
 #include "fbm.cuh"
 #include "grid.cuh"
+#include "lanes.cuh"
 #include "sweeps.cuh"
 #include "tape.cuh"
 #include "wcsph.cuh"
@@ -83,8 +84,10 @@ __device__ __forceinline__ double small_psi_sum(const double *warp_sums, int64_t
     return acc;
 }
 
-// P: phases of the volume-fraction update, 0 without it.
-template <int DIM, bool ST, int P>
+// P: phases of the volume-fraction update, 0 without it.  L: lanes per particle of
+// the neighbour sweeps (lanes.cuh); with more than one, a block's warps hold all of
+// its runs of 32 particles at a time (launch_small_step).
+template <int DIM, bool ST, int P, int L>
 struct SmallStep {
     const KConst &k;
     const FluidBuf &F;
@@ -100,14 +103,9 @@ struct SmallStep {
     __device__ __forceinline__ bool first_block() const { return blockIdx.x == 0; }
     __device__ __forceinline__ bool last_block() const { return blockIdx.x == gridDim.x - 1; }
 
-    // Zeroes the step's counters; with the CFL condition on, the block's largest |v|.
-    __device__ __forceinline__ void begin() {
+    // With the CFL condition on, the block's largest |v|.
+    __device__ __forceinline__ void largest_speed() {
         const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
-        for (int64_t i = tid; i < k.total_nodes; i += nt) {
-            F.count[i] = 0;
-            B.count[i] = 0;
-        }
-        if (tid < (int64_t)(sizeof(SceneStep) / 4)) reinterpret_cast<int *>(&st())[tid] = 0;
         if (a.record && tid == 0) a.tape.meta[a.slot] = TapeMeta{};
         if (!a.with_cfl) return;
         float m = 0.f;
@@ -147,12 +145,15 @@ struct SmallStep {
         k.sp[0].time_count += (double)dt;
     }
 
-    // The block's cells [lo, hi) of the two grids' counts.
+    // The block's cells [lo, hi) of the two grids (lo a multiple of four).
     __device__ __forceinline__ void cell_range(int64_t &lo, int64_t &hi) const {
-        const int64_t per = (k.total_nodes + gridDim.x - 1) / gridDim.x;
+        const int64_t per = ((k.total_nodes + gridDim.x - 1) / gridDim.x + 3) & ~(int64_t)3;
         lo = blockIdx.x * per < k.total_nodes ? blockIdx.x * per : k.total_nodes;
         hi = lo + per < k.total_nodes ? lo + per : k.total_nodes;
     }
+    // Few enough cells that each block adds up the counts before its own (four loads
+    // a thread at the most) rather than meet at a barrier for the blocks' totals.
+    __device__ __forceinline__ bool few_cells() const { return k.total_nodes <= 16384; }
     __device__ __forceinline__ void count_totals() {
         int64_t lo, hi;
         cell_range(lo, hi);
@@ -164,14 +165,25 @@ struct SmallStep {
             if (threadIdx.x == 0) a.x.totals[2 * blockIdx.x + g] = total;
         }
     }
+    // The cells' starts; the last block sets the step's scalars.
     __device__ __forceinline__ void scan_cells() {
         int64_t lo, hi;
         cell_range(lo, hi);
+        int in[2];
         for (int g = 0; g < 2; ++g) {
             const int *count = g ? B.count : F.count;
             int *start = g ? B.start : F.start;
             int before = 0, total;
-            for (int i = threadIdx.x; i < (int)blockIdx.x; i += blockDim.x) before += __ldcg(a.x.totals + 2 * i + g);
+            if (few_cells()) {
+                const int4 *c4 = reinterpret_cast<const int4 *>(count);
+                for (int64_t i = threadIdx.x; i < lo / 4; i += blockDim.x) {
+                    const int4 v = __ldcg(c4 + i);
+                    before += (v.x + v.y) + (v.z + v.w);
+                }
+                for (int64_t i = lo / 4 * 4 + threadIdx.x; i < lo; i += blockDim.x) before += __ldcg(count + i);
+            } else {
+                for (int i = threadIdx.x; i < (int)blockIdx.x; i += blockDim.x) before += __ldcg(a.x.totals + 2 * i + g);
+            }
             small_block_scan(before, sh_i, total);
             int run = total;  // particles in the cells before this block's
             for (int64_t i0 = lo; i0 < hi; i0 += blockDim.x) {
@@ -181,18 +193,65 @@ struct SmallStep {
                 if (i < hi) start[i] = run + incl - v;
                 run += total;
             }
-            if (last_block() && threadIdx.x == 0) {
-                start[k.total_nodes] = run;
-                if (g) st().b_in = run;
-                else st().f_in = run;
-            }
+            in[g] = run;
+            if (last_block() && threadIdx.x == 0) start[k.total_nodes] = run;
         }
+        if (!last_block() || threadIdx.x != 0) return;
+        SceneStep z = {};
+        z.f_in = in[0];
+        z.b_in = in[1];
+        z.f_tail = (int)__ldcg(a.x.bar + kBarTailF);
+        z.b_tail = (int)__ldcg(a.x.bar + kBarTailB);
+        z.status = (int)__ldcg(a.x.bar + kBarStatus);
+        st() = z;
+    }
+    // Zero counts for the next step (no phase reads them any more).
+    __device__ __forceinline__ void clear_counts() {
+        int64_t lo, hi;
+        cell_range(lo, hi);
+        for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) F.count[i] = B.count[i] = 0;
+        if (first_block() && threadIdx.x == 0) a.x.bar[kBarTailF] = a.x.bar[kBarTailB] = a.x.bar[kBarStatus] = 0;
     }
 
     // The warp's share of the scene's psi_sum.
     __device__ __forceinline__ void put_warp_sum(double v, int64_t warp) {
         v = warp_sum(v);
         if ((threadIdx.x & 31) == 0) a.x.sums[warp] = v;
+    }
+
+    // f(lanes, slot) -> the particle's share of psi_sum, over the fluid's slots and,
+    // with L > 1, L lanes per particle; the shares are summed per run of 32 slots
+    // (in f's last act of the phase: the block synchronises).  fb over the
+    // boundary's nb.
+    template <bool SUM, class FN, class FB>
+    __device__ __forceinline__ void lane_sweep(int64_t nb, FN &&f, FB &&fb) {
+        if constexpr (L == 1) {
+            for_items(ns, nb, [&](int64_t s, int64_t w) {
+                const double v = f(Lanes<1>(), s);
+                if (SUM) put_warp_sum(v, w);
+            }, fb);
+        } else {
+            lane_sweep_wide<SUM>(nb, f, fb);
+        }
+    }
+    template <bool SUM, class FN, class FB>
+    __device__ __forceinline__ void lane_sweep_wide(int64_t nb, FN &&f, FB &&fb) {
+        const WarpShare fl(ns), bo(nb);
+        const Lanes<L> ln;
+        const int64_t mine = fl.count() * L, total = mine + bo.count();
+        for (int64_t w = threadIdx.x >> 5; w < total; w += blockDim.x >> 5) {
+            if (w < mine) {
+                const int64_t in = w * ln.PPW + ln.p;  // slot within the block's runs
+                const double v = f(ln, fl.first * 32 + in);
+                if (SUM && ln.q == 0) sh_d[in] = v;
+            } else {
+                fb((bo.first + w - mine) * 32 + (threadIdx.x & 31));
+            }
+        }
+        if (!SUM) return;
+        __syncthreads();
+        for (int64_t r = threadIdx.x >> 5; r < fl.count(); r += blockDim.x >> 5)
+            put_warp_sum(sh_d[r * 32 + (threadIdx.x & 31)], fl.first + r);
     }
 
     // One pressure solve (k_solve_begin, k_psi, k_vel); psi_done: the first psi sweep
@@ -206,17 +265,18 @@ struct SmallStep {
         bool cond = 0 < c.iter_min || *(volatile double *)&k.sp[0].compression > tol;
         while (cond) {
             if (!psi_done) {
-                for_items(ns, 0, [&](int64_t s, int64_t w) {
-                    const Lanes<1> ln;
-                    put_warp_sum(psi_item<DIM, 1, false, false>(k, F, B, 0, c, st(), cur, ln, s, s < c.f_n), w);
+                lane_sweep<true>(0, [&](const Lanes<L> &ln, int64_t s) {
+                    if constexpr (L == 1) return psi_item<DIM, 1, false, false>(k, F, B, 0, c, st(), cur, ln, s, s < c.f_n);
+                    else return psi_lanes<DIM, L>(k, F, B, c, st(), cur, ln, s, s < c.f_n);
                 }, [](int64_t) {});
                 if (!bar.sync()) return false;
             }
             psi_done = false;
-            for_items(ns, 0, [&](int64_t s, int64_t) {
-                const Lanes<1> ln;
-                if (a.record) tape_iter_item(k, F, a.tape, slot, kind, it, cur, s);
-                vel_item<DIM, 1, false, false>(k, F, B, 0, c, st(), cur, ln, s, s < c.f_n);
+            lane_sweep<false>(0, [&](const Lanes<L> &ln, int64_t s) {
+                if (a.record && ln.q == 0) tape_iter_item(k, F, a.tape, slot, kind, it, cur, s);
+                if constexpr (L == 1) vel_item<DIM, 1, false, false>(k, F, B, 0, c, st(), cur, ln, s, s < c.f_n);
+                else vel_lanes<DIM, L>(k, F, B, c, st(), cur, ln, s, s < c.f_n);
+                return 0.0;
             }, [](int64_t) {});
             ++it;
             const bool capped = it > c.iter_max;
@@ -280,15 +340,21 @@ struct SmallStep {
 
     __device__ __forceinline__ bool run() {
         const SceneConst &c = k.s0;
-        begin();
-        if (!bar.sync()) return false;
-        time_step();
+        largest_speed();
+        int *ctr = reinterpret_cast<int *>(a.x.bar);
         for_items(a.f.n, a.b.n,
-                  [&](int64_t i, int64_t) { if (i < a.f.n) encode_item<DIM>(k, a.f, 0, F.count, F.slot, i); },
-                  [&](int64_t i) { if (i < a.b.n) encode_item<DIM>(k, a.b, 1, B.count, B.slot, i); });
+            [&](int64_t i, int64_t) {
+                if (i < a.f.n) encode_item<DIM>(k, a.f, 0, F.count, F.slot, ctr + kBarTailF, ctr + kBarStatus, i);
+            },
+            [&](int64_t i) {
+                if (i < a.b.n) encode_item<DIM>(k, a.b, 0, B.count, B.slot, ctr + kBarTailB, ctr + kBarStatus, i);
+            });
         if (!bar.sync()) return false;
-        count_totals();
-        if (!bar.sync()) return false;
+        if (!few_cells()) {
+            count_totals();
+            if (!bar.sync()) return false;
+        }
+        time_step();
         scan_cells();
         if (!bar.sync()) return false;
         for_items(a.f.n, a.b.n,
@@ -299,19 +365,25 @@ struct SmallStep {
                 if (i < a.b.n) scatter_item(k, 1, a.b.neighb_cell_seq, B.slot, B.start, B.perm_u, i);
             });
         if (!bar.sync()) return false;
+        clear_counts();
         for_items(a.f.n, a.b.n,
                   [&](int64_t u, int64_t) { if (u < a.f.n) gather_fluid_item<DIM>(k, a.f, F, c, st(), u); },
                   [&](int64_t u) { if (u < a.b.n) gather_bound_item<DIM>(k, a.b, B, c, 0, u); });
         if (!bar.sync()) return false;
         const bool psi0 = density_does_psi(c, *(volatile double *)&k.sp[0].compression);
         const int slot = a.slot;
-        for_items(ns, a.b.n,
-            [&](int64_t s, int64_t w) {
+        lane_sweep<true>(a.b.n,
+            [&](const Lanes<L> &ln, int64_t s) {
                 double v = 0.0;
-                if (s < c.f_n) v = density_fluid_item<DIM, false, true, false>(k, F, B, 0, c, st(), 0, psi0, s);
-                put_warp_sum(v, w);
+                if constexpr (L == 1) {
+                    if (s < c.f_n) v = density_fluid_item<DIM, false, true, false>(k, F, B, 0, c, st(), 0, psi0, s);
+                } else {
+                    v = density_fluid_lanes<DIM, L>(k, F, B, c, st(), 0, psi0, ln, s, s < c.f_n);
+                }
+                if (ln.q != 0) return v;
                 if (a.record) tape_state_fluid_item(k, F, a.tape, slot, s);
                 if (a.density_out && s < c.f_n) a.density_out[F.perm[s]] = F.dens[s].y;
+                return v;
             },
             [&](int64_t s) {
                 if (s >= c.b_n) return;
@@ -328,16 +400,19 @@ struct SmallStep {
         cur = 0;
         if (!solve(kSolveDiv, psi0)) return false;
         if (ST) {
-            for_items(ns, 0, [&](int64_t s, int64_t) {
-                const Lanes<1> ln;
-                normal_item<DIM, 1, false, false>(k, F, B, c, st(), ln, s, s < c.f_n);
+            lane_sweep<false>(0, [&](const Lanes<L> &ln, int64_t s) {
+                if constexpr (L == 1) normal_item<DIM, 1, false, false>(k, F, B, c, st(), ln, s, s < c.f_n);
+                else normal_lanes<DIM, L>(k, F, B, c, st(), ln, s, s < c.f_n);
+                return 0.0;
             }, [](int64_t) {});
             if (!bar.sync()) return false;
         }
-        for_items(ns, 0, [&](int64_t s, int64_t) {
-            const Lanes<1> ln;
-            advect_item<DIM, ST, 1, false, false>(k, F, B, 0, c, st(), cur, ln, s, s < c.f_n, 1.f, 1.f);
-            if (a.record) tape_vmid_item(k, F, a.tape, slot, s);
+        lane_sweep<false>(0, [&](const Lanes<L> &ln, int64_t s) {
+            if constexpr (L == 1)
+                advect_item<DIM, ST, 1, false, false>(k, F, B, 0, c, st(), cur, ln, s, s < c.f_n, 1.f, 1.f);
+            else advect_lanes<DIM, ST, L>(k, F, B, c, st(), cur, ln, s, s < c.f_n);
+            if (a.record && ln.q == 0) tape_vmid_item(k, F, a.tape, slot, s);
+            return 0.0;
         }, [](int64_t) {});
         if (!bar.sync()) return false;
         cur = 1 - cur;
@@ -390,26 +465,27 @@ struct SmallStep {
 };
 
 // One block per SM; 64 registers let the largest block have 1,024 threads.
-template <int DIM, bool ST, int P>
+template <int DIM, bool ST, int P, int L>
 __global__ void __launch_bounds__(1024, 1) k_small_step(const __grid_constant__ KConst k,
                                                         const __grid_constant__ FluidBuf F,
                                                         const __grid_constant__ BoundBuf B,
                                                         const __grid_constant__ SmallArgs a) {
     __shared__ double sh_d[kSmallSums];
     __shared__ int sh_i[33];
-    SmallStep<DIM, ST, P> step{k, F, B, a, {a.x.bar, 0u}, sh_d, sh_i, (a.f.n + kBlock - 1) / kBlock * kBlock, 0};
+    SmallStep<DIM, ST, P, L> step{k, F, B, a, {a.x.bar, 0u}, sh_d, sh_i, (a.f.n + kBlock - 1) / kBlock * kBlock, 0};
     const bool done = step.run();
     step.leave(done);
 }
 
-template <int DIM>
-cudaError_t launch_small_dim(tsph_ctx &c, const SmallArgs &a, int threads, cudaStream_t st) {
+// The instances with DIM and L (a translation unit each).
+template <int DIM, int L>
+cudaError_t launch_small_lanes(tsph_ctx &c, const SmallArgs &a, int threads, cudaStream_t st) {
     const bool fbm = c.p.fbm_enabled != 0;
     if (c.st_on)
-        return fbm ? launch_coop(k_small_step<DIM, true, 2>, c.sms, threads, st, c.k, c.F, c.B, a)
-                   : launch_coop(k_small_step<DIM, true, 0>, c.sms, threads, st, c.k, c.F, c.B, a);
-    return fbm ? launch_coop(k_small_step<DIM, false, 2>, c.sms, threads, st, c.k, c.F, c.B, a)
-               : launch_coop(k_small_step<DIM, false, 0>, c.sms, threads, st, c.k, c.F, c.B, a);
+        return fbm ? launch_coop(k_small_step<DIM, true, 2, L>, c.sms, threads, st, c.k, c.F, c.B, a)
+                   : launch_coop(k_small_step<DIM, true, 0, L>, c.sms, threads, st, c.k, c.F, c.B, a);
+    return fbm ? launch_coop(k_small_step<DIM, false, 2, L>, c.sms, threads, st, c.k, c.F, c.B, a)
+               : launch_coop(k_small_step<DIM, false, 0, L>, c.sms, threads, st, c.k, c.F, c.B, a);
 }
 
 }  // namespace tsph

@@ -1,0 +1,6 @@
+// The one-launch step in 3D with 8 lanes per particle.
+#include "small.cuh"
+
+namespace tsph {
+template cudaError_t launch_small_lanes<3, 8>(tsph_ctx &, const SmallArgs &, int, cudaStream_t);
+}  // namespace tsph

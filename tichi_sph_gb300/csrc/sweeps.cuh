@@ -192,6 +192,38 @@ __device__ __forceinline__ bool density_does_psi(const SceneConst &c, double com
     return c.f_n > 0 && ((0 < c.iter_min) || (compression > (double)c.div_tol));
 }
 
+// The results of the density sweep of one particle from its sums; returns its share
+// of the scene's psi_sum (0 without psi0).
+__device__ __forceinline__ double density_store(const KConst &k, const FluidBuf &F, int sc, int cur, bool psi0,
+                                                float4 pi, const DensAcc &a, int64_t s) {
+    const float4 mp = F.mpsi[s];
+    float alpha = __fmaf_rn(a.a1z, a.a1z, __fmaf_rn(a.a1y, a.a1y, __fmul_rn(a.a1x, a.a1x))) / mp.x + a.a2;
+    if (alpha < 1e-4f) alpha = 1e-4f;
+    // the compensated sums rounded once; psi keeps the remainder as its low part
+    const float rho_f = __fadd_rn(a.rho, a.rho_e), comp_f = __fadd_rn(a.comp, a.comp_e);
+    const float psi = k.vfsph ? comp_f : rho_f;
+    const float psilo = k.vfsph ? __fsub_rn(a.comp_e, __fsub_rn(comp_f, a.comp))
+                                : __fsub_rn(a.rho_e, __fsub_rn(rho_f, a.rho));
+    F.dens[s] = make_float4(a.wsum, rho_f, comp_f, a.a2);
+    F.a1[s] = make_float4(a.a1x, a.a1y, a.a1z, alpha);  // w: alpha again, for the write-back
+    F.psilo[s] = psilo;
+    F.mpsi[s] = make_float4(mp.x, psi, mp.z, alpha);
+    // psi also rides in the current v_adv's unused w (the velocity sweeps carry
+    // it along), so the advection sweep gets it with the neighbour's v_adv
+    F.vadv[(int64_t)cur * F.cap + s].w = psi;
+    if (psi0) {
+        // IPPE_adv_psi_init + IPPE_psi_adv_non_negative, as k_psi
+        float pa = ((psi - mp.z) + psilo) + a.pacc * k.sp[sc].dt;
+        if (pa < 0.f) pa = 0.f;
+        const float kap = pa / alpha;
+        F.psiadv[s] = pa;
+        F.kappa[s] = kap;
+        F.pk[s] = make_float4(pi.x, pi.y, pi.z, kap);
+        return (double)(pa / mp.z);
+    }
+    return 0.0;
+}
+
 // Returns the particle's share of the scene's psi_sum (0 without psi0).
 template <int DIM, bool M, bool R1, bool NC>
 __device__ __forceinline__ double density_fluid_item(const KConst &k, const FluidBuf &F, const BoundBuf &B, int sc,
@@ -263,32 +295,7 @@ __device__ __forceinline__ double density_fluid_item(const KConst &k, const Flui
         density_exact<DIM, M, NC>(k, F, B, sc, cur, s, psi0, e);
         a = e;
     }
-    const float4 mp = F.mpsi[s];
-    float alpha = __fmaf_rn(a.a1z, a.a1z, __fmaf_rn(a.a1y, a.a1y, __fmul_rn(a.a1x, a.a1x))) / mp.x + a.a2;
-    if (alpha < 1e-4f) alpha = 1e-4f;
-    // the compensated sums rounded once; psi keeps the remainder as its low part
-    const float rho_f = __fadd_rn(a.rho, a.rho_e), comp_f = __fadd_rn(a.comp, a.comp_e);
-    const float psi = k.vfsph ? comp_f : rho_f;
-    const float psilo = k.vfsph ? __fsub_rn(a.comp_e, __fsub_rn(comp_f, a.comp))
-                                : __fsub_rn(a.rho_e, __fsub_rn(rho_f, a.rho));
-    F.dens[s] = make_float4(a.wsum, rho_f, comp_f, a.a2);
-    F.a1[s] = make_float4(a.a1x, a.a1y, a.a1z, alpha);  // w: alpha again, for the write-back
-    F.psilo[s] = psilo;
-    F.mpsi[s] = make_float4(mp.x, psi, mp.z, alpha);
-    // psi also rides in the current v_adv's unused w (the velocity sweeps carry
-    // it along), so the advection sweep gets it with the neighbour's v_adv
-    F.vadv[(int64_t)cur * F.cap + s].w = psi;
-    if (psi0) {
-        // IPPE_adv_psi_init + IPPE_psi_adv_non_negative, as k_psi
-        float pa = ((psi - mp.z) + psilo) + a.pacc * k.sp[sc].dt;
-        if (pa < 0.f) pa = 0.f;
-        const float kap = pa / alpha;
-        F.psiadv[s] = pa;
-        F.kappa[s] = kap;
-        F.pk[s] = make_float4(pi.x, pi.y, pi.z, kap);
-        return (double)(pa / mp.z);
-    }
-    return 0.0;
+    return density_store(k, F, sc, cur, psi0, pi, a, s);
 }
 
 // The boundary's own sums: SPH_prepare_attr (b,b)(b,f), SPH_prepare_alpha_2 (b,f),
@@ -367,6 +374,19 @@ __device__ __forceinline__ void density_bound_item(const KConst &k, const FluidB
 }
 
 // ----------------------------------------------------------------------------- solver
+// IPPE_adv_psi_init + IPPE_psi_adv_non_negative of one particle from its pair sum;
+// returns its share of the scene's psi_sum.
+__device__ __forceinline__ double psi_store(const FluidBuf &F, float4 pi, float4 mp, float psilo, float dt, float acc,
+                                            int64_t s) {
+    float psi = ((mp.y - mp.z) + psilo) + acc * dt;
+    if (psi < 0.f) psi = 0.f;
+    const float kap = psi / mp.w;
+    F.psiadv[s] = psi;
+    F.kappa[s] = kap;
+    F.pk[s] = make_float4(pi.x, pi.y, pi.z, kap);
+    return (double)(psi / mp.z);
+}
+
 // Sweep A of one particle (the TPP lanes of ln): psi_adv and kappa; returns its
 // share of the scene's psi_sum (in the particle's first lane).
 template <int DIM, int TPP, bool M, bool NC>
@@ -404,18 +424,19 @@ __device__ __forceinline__ double psi_item(const KConst &k, const FluidBuf &F, c
             [&](int j, auto listed) { term(B.pos, B.vadv, j, listed); });
     }
     acc = ln.sum(acc);
-    double contrib = 0.0;
-    if (act && ln.q == 0) {
-        const float4 mp = F.mpsi[s];
-        float psi = ((mp.y - mp.z) + F.psilo[s]) + acc * k.sp[sc].dt;
-        if (psi < 0.f) psi = 0.f;
-        const float kap = psi / mp.w;
-        F.psiadv[s] = psi;
-        F.kappa[s] = kap;
-        F.pk[s] = make_float4(pi.x, pi.y, pi.z, kap);
-        contrib = (double)(psi / mp.z);
-    }
-    return contrib;
+    return act && ln.q == 0 ? psi_store(F, pi, F.mpsi[s], F.psilo[s], k.sp[sc].dt, acc, s) : 0.0;
+}
+
+// m: mass, vi: the current v_adv.
+__device__ __forceinline__ void vel_store(const FluidBuf &F, int cur, float4 pi, float ki, float4 a1, float m,
+                                          float4 vi, float dt, float sx, float sy, float sz, int64_t s) {
+    const float Xi = pi.w;
+    // (written out: wherever it is inlined, the same products are fused)
+    const float ax = __fmaf_rn(Xi, sx, __fmul_rn(ki, a1.x)), ay = __fmaf_rn(Xi, sy, __fmul_rn(ki, a1.y)),
+                az = __fmaf_rn(Xi, sz, __fmul_rn(ki, a1.z));
+    float4 *vout = F.vadv + (1 - cur) * F.cap;
+    const float sc_ = -(1.f / dt) / m;
+    vout[s] = make_float4(vi.x + sc_ * ax, vi.y + sc_ * ay, vi.z + sc_ * az, vi.w);  // w: psi
 }
 
 // Sweep B of one particle (the TPP lanes of ln), into the other v_adv buffer.
@@ -456,19 +477,18 @@ __device__ __forceinline__ void vel_item(const KConst &k, const FluidBuf &F, con
     sx = ln.sum(sx);
     sy = ln.sum(sy);
     sz = ln.sum(sz);
-    if (act && ln.q == 0) {
-        const float ki = F.kappa[s], Xi = pi.w;
-        const float4 a1 = F.a1[s];
-        const float ax = ki * a1.x + Xi * sx, ay = ki * a1.y + Xi * sy, az = ki * a1.z + Xi * sz;
-        const float4 *vin = F.vadv + cur * F.cap;
-        float4 *vout = F.vadv + (1 - cur) * F.cap;
-        const float sc_ = -(1.f / k.sp[sc].dt) / F.mpsi[s].x;
-        const float4 vi = vin[s];
-        vout[s] = make_float4(vi.x + sc_ * ax, vi.y + sc_ * ay, vi.z + sc_ * az, vi.w);  // w: psi
-    }
+    if (act && ln.q == 0)
+        vel_store(F, cur, pi, F.kappa[s], F.a1[s], F.mpsi[s].x, F.vadv[cur * F.cap + s], k.sp[sc].dt, sx, sy, sz, s);
 }
 
 // ----------------------------------------------------------------------------- advection
+__device__ __forceinline__ void normal_store(const FluidBuf &F, const Geo &g, float nx, float ny, float nz,
+                                             int64_t s) {
+    // w: what the surface-tension pass reads of a neighbour beside its normal
+    const float w = F.vf[s] > 0.99f ? F.mpsi[s].y : __uint_as_float(kNoSurfTension);
+    F.normal[s] = make_float4(nx * g.h, ny * g.h, nz * g.h, w);
+}
+
 // First pass of SPH_advection_surface_tension_acc, sph.py:134-150: surface normals.
 template <int DIM, int TPP, bool M, bool NC>
 __device__ __forceinline__ void normal_item(const KConst &k, const FluidBuf &F, const BoundBuf &B,
@@ -502,11 +522,22 @@ __device__ __forceinline__ void normal_item(const KConst &k, const FluidBuf &F, 
     nx = ln.sum(nx);
     ny = ln.sum(ny);
     nz = ln.sum(nz);
-    if (act && ln.q == 0) {
-        // w: what the surface-tension pass reads of a neighbour beside its normal
-        const float w = F.vf[s] > 0.99f ? F.mpsi[s].y : __uint_as_float(kNoSurfTension);
-        F.normal[s] = make_float4(nx * g.h, ny * g.h, nz * g.h, w);
-    }
+    if (act && ln.q == 0) normal_store(F, g, nx, ny, nz, s);
+}
+
+template <int DIM>
+__device__ __forceinline__ void advect_store(const KConst &k, const FluidBuf &F, int sc, const SceneConst &c, int cur,
+                                             float4 vi, float vx, float vy, float vz, float sx, float sy, float sz,
+                                             float gs, float vs, int64_t s) {
+    float4 *vout = F.vadv + (1 - cur) * F.cap;
+    const float dt = k.sp[sc].dt;
+    const float mu = (c.mu * vs) / F.rho0[s];
+    const float ax = c.g[0] * gs + vx * mu + sx;
+    const float ay = c.g[1] * gs + vy * mu + sy;
+    const float az = (DIM == 3 ? c.g[2] * gs : 0.f) + vz * mu + sz;
+    F.acc[s] = make_float4(ax, ay, az, 0.f);
+    F.vel[s] = vi;
+    vout[s] = make_float4(vi.x + ax * dt, vi.y + ay * dt, vi.z + az * dt, 0.f);
 }
 
 // SPH_vel_adv_2_vel + SPH_advection_gravity_acc + SPH_advection_viscosity_acc
@@ -641,17 +672,7 @@ __device__ __forceinline__ void advect_item(const KConst &k, const FluidBuf &F, 
         sy = ln.sum(sy);
         sz = ln.sum(sz);
     }
-    if (act && ln.q == 0) {
-        float4 *vout = F.vadv + (1 - cur) * F.cap;
-        const float dt = k.sp[sc].dt;
-        const float mu = (c.mu * vs) / F.rho0[s];
-        const float ax = c.g[0] * gs + vx * mu + sx;
-        const float ay = c.g[1] * gs + vy * mu + sy;
-        const float az = (DIM == 3 ? c.g[2] * gs : 0.f) + vz * mu + sz;
-        F.acc[s] = make_float4(ax, ay, az, 0.f);
-        F.vel[s] = vi;
-        vout[s] = make_float4(vi.x + ax * dt, vi.y + ay * dt, vi.z + az * dt, 0.f);
-    }
+    if (act && ln.q == 0) advect_store<DIM>(k, F, sc, c, cur, vi, vx, vy, vz, sx, sy, sz, gs, vs, s);
 }
 
 }  // namespace tsph
