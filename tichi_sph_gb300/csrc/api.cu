@@ -476,6 +476,7 @@ int create_impl(const tsph_params *ps, int S, const int64_t *fn, const int64_t *
     F.facc = A.get<float4>(fcap);
     F.zeta = A.get<float>(fcap);
     F.flagpass = A.get<int>(fcap);
+    F.redo = ps[0].fbm_enabled ? A.get<int>(2 * fcap) : nullptr;
     F.nbr = A.get<int>((long long)k.nbr_max * fcap);
     F.pk = A.get<float4>(fcap);
     F.nbr_cnt = A.get<unsigned int>(fcap);

@@ -201,6 +201,7 @@ struct FluidBuf {
     float4 *facc;            // acce (fbm_acce)
     float *zeta;
     int *flagpass;           // 0 = unflagged, else the FBM pass that flagged it
+    int *redo;               // [2][cap]: by parity, the pass that must sum the particle's fluxes again
     // Neighbours with 0 < r < h, recorded by the density sweep in candidate order:
     // first the fluid neighbours of sorted particle s, then its boundary ones, in
     // blocks of four: entry t sits at nbr[nbr_index(t, s, cap)], so block t / 4 of

