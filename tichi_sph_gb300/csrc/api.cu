@@ -265,6 +265,7 @@ int run_step(tsph_ctx *c, const tsph_set *f, const tsph_set *b, void *stream, bo
             return TSPH_OK;
         }
     }
+    c->scalars_on_host = 0;
     if (c->rec_tape) {
         rc = tape_begin(*c->rec_tape, c->rec_slot, st);
         if (rc) return rc;
@@ -871,8 +872,10 @@ int tsph_read_scene_stats(tsph_ctx *c, int first, int count, tsph_stats *out, vo
     if (!c || !out || first < 0 || count < 0 || first + count > c->n_scenes)
         return fail(TSPH_ERR_INVALID, "bad scene range");
     cudaStream_t st = (cudaStream_t)stream;
-    TSPH_CK(cudaMemcpyAsync(c->host_ss, c->k.ss, sizeof(SceneStep) * c->n_scenes, cudaMemcpyDeviceToHost, st));
-    TSPH_CK(cudaMemcpyAsync(c->host_sp, c->k.sp, sizeof(ScenePersist) * c->n_scenes, cudaMemcpyDeviceToHost, st));
+    if (!c->scalars_on_host) {
+        TSPH_CK(cudaMemcpyAsync(c->host_ss, c->k.ss, sizeof(SceneStep) * c->n_scenes, cudaMemcpyDeviceToHost, st));
+        TSPH_CK(cudaMemcpyAsync(c->host_sp, c->k.sp, sizeof(ScenePersist) * c->n_scenes, cudaMemcpyDeviceToHost, st));
+    }
     TSPH_CK(cudaStreamSynchronize(st));
     if (c->host_ss[0].status & kStGaveUp) {
         c->counts_zero = 0;
@@ -940,6 +943,7 @@ int tsph_profile_phases(tsph_ctx *c, const tsph_set *f, const tsph_set *b, int r
 
 int tsph_set_state(tsph_ctx *c, double time_count, float dt, double compression, void *stream) {
     if (!c) return fail(TSPH_ERR_INVALID, "null ctx");
+    c->scalars_on_host = 0;
     k_set_state<<<(c->n_scenes + 127) / 128, 128, 0, (cudaStream_t)stream>>>(c->k, time_count, dt, compression);
     TSPH_CK(cudaGetLastError());
     return TSPH_OK;

@@ -15,6 +15,7 @@ struct tsph_ctx {
     tsph::Scratch S;
     tsph::SmallScratch X;     // of the one-launch step
     int sms;                  // SMs of the device; 0: no cooperative launches
+    int scalars_on_host;      // host_ss / host_sp hold what the last enqueued work leaves on the device
     int counts_zero;          // the grids' counts and X's counters are zero (the one-launch step leaves them so)
     tsph::SceneConst *host_sc;  // host copy of the scene table (pinned)
     tsph::SceneStep *host_ss;   // pinned mirrors for host-loop mode and stats

@@ -362,6 +362,7 @@ void join_side(tsph_ctx &c, cudaStream_t st) {
 }
 
 void launch_step_begin(tsph_ctx &c, cudaStream_t st) {
+    c.scalars_on_host = 0;
     cudaMemsetAsync(c.k.ss, 0, sizeof(SceneStep) * c.k.n_scenes, st);
     cudaMemsetAsync(c.k.dg, 0, sizeof(DevGlobal), st);
 }
@@ -370,6 +371,7 @@ void launch_cfl(tsph_ctx &c, const tsph_set &f, cudaStream_t st) {
     int nb = blocks_for(f.n);
     if (nb < 1) nb = 1;
     if (nb > 4 * 152) nb = 4 * 152;
+    c.scalars_on_host = 0;
     c.launches += 1;
     if (c.k.dim == 3) TSPH_LAUNCH((k_cfl<3>), nb, kBlock, st, c.k, f.vel, f.n);
     else TSPH_LAUNCH((k_cfl<2>), nb, kBlock, st, c.k, f.vel, f.n);

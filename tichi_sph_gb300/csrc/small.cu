@@ -32,6 +32,8 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
     a.f = f;
     a.b = b;
     a.x = c.X;
+    a.host_st = c.host_ss;
+    a.host_sp = c.host_sp;
     a.with_cfl = with_cfl ? 1 : 0;
     a.st_on = c.st_on;
     a.wc = c.p.wcsph_enabled;
@@ -59,6 +61,7 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
         if (e != cudaSuccess) return e;
     }
     c.counts_zero = 1;
+    c.scalars_on_host = cap == cudaStreamCaptureStatusNone;
     const bool d3 = c.k.dim == 3;
     switch (lanes) {
         case 8: return d3 ? launch_small_lanes<3, 8>(c, a, threads, st) : launch_small_lanes<2, 8>(c, a, threads, st);

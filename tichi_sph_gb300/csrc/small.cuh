@@ -27,6 +27,8 @@ namespace tsph {
 struct SmallArgs {
     tsph_set f, b;
     SmallScratch x;
+    SceneStep *host_st;  // pinned host copies of the scalars
+    ScenePersist *host_sp;
     TapeArrays tape;
     float *density_out;  // not null: only the grid and the densities (in the caller's order), no step
     int slot;            // of the tape
@@ -440,7 +442,10 @@ struct SmallStep {
         return true;
     }
 
-    // The last block to leave: the energies, the running totals, the barrier's reset.
+    // The last block to leave: the energies, the running totals, the barrier's reset,
+    // and the scalars' copies in pinned host memory, so that a caller who reads them
+    // after every substep waits for the kernel alone (two small copies behind it
+    // cost a time loop about 25 us a substep).
     __device__ __forceinline__ void leave(bool done) {
         if (!last_block_done(a.x.bar + kBarLeft, gridDim.x)) return;
         double ke = 0.0, pe = 0.0;
@@ -450,17 +455,23 @@ struct SmallStep {
         }
         ke = coop_sum256(ke, sh_d);
         pe = coop_sum256(pe, sh_d);
-        if (threadIdx.x != 0) return;
-        if (done && !__ldcg(a.x.bar + kBarGaveUp)) {
-            if (!a.density_out) {
-                st().kinetic_energy = ke;
-                st().potential_energy = pe;
-                step_totals(k.sp[0], st());
+        if (threadIdx.x == 0) {
+            if (done && !__ldcg(a.x.bar + kBarGaveUp)) {
+                if (!a.density_out) {
+                    st().kinetic_energy = ke;
+                    st().potential_energy = pe;
+                    step_totals(k.sp[0], st());
+                }
+            } else {
+                atomicOr(&st().status, kStGaveUp);
             }
-        } else {
-            atomicOr(&st().status, kStGaveUp);
+            a.x.bar[kBarCount] = a.x.bar[kBarGaveUp] = a.x.bar[kBarLeft] = 0;
         }
-        a.x.bar[kBarCount] = a.x.bar[kBarGaveUp] = a.x.bar[kBarLeft] = 0;
+        __syncthreads();
+        // the scalars, to their host copies
+        const int i = threadIdx.x, ns4 = (int)(sizeof(SceneStep) / 4), np4 = (int)(sizeof(ScenePersist) / 4);
+        if (i < ns4) reinterpret_cast<int *>(a.host_st)[i] = __ldcg(reinterpret_cast<const int *>(k.ss) + i);
+        if (i < np4) reinterpret_cast<int *>(a.host_sp)[i] = __ldcg(reinterpret_cast<const int *>(k.sp) + i);
     }
 };
 

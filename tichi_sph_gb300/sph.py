@@ -47,14 +47,28 @@ context; the particle arrays hold the previous step's values until the update
 group has run.  A step composed in ``main.py``'s order equals the fused
 ``sph_step`` bit for bit (the same kernels in the same order).
 """
+import contextlib
+import struct
+
 import torch
 
 from . import _native
 from ._native import check
 
+# tsph_stats as one struct (no padding between its fields)
+_STATS_NAMES = [k for k, _ in _native.Stats._fields_]
+_STATS_FORMAT = struct.Struct("=5d8i3qd4i")
+assert _STATS_FORMAT.size == _native.C.sizeof(_native.Stats)
+_HERE = contextlib.nullcontext()
+
 
 def _stream_handle(device):
     return torch.cuda.current_stream(device).cuda_stream
+
+
+def _on(device):
+    """``torch.cuda.device(device)``, at no cost where it is the current one."""
+    return _HERE if device.index in (None, torch.cuda.current_device()) else torch.cuda.device(device)
 
 
 class Solver:
@@ -148,7 +162,7 @@ class Solver:
     def substep(self):
         """cfl_condition + clock + sph_step (main.py:348-350) as one graph launch."""
         f, b = self._sets()
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(self._lib.tsph_substep(self.ctx, f, b, _native.C.c_void_p(_stream_handle(self.device))),
                   "tsph_substep")
 
@@ -222,7 +236,7 @@ class Solver:
         """Synchronises and returns the step's scalars; also refreshes the
         reference-visible scalars (``config.dt[None]``, ``fluid.compression[None]``,
         ``fluid.statistics_*_energy[None]``, ``fluid.general_flag[None]``)."""
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             check(self._lib.tsph_read_stats(self.ctx, _native.C.byref(self._stats),
                                             _native.C.c_void_p(_stream_handle(self.device))), "tsph_read_stats")
         s = self._stats
@@ -232,7 +246,7 @@ class Solver:
         self.fluid.statistics_kinetic_energy[None] = s.kinetic_energy
         self.fluid.statistics_gravity_potential_energy[None] = s.potential_energy
         self.fluid.general_flag[None] = s.general_flag
-        return {k: getattr(s, k) for k, _ in _native.Stats._fields_}
+        return dict(zip(_STATS_NAMES, _STATS_FORMAT.unpack_from(s)))
 
     def profile_phases(self, reps=10):
         """Mean milliseconds per launch of each step phase (CUDA events on the
