@@ -124,3 +124,114 @@ def test_recorded_substep_and_its_reverse(dim, n, nb, gamma):
     assert torch.equal(p0, p1)
     for x, y in zip(g0, g1):
         assert float((x - y).abs().max()) <= 1e-4 * max(float(y.abs().max()), 1e-30)
+
+
+def _same(a, b):
+    for oa, ob in ((a.fluid, b.fluid), (a.bound, b.bound)):
+        for f in FIELDS:
+            x, y = getattr(oa, f), getattr(ob, f)
+            assert torch.equal(torch.nan_to_num(x.double()), torch.nan_to_num(y.double())), f
+
+
+def test_after_a_step_of_another_size():
+    """A step too large for one launch leaves other counters behind, also when its
+    graph is a cached one: the one-launch steps between such steps are those of
+    separate kernels, bit for bit."""
+    _need_cuda()
+    from tichi_sph_gb300 import Fluid, Solver, sph_config
+    side, few = 137, 90   # 137^3 boundary particles: too many for one launch
+    cfg_d, scen, _ = _scene(3, 6)
+    scen["sim_env"]["sim_space_rt"] = [(side + 3) * H] * 3
+    rng = np.random.default_rng(5)
+    ax = (np.arange(side) + 1.4) * H
+    lattice = np.stack(np.meshgrid(ax, ax, ax, indexing="ij"), -1).reshape(-1, 3).astype(np.float32)
+    cloud = rng.uniform(2 * H, 12 * H, (700, 3)).astype(np.float32)
+    runs = []
+    for use_graph in (True, False):
+        cfg = sph_config.Config(cfg_d, scen)
+        sets = []
+        for uid, pos in enumerate((cloud, lattice)):
+            o = Fluid(len(pos), cfg, uid, device="cuda")
+            o.part_num[None] = len(pos)
+            o.pos[:] = torch.as_tensor(pos, device="cuda")
+            o.volume_frac[:] = 1.0
+            o.rest_volume[:] = float(cfg.part_size[3])
+            o.update_mass_all()
+            sets.append(o)
+        s = Solver(cfg, sets[0], sets[1], use_graph=use_graph)
+        launches = []
+        for n in (few, len(lattice), few, len(lattice), few):
+            sets[1].part_num[None] = n
+            s.substep()
+            launches.append(s.stats()["launches_per_step"])
+        if use_graph:
+            assert [x == 1 for x in launches] == [True, False, True, False, True]
+        runs.append(s)
+    _same(*runs)
+    for s in runs:
+        s.close()
+
+
+def test_after_a_replay_of_captured_calls():
+    """Phase calls in a caller's graph change the context's counters and scalars at
+    each replay: the steps and scalars that follow are those of direct calls."""
+    _need_cuda()
+    from tichi_sph_gb300 import _native
+
+    def phases(s):
+        s.grid_build()
+        s.density_alpha()
+        for kind in (_native.SOLVE_DIV, _native.SOLVE_DENS):
+            for _ in range(2):
+                s.adv_psi(kind, read=False)
+                s.update_vel_adv(kind)
+            if kind == _native.SOLVE_DIV:
+                s.nonpressure()
+        s.update()
+
+    runs, scalars = [], []
+    for captured in (True, False):
+        s = _solver(3, 900, 300, False, True)
+        s.substep()
+        got = [s.stats()]
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                phases(s)
+        for _ in range(2):
+            s.substep()
+            if captured:
+                graph.replay()
+            else:
+                phases(s)
+            got.append(s.stats())
+            s.substep()
+            got.append(s.stats())
+        runs.append(s)
+        scalars.append(got)
+    for x, y in zip(*scalars):
+        for k in SCALARS:
+            assert x[k] == y[k] or (x[k] != x[k] and y[k] != y[k]), k
+    _same(*runs)
+    for s in runs:
+        s.close()
+
+
+def test_two_scenes_on_two_streams():
+    """One-launch steps of two contexts, enqueued on two streams without waiting for
+    one another, are those of each context alone."""
+    _need_cuda()
+    runs = []
+    for streams in ([torch.cuda.Stream(), torch.cuda.Stream()], [torch.cuda.current_stream()] * 2):
+        ss = [_solver(3, 900, 300, False, True), _solver(2, 700, 90, True, True)]
+        torch.cuda.synchronize()
+        for _ in range(20):
+            for s, q in zip(ss, streams):
+                with torch.cuda.stream(q):
+                    s.substep()
+        torch.cuda.synchronize()
+        runs.append(ss)
+    for a, b in zip(*runs):
+        _same(a, b)
+        a.close()
+        b.close()

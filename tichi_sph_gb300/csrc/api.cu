@@ -234,11 +234,24 @@ int bind_sets(tsph_ctx *c, const tsph_set *f, const tsph_set *b) {
     return TSPH_OK;
 }
 
+// Whether the caller captures `st`.  From then on what the context's flags say of the
+// device (scalars_on_host, counts_zero) may change by a replay, unseen: they
+// stay off for good.
+bool capturing(tsph_ctx *c, cudaStream_t st) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) (void)cudaGetLastError();
+    if (cap == cudaStreamCaptureStatusNone) return false;
+    c->captured = 1;
+    c->scalars_on_host = c->counts_zero = 0;
+    return true;
+}
+
 // The step (or, with density_out, its first part) as one cooperative launch, where
-// the sets take it (`taken`).
+// the sets take it (`taken`); a captured call keeps the separate launches (a
+// captured step fails there with the graph's launch, as one of any size).
 int small_step(tsph_ctx *c, const tsph_set *f, const tsph_set *b, bool with_cfl, float *density_out, cudaStream_t st,
                bool &taken) {
-    taken = small_step_fits(*c, *f, *b);
+    taken = c->use_graph && !capturing(c, st) && small_step_fits(*c, *f, *b);
     if (!taken) return TSPH_OK;
     const cudaError_t e = launch_small_step(*c, *f, *b, with_cfl, density_out, st);
     if (e == cudaSuccess) return TSPH_OK;
@@ -254,18 +267,16 @@ int run_step(tsph_ctx *c, const tsph_set *f, const tsph_set *b, void *stream, bo
     int rc = bind_sets(c, f, b);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    if (c->use_graph) {
-        bool taken;
-        rc = small_step(c, f, b, with_cfl, nullptr, st, taken);
-        if (rc) return rc;
-        if (taken) {
-            c->launches_per_step = 1;
-            c->launches_per_iter = c->launches_per_pass = 0;
-            c->stepped++;
-            return TSPH_OK;
-        }
+    bool taken;
+    rc = small_step(c, f, b, with_cfl, nullptr, st, taken);
+    if (rc) return rc;
+    if (taken) {
+        c->launches_per_step = 1;
+        c->launches_per_iter = c->launches_per_pass = 0;
+        c->stepped++;
+        return TSPH_OK;
     }
-    c->scalars_on_host = 0;
+    c->scalars_on_host = c->counts_zero = 0;  // (a cached graph comes by no launcher that says so)
     if (c->rec_tape) {
         rc = tape_begin(*c->rec_tape, c->rec_slot, st);
         if (rc) return rc;
@@ -304,8 +315,12 @@ int run_step(tsph_ctx *c, const tsph_set *f, const tsph_set *b, void *stream, bo
             return fail_cuda(e, "cudaGraphInstantiate");
         }
         std::memcpy(c->graph_key[gi], key, sizeof(key));
+        c->graph_launches[gi] = c->launches_per_step;
     }
     TSPH_CK(cudaGraphLaunch(exec, st));
+    c->launches_per_step = c->graph_launches[gi];
+    c->launches_per_iter = 2;
+    c->launches_per_pass = 1;
     c->stepped++;
     return TSPH_OK;
 }
@@ -666,6 +681,7 @@ int tsph_set_threads_per_particle(tsph_ctx *c, int tpp) {
 int tsph_cfl_condition(tsph_ctx *c, const tsph_set *f, void *stream) {
     if (!c || !f) return fail(TSPH_ERR_INVALID, "null argument");
     cudaStream_t st = (cudaStream_t)stream;
+    (void)capturing(c, st);
     TSPH_CK(cudaMemsetAsync(c->k.dg->ticket, 0, sizeof(unsigned int), st));
     launch_cfl(*c, *f, st);
     TSPH_CK(cudaGetLastError());
@@ -684,8 +700,9 @@ int tsph_substep(tsph_ctx *c, const tsph_set *f, const tsph_set *b, void *stream
 // The phases of enqueue_step one call at a time; the caller runs the solver and
 // volume-fraction loops on the host, as main.py:199-250 does.
 
-static int kl_check(tsph_ctx *c, const char *what) {
+static int kl_check(tsph_ctx *c, const char *what, void *stream) {
     if (!c) return fail(TSPH_ERR_INVALID, "null ctx");
+    (void)capturing(c, (cudaStream_t)stream);
     if (c->n_scenes != 1) {
         std::snprintf(g_last_error, sizeof(g_last_error), "%s: kernel-level calls take a one-scene context", what);
         return TSPH_ERR_INVALID;
@@ -707,7 +724,7 @@ static int kl_read_step(tsph_ctx *c, cudaStream_t st) {
 }
 
 int tsph_grid_build(tsph_ctx *c, const tsph_set *f, const tsph_set *b, void *stream) {
-    int rc = kl_check(c, "tsph_grid_build");
+    int rc = kl_check(c, "tsph_grid_build", stream);
     if (rc) return rc;
     rc = bind_sets(c, f, b);
     if (rc) return rc;
@@ -722,7 +739,7 @@ int tsph_grid_build(tsph_ctx *c, const tsph_set *f, const tsph_set *b, void *str
 }
 
 int tsph_density_alpha(tsph_ctx *c, void *stream) {
-    int rc = kl_check(c, "tsph_density_alpha");
+    int rc = kl_check(c, "tsph_density_alpha", stream);
     if (rc) return rc;
     if (c->kl_phase != 1) return kl_state("tsph_density_alpha", "it follows tsph_grid_build");
     cudaStream_t st = (cudaStream_t)stream;
@@ -744,7 +761,7 @@ static int kl_solve_phase(tsph_ctx *c, int kind, const char *what) {
 }
 
 int tsph_adv_psi(tsph_ctx *c, int kind, double *compression_out, void *stream) {
-    int rc = kl_check(c, "tsph_adv_psi");
+    int rc = kl_check(c, "tsph_adv_psi", stream);
     if (rc) return rc;
     rc = kl_solve_phase(c, kind, "tsph_adv_psi");
     if (rc) return rc;
@@ -761,7 +778,7 @@ int tsph_adv_psi(tsph_ctx *c, int kind, double *compression_out, void *stream) {
 }
 
 int tsph_update_vel_adv(tsph_ctx *c, int kind, void *stream) {
-    int rc = kl_check(c, "tsph_update_vel_adv");
+    int rc = kl_check(c, "tsph_update_vel_adv", stream);
     if (rc) return rc;
     rc = kl_solve_phase(c, kind, "tsph_update_vel_adv");
     if (rc) return rc;
@@ -774,7 +791,7 @@ int tsph_update_vel_adv(tsph_ctx *c, int kind, void *stream) {
 
 int tsph_solve(tsph_ctx *c, int kind, double tol, int32_t it_min, int32_t it_max, int32_t *it_out, double *err_out,
                void *stream) {
-    int rc = kl_check(c, "tsph_solve");
+    int rc = kl_check(c, "tsph_solve", stream);
     if (rc) return rc;
     rc = kl_solve_phase(c, kind, "tsph_solve");
     if (rc) return rc;
@@ -810,7 +827,7 @@ int tsph_solve(tsph_ctx *c, int kind, double tol, int32_t it_min, int32_t it_max
 }
 
 int tsph_nonpressure(tsph_ctx *c, int32_t terms, void *stream) {
-    int rc = kl_check(c, "tsph_nonpressure");
+    int rc = kl_check(c, "tsph_nonpressure", stream);
     if (rc) return rc;
     if (c->kl_phase != 2) return kl_state("tsph_nonpressure", "it follows tsph_density_alpha and the divergence solve");
     if (terms & ~TSPH_TERM_ALL) return fail(TSPH_ERR_INVALID, "tsph_nonpressure: unknown TSPH_TERM_* bits");
@@ -824,7 +841,7 @@ int tsph_nonpressure(tsph_ctx *c, int32_t terms, void *stream) {
 }
 
 int tsph_wc_pressure(tsph_ctx *c, const tsph_set *b, void *stream) {
-    int rc = kl_check(c, "tsph_wc_pressure");
+    int rc = kl_check(c, "tsph_wc_pressure", stream);
     if (rc) return rc;
     if (!b) return fail(TSPH_ERR_INVALID, "null argument");
     if (!c->p.wcsph_enabled) return fail(TSPH_ERR_INVALID, "tsph_wc_pressure: the context has wcsph_enabled = 0");
@@ -836,7 +853,7 @@ int tsph_wc_pressure(tsph_ctx *c, const tsph_set *b, void *stream) {
 }
 
 int tsph_fbm_pass(tsph_ctx *c, int32_t *general_flag_out, void *stream) {
-    int rc = kl_check(c, "tsph_fbm_pass");
+    int rc = kl_check(c, "tsph_fbm_pass", stream);
     if (rc) return rc;
     if (!c->p.fbm_enabled) return fail(TSPH_ERR_INVALID, "tsph_fbm_pass: the context has fbm_enabled = 0");
     if (c->kl_phase < 3 || c->kl_phase > 5)
@@ -856,7 +873,7 @@ int tsph_fbm_pass(tsph_ctx *c, int32_t *general_flag_out, void *stream) {
 }
 
 int tsph_update(tsph_ctx *c, const tsph_set *f, const tsph_set *b, void *stream) {
-    int rc = kl_check(c, "tsph_update");
+    int rc = kl_check(c, "tsph_update", stream);
     if (rc) return rc;
     if (c->kl_phase < 2) return kl_state("tsph_update", "it ends a step begun by tsph_grid_build and tsph_density_alpha");
     rc = bind_sets(c, f, b);
@@ -943,6 +960,7 @@ int tsph_profile_phases(tsph_ctx *c, const tsph_set *f, const tsph_set *b, int r
 
 int tsph_set_state(tsph_ctx *c, double time_count, float dt, double compression, void *stream) {
     if (!c) return fail(TSPH_ERR_INVALID, "null ctx");
+    (void)capturing(c, (cudaStream_t)stream);
     c->scalars_on_host = 0;
     k_set_state<<<(c->n_scenes + 127) / 128, 128, 0, (cudaStream_t)stream>>>(c->k, time_count, dt, compression);
     TSPH_CK(cudaGetLastError());
@@ -972,7 +990,7 @@ int tsph_density_record(tsph_ctx *c, const tsph_set *f, const tsph_set *b, tsph_
     c->rec_tape = t;
     c->rec_slot = slot;
     bool taken = false;
-    if (c->use_graph) rc = small_step(c, f, b, false, out, st, taken);
+    rc = small_step(c, f, b, false, out, st, taken);
     if (!rc && !taken) rc = tape_begin(*t, slot, st);
     if (rc || taken) {
         c->rec_tape = nullptr;

@@ -17,6 +17,7 @@ struct tsph_ctx {
     int sms;                  // SMs of the device; 0: no cooperative launches
     int scalars_on_host;      // host_ss / host_sp hold what the last enqueued work leaves on the device
     int counts_zero;          // the grids' counts and X's counters are zero (the one-launch step leaves them so)
+    int captured;             // a caller has captured launches of this context
     tsph::SceneConst *host_sc;  // host copy of the scene table (pinned)
     tsph::SceneStep *host_ss;   // pinned mirrors for host-loop mode and stats
     tsph::ScenePersist *host_sp;
@@ -33,6 +34,7 @@ struct tsph_ctx {
     // array pointers and the recording tape
     cudaGraphExec_t exec[2];
     unsigned long long graph_key[2][4];
+    int graph_launches[2];    // their top-level kernels
     tsph_tape *rec_tape;      // non-null while a recorded step is enqueued
     int rec_slot;             // its tape slot
     int launches;             // kernel launches enqueued (counted by the launchers)

@@ -50,18 +50,14 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
     const int lanes = runs * 8 <= 32 ? 8 : runs * 4 <= 32 ? 4 : 1;
     const int64_t bruns = ((b.n + 31) / 32 + c.sms - 1) / c.sms;
     const int threads = coop_threads((runs * lanes + bruns) * c.sms, c.sms);
-    // the kernel leaves zero counters behind, other grid builds do not; a captured
-    // launch must not rely on what came before it
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(st, &cap);
-    if (!c.counts_zero || cap != cudaStreamCaptureStatusNone) {
+    // the kernel leaves zero counters behind, other grid builds do not
+    if (!c.counts_zero) {
         cudaError_t e = cudaMemsetAsync(c.F.count, 0, sizeof(int) * c.k.total_nodes, st);
         if (e == cudaSuccess) e = cudaMemsetAsync(c.B.count, 0, sizeof(int) * c.k.total_nodes, st);
         if (e == cudaSuccess) e = cudaMemsetAsync(c.X.bar + kBarTailF, 0, 4 * (kBarWords - kBarTailF), st);
         if (e != cudaSuccess) return e;
     }
-    c.counts_zero = 1;
-    c.scalars_on_host = cap == cudaStreamCaptureStatusNone;
+    c.counts_zero = c.scalars_on_host = !c.captured;
     const bool d3 = c.k.dim == 3;
     switch (lanes) {
         case 8: return d3 ? launch_small_lanes<3, 8>(c, a, threads, st) : launch_small_lanes<2, 8>(c, a, threads, st);
