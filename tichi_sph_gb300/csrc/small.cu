@@ -10,15 +10,20 @@ TSPH_SMALL(3, 1) TSPH_SMALL(3, 4) TSPH_SMALL(3, 8)
 #undef TSPH_SMALL
 
 // One-scene contexts on the default settings (the solver loops on the device, one
-// thread per particle) whose options the kernel has, up to 512 warps of
-// particles per SM.  What separate launches lose (about 90 us at 1M particles:
-// drained and refilled SMs, tail reductions, while nodes) shrinks beside the
-// work as scenes grow, and a fixed share of the particles per SM, 32 warps
-// resident, is the weaker schedule for the sweeps themselves.  Separate launches
-// and one launch, us per substep (fluid particles of a 3D dam break): 8k 235 / 154,
-// 27k 236 / 170, 99k 352 / 250, 205k 518 / 423, 343k 721 / 606, 1M 1619 / 1533,
-// 4.1M 5632 / 6185; in 2D 61k 189 / 111, 300k 406 / 274, 1M 928 / 865.
-constexpr int64_t kSmallWarpsPerSm = 512;
+// thread per particle) whose options the kernel has, up to 208 warps of
+// particles per SM (fluid and boundary together, a million particles).  What
+// separate launches lose (drained and refilled SMs, tail reductions, while
+// nodes) shrinks beside the work as scenes grow, while one launch gives every SM a
+// fixed share of the particles and 32 resident warps.  Once a flow has
+// developed, those shares are no longer equal work, and that decides at the top end.
+// Separate launches and one launch, us per substep (fluid particles of a 3D dam break,
+// boundary 567k): after 500 substeps 216k 523 / 479, 287k 656 / 529, 373k 718 / 671,
+// 439k 795 / 752, 512k 893 / 927, 1M 1467 / 1614; from rest 8k 235 / 154,
+// 27k 236 / 170, 99k 352 / 250, 205k 518 / 423, 439k 834 / 722, 1M 1595 / 1529,
+// 4.1M 5632 / 6185; in 2D 61k 189 / 111, 300k 409 / 292.  Shares dealt to the SMs in
+// groups of 256 particles instead: 1M 1530 after 500 substeps, but 1610 from rest
+// and 205k 424 -> 443 (neighbours no longer share an SM's L1).
+constexpr int64_t kSmallWarpsPerSm = 208;
 
 bool small_step_fits(const tsph_ctx &c, const tsph_set &f, const tsph_set &b) {
     if (c.n_scenes != 1 || c.batch || !c.sms || !c.scan_r1 || c.tpp != 1 || f.n < 1) return false;
