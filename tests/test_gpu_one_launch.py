@@ -62,9 +62,11 @@ def _solver(dim, n, nb, two, use_graph, gamma=0.0, inside=False):
 @pytest.mark.parametrize("dim,n,nb,two", [(2, 1, 0, False), (2, 33, 40, False), (2, 257, 0, True),
                                           (2, 700, 90, True), (3, 31, 1, False), (3, 256, 257, False),
                                           (3, 900, 300, True), (3, 5000, 700, False), (2, 21000, 500, True),
-                                          (3, 25000, 900, False), (2, 60000, 0, False)])
+                                          (3, 25000, 900, False), (2, 60000, 0, False),
+                                          (3, 156000, 700, False), (3, 467000, 300, True)])
 def test_one_launch_equals_separate_kernels(dim, n, nb, two):
-    # (above 19,456 particles four lanes of a warp share one, above 38,912 one has it)
+    # (above 19,456 particles four lanes of a warp share one, above 38,912 one has it;
+    # in 3D warps take runs from a queue above 155,648, of dealt groups from 466,944 on)
     _need_cuda()
     runs = []
     for use_graph in (True, False):

@@ -16,7 +16,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 BUILD = os.path.join(HERE, "_build")
 LIBDIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIBDIR, "libtichi_sph.so")
-SOURCES = ["small.cu", "small_2d_1.cu", "small_2d_4.cu", "small_2d_8.cu", "small_3d_1.cu", "small_3d_4.cu",
+SOURCES = ["small.cu", "small_2d_1.cu", "small_2d_4.cu", "small_2d_8.cu", "small_3d_1.cu", "small_3d_q.cu", "small_3d_4.cu",
            "small_3d_8.cu", "grid.cu", "sweeps.cu", "fbm.cu", "api.cu", "noalloc.cu", "adjoint.cu", "wcsph.cu", "measure.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", INCLUDE]

@@ -605,8 +605,8 @@ __global__ void __launch_bounds__(1024, 1) k_adj_step(const __grid_constant__ Sl
     auto sweep = [&](auto &&item) {
         const WarpShare w(v.n);
         const Lanes<TPP> ln;
-        for (int64_t i = threadIdx.x >> 5; i < w.count() * TPP; i += blockDim.x >> 5)
-            item(ln, (w.first * TPP + i) * ln.PPW + ln.p);
+        for (int64_t i = threadIdx.x >> 5; i < (int64_t)w.runs * TPP; i += blockDim.x >> 5)
+            item(ln, ((int64_t)w.first * TPP + i) * ln.PPW + ln.p);
     };
     auto own = [&](const Lanes<TPP> &ln, int64_t s) { return s < v.n && ln.q == 0; };
     auto solve = [&](int kind, int iters) {

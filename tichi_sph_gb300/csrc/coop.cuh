@@ -2,6 +2,7 @@
 // items, sums in the order of the separate kernels, the launch.
 #pragma once
 
+#include <type_traits>
 #include <utility>
 
 #include "ctx.h"
@@ -51,26 +52,78 @@ struct GridBarrier {
 // The block's share of n items: contiguous runs of 32, shares that differ by one
 // run at most.
 struct WarpShare {
-    int64_t first, last;  // runs [first, last)
+    unsigned int first, runs;
     __device__ __forceinline__ WarpShare(int64_t n) {
         const unsigned int nw = (unsigned int)((n + 31) >> 5), per = nw / gridDim.x, more = nw % gridDim.x;
-        first = (int64_t)blockIdx.x * per + min(blockIdx.x, more);
-        last = first + per + (blockIdx.x < more ? 1 : 0);
+        first = blockIdx.x * per + min(blockIdx.x, more);
+        runs = per + (blockIdx.x < more ? 1u : 0u);
     }
-    __device__ __forceinline__ int64_t count() const { return last - first; }
+    __device__ __forceinline__ unsigned int run(unsigned int w) const { return first + w; }
 };
 
-// Runs ff(i, warp) over the fluid's nf items and fb(i) over the boundary's nb in
-// the block's warps (every lane of a warp calls, i may be past the end).
-template <class FF, class FB>
-__device__ __forceinline__ void for_items(int64_t nf, int64_t nb, FF &&ff, FB &&fb) {
-    const WarpShare f(nf), b(nb);
-    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    const int64_t total = f.count() + b.count();
-    for (int64_t w = threadIdx.x >> 5; w < total; w += warps) {
-        if (w < f.count()) ff((f.first + w) * 32 + lane, f.first + w);
-        else fb((b.first + w - f.count()) * 32 + lane);
+// The block's share of n items where its warps take several runs each (QUEUE): up to
+// kDealt runs per block WarpShare's, whose neighbours share the SM's L1, from
+// there on groups of 16 neighbouring runs dealt to the blocks in turn.  Once a
+// flow has developed, a share that lies together is all surface or all interior, and
+// a sweep waits for the interior's (us a substep of a dam break after 500
+// substeps, together and dealt: 439k 706 / 716, 512k 849 / 809, 1M
+// 1535 / 1385; with groups of 8 the 1M step from rest takes 1610 instead of 1528).
+struct QueueShare {
+    static constexpr unsigned int kGroup = 16, kDealt = 96;
+    unsigned int first, runs, skip;  // skip: runs between the block's groups
+    __device__ __forceinline__ QueueShare(int64_t n) {
+        const unsigned int nw = (unsigned int)((n + 31) >> 5);
+        if (nw >= kDealt * gridDim.x) {
+            const unsigned int ng = (nw + kGroup - 1) / kGroup, per = ng / gridDim.x, more = ng % gridDim.x;
+            first = blockIdx.x * kGroup;
+            runs = (per + (blockIdx.x < more ? 1u : 0u)) * kGroup;
+            if ((ng - 1) % gridDim.x == blockIdx.x) runs -= ng * kGroup - nw;
+            skip = (gridDim.x - 1) * kGroup;
+        } else {
+            const WarpShare w(n);
+            first = w.first;
+            runs = w.runs;
+            skip = 0;
+        }
     }
+    // the block's w-th run
+    __device__ __forceinline__ unsigned int run(unsigned int w) const { return first + w + w / kGroup * skip; }
+};
+
+// What a block's warps take runs from: a count in shared memory, and its value at
+// the start of the phase (the same in every thread).
+struct RunQueue {
+    unsigned int *next;
+    unsigned int base;
+};
+
+// Runs ff(i, run) over the fluid's nf items and fb(i) over the boundary's nb in
+// the block's warps (every lane of a warp calls, i may be past the end).  With QUEUE
+// a warp takes its first run by its place and the others as it gets to them; two
+// calls are then a barrier of the block apart.
+template <bool QUEUE, class FF, class FB>
+__device__ __forceinline__ void for_items(RunQueue &q, int64_t nf, int64_t nb, FF &&ff, FB &&fb) {
+    using Share = std::conditional_t<QUEUE, QueueShare, WarpShare>;
+    const Share f(nf), b(nb);
+    const int lane = threadIdx.x & 31;
+    const unsigned int warps = blockDim.x >> 5, total = f.runs + b.runs;
+    for (unsigned int w = threadIdx.x >> 5; w < total;) {
+        if (w < f.runs) {
+            const int64_t r = f.run(w);
+            ff(r * 32 + lane, r);
+        } else {
+            fb((int64_t)b.run(w - f.runs) * 32 + lane);
+        }
+        if (!QUEUE) {
+            w += warps;
+        } else {
+            if (total <= warps) break;
+            if (lane == 0) w = warps + (atomicAdd(q.next, 1u) - q.base);
+            w = __shfl_sync(0xffffffffu, w, 0);
+        }
+    }
+    // (total - warps taken, and every warp once more in vain)
+    if (QUEUE && total > warps) q.base += total;
 }
 
 // The tree of block_sum over a 256-thread block's eight warp sums.

@@ -4,26 +4,24 @@
 
 namespace tsph {
 
-#define TSPH_SMALL(D, L) extern template cudaError_t launch_small_lanes<D, L>(tsph_ctx &, const SmallArgs &, int, cudaStream_t);
-TSPH_SMALL(2, 1) TSPH_SMALL(2, 4) TSPH_SMALL(2, 8)
-TSPH_SMALL(3, 1) TSPH_SMALL(3, 4) TSPH_SMALL(3, 8)
+#define TSPH_SMALL(D, L, Q) \
+    extern template cudaError_t launch_small_lanes<D, L, Q>(tsph_ctx &, const SmallArgs &, int, cudaStream_t);
+TSPH_SMALL(2, 1, false) TSPH_SMALL(2, 4, false) TSPH_SMALL(2, 8, false)
+TSPH_SMALL(3, 1, true) TSPH_SMALL(3, 1, false) TSPH_SMALL(3, 4, false) TSPH_SMALL(3, 8, false)
 #undef TSPH_SMALL
 
 // One-scene contexts on the default settings (the solver loops on the device, one
-// thread per particle) whose options the kernel has, up to 208 warps of
-// particles per SM (fluid and boundary together, a million particles).  What
-// separate launches lose (drained and refilled SMs, tail reductions, while
-// nodes) shrinks beside the work as scenes grow, while one launch gives every SM a
-// fixed share of the particles and 32 resident warps.  Once a flow has
-// developed, those shares are no longer equal work, and that decides at the top end.
-// Separate launches and one launch, us per substep (fluid particles of a 3D dam break,
-// boundary 567k): after 500 substeps 216k 523 / 479, 287k 656 / 529, 373k 718 / 671,
-// 439k 795 / 752, 512k 893 / 927, 1M 1467 / 1614; from rest 8k 235 / 154,
-// 27k 236 / 170, 99k 352 / 250, 205k 518 / 423, 439k 834 / 722, 1M 1595 / 1529,
-// 4.1M 5632 / 6185; in 2D 61k 189 / 111, 300k 409 / 292.  Shares dealt to the SMs in
-// groups of 256 particles instead: 1M 1530 after 500 substeps, but 1610 from rest
-// and 205k 424 -> 443 (neighbours no longer share an SM's L1).
-constexpr int64_t kSmallWarpsPerSm = 208;
+// thread per particle) whose options the kernel has, up to 512 warps of
+// particles per SM (fluid and boundary together).  What separate launches lose
+// (drained and refilled SMs, tail reductions, while nodes) shrinks beside the work
+// as scenes grow, while one launch has 32 warps resident per SM and a share of the
+// particles for each SM.  Separate launches and one launch, us per substep (fluid
+// particles of a 3D dam break): after 500 substeps 216k 515 / 442, 439k 795 / 716,
+// 512k 893 / 809, 1M 1464 / 1385, 2.1M (past the line) 2596 / 2550, 4.1M
+// 4546 / 4668; from rest 8k 235 / 154, 27k 236 / 170, 99k 352 / 250, 205k 514 / 424,
+// 1M 1595 / 1528, 2.1M 2963 / 2963, 4.1M 5567 / 5721; in 2D 61k 189 / 111, 300k after
+// 1,500 substeps 491 / 363, 900k 1430 / 1371.
+constexpr int64_t kSmallWarpsPerSm = 512;
 
 bool small_step_fits(const tsph_ctx &c, const tsph_set &f, const tsph_set &b) {
     if (c.n_scenes != 1 || c.batch || !c.sms || !c.scan_r1 || c.tpp != 1 || f.n < 1) return false;
@@ -53,6 +51,10 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
     // 93, 8k 155 / 95, 27k 177 / 143; in 2D, a third of the neighbours, 5k 132 / 122)
     const int64_t runs = ((f.n + kBlock - 1) / kBlock * (kBlock / 32) + c.sms - 1) / c.sms;
     const int lanes = runs * 8 <= 32 ? 8 : runs * 4 <= 32 ? 4 : 1;
+    // several runs a warp in 3D: taken from a queue (us a substep of a developed flow
+    // with fixed turns and with the queue: 216k 478 / 442, 439k 756 / 706, 1M
+    // 1614 / 1385; 205k from rest 425 / 424).  In 2D, with less work a run, it gave
+    // nothing: 300k 363 / 362, 900k 1371 / 1395.
     const int64_t bruns = ((b.n + 31) / 32 + c.sms - 1) / c.sms;
     const int threads = coop_threads((runs * lanes + bruns) * c.sms, c.sms);
     // the kernel leaves zero counters behind, other grid builds do not
@@ -65,9 +67,16 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
     c.counts_zero = c.scalars_on_host = !c.captured;
     const bool d3 = c.k.dim == 3;
     switch (lanes) {
-        case 8: return d3 ? launch_small_lanes<3, 8>(c, a, threads, st) : launch_small_lanes<2, 8>(c, a, threads, st);
-        case 4: return d3 ? launch_small_lanes<3, 4>(c, a, threads, st) : launch_small_lanes<2, 4>(c, a, threads, st);
-        default: return d3 ? launch_small_lanes<3, 1>(c, a, threads, st) : launch_small_lanes<2, 1>(c, a, threads, st);
+        case 8:
+            return d3 ? launch_small_lanes<3, 8, false>(c, a, threads, st)
+                      : launch_small_lanes<2, 8, false>(c, a, threads, st);
+        case 4:
+            return d3 ? launch_small_lanes<3, 4, false>(c, a, threads, st)
+                      : launch_small_lanes<2, 4, false>(c, a, threads, st);
+        default:
+            if (!d3) return launch_small_lanes<2, 1, false>(c, a, threads, st);
+            return runs > 32 ? launch_small_lanes<3, 1, true>(c, a, threads, st)
+                             : launch_small_lanes<3, 1, false>(c, a, threads, st);
     }
 }
 

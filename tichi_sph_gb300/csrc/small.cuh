@@ -88,14 +88,16 @@ __device__ __forceinline__ double small_psi_sum(const double *warp_sums, int64_t
 
 // P: phases of the volume-fraction update, 0 without it.  L: lanes per particle of
 // the neighbour sweeps (lanes.cuh); with more than one, a block's warps hold all of
-// its runs of 32 particles at a time (launch_small_step).
-template <int DIM, bool ST, int P, int L>
+// its runs of 32 particles at a time (launch_small_step).  Q: warps take runs from a
+// queue (for_items).
+template <int DIM, bool ST, int P, int L, bool Q>
 struct SmallStep {
     const KConst &k;
     const FluidBuf &F;
     const BoundBuf &B;
     const SmallArgs &a;
     GridBarrier bar;
+    RunQueue queue;
     double *sh_d;
     int *sh_i;
     int64_t ns;  // the fluid's slots in whole blocks of the separate kernels
@@ -228,7 +230,7 @@ struct SmallStep {
     template <bool SUM, class FN, class FB>
     __device__ __forceinline__ void lane_sweep(int64_t nb, FN &&f, FB &&fb) {
         if constexpr (L == 1) {
-            for_items(ns, nb, [&](int64_t s, int64_t w) {
+            for_items<Q>(queue, ns, nb, [&](int64_t s, int64_t w) {
                 const double v = f(Lanes<1>(), s);
                 if (SUM) put_warp_sum(v, w);
             }, fb);
@@ -240,20 +242,20 @@ struct SmallStep {
     __device__ __forceinline__ void lane_sweep_wide(int64_t nb, FN &&f, FB &&fb) {
         const WarpShare fl(ns), bo(nb);
         const Lanes<L> ln;
-        const int64_t mine = fl.count() * L, total = mine + bo.count();
+        const int64_t mine = (int64_t)fl.runs * L, total = mine + bo.runs;
         for (int64_t w = threadIdx.x >> 5; w < total; w += blockDim.x >> 5) {
             if (w < mine) {
                 const int64_t in = w * ln.PPW + ln.p;  // slot within the block's runs
-                const double v = f(ln, fl.first * 32 + in);
+                const double v = f(ln, (int64_t)fl.first * 32 + in);
                 if (SUM && ln.q == 0) sh_d[in] = v;
             } else {
-                fb((bo.first + w - mine) * 32 + (threadIdx.x & 31));
+                fb(((int64_t)bo.first + w - mine) * 32 + (threadIdx.x & 31));
             }
         }
         if (!SUM) return;
         __syncthreads();
-        for (int64_t r = threadIdx.x >> 5; r < fl.count(); r += blockDim.x >> 5)
-            put_warp_sum(sh_d[r * 32 + (threadIdx.x & 31)], fl.first + r);
+        for (int64_t r = threadIdx.x >> 5; r < (int64_t)fl.runs; r += blockDim.x >> 5)
+            put_warp_sum(sh_d[r * 32 + (threadIdx.x & 31)], (int64_t)fl.first + r);
     }
 
     // One pressure solve (k_solve_begin, k_psi, k_vel); psi_done: the first psi sweep
@@ -302,10 +304,10 @@ struct SmallStep {
     // The weakly compressible pressure block (k_wc_pressure, k_wc_acce).
     __device__ __forceinline__ bool weakly_compressible() {
         const SceneConst &c = k.s0;
-        for_items(c.f_n, c.b_n, [&](int64_t s, int64_t) { if (s < c.f_n) wc_pressure_fluid_item(F, c, s); },
+        for_items<Q>(queue, c.f_n, c.b_n, [&](int64_t s, int64_t) { if (s < c.f_n) wc_pressure_fluid_item(F, c, s); },
                   [&](int64_t s) { if (s < c.b_n) wc_pressure_bound_item(B, a.b.pressure, s); });
         if (!bar.sync()) return false;
-        for_items(c.f_n, 0, [&](int64_t s, int64_t) {
+        for_items<Q>(queue, c.f_n, 0, [&](int64_t s, int64_t) {
             if (s < c.f_n) wc_acce_item<DIM, false, false>(k, F, B, 0, c, st(), cur, s);
         }, [](int64_t) {});
         return bar.sync();
@@ -314,7 +316,7 @@ struct SmallStep {
     // The volume-fraction update (k_fbm_drift, k_fbm_begin, k_fbm_pass).
     __device__ __forceinline__ bool mixture() {
         const SceneConst &c = k.s0;
-        for_items(c.f_n, 0, [&](int64_t s, int64_t) {
+        for_items<Q>(queue, c.f_n, 0, [&](int64_t s, int64_t) {
             if (s >= c.f_n) return;
             F.flagpass[s] = 0;
             fbm_drift_item<DIM, P ? P : 1>(k, F, 0, c, cur, s);
@@ -324,7 +326,7 @@ struct SmallStep {
         bool flagged;
         do {
             ++pass;
-            for_items(c.f_n, 0, [&](int64_t s, int64_t) {
+            for_items<Q>(queue, c.f_n, 0, [&](int64_t s, int64_t) {
                 const bool neg = s < c.f_n && fbm_pass_item<DIM, P ? P : 1, false, false>(k, F, B, 0, c, st(), pass, s);
                 if (__any_sync(0xffffffffu, neg) && (threadIdx.x & 31) == 0) atomicMax(&st().general_flag, pass);
             }, [](int64_t) {});
@@ -344,7 +346,7 @@ struct SmallStep {
         const SceneConst &c = k.s0;
         largest_speed();
         int *ctr = reinterpret_cast<int *>(a.x.bar);
-        for_items(a.f.n, a.b.n,
+        for_items<Q>(queue, a.f.n, a.b.n,
             [&](int64_t i, int64_t) {
                 if (i < a.f.n) encode_item<DIM>(k, a.f, 0, F.count, F.slot, ctr + kBarTailF, ctr + kBarStatus, i);
             },
@@ -359,7 +361,7 @@ struct SmallStep {
         time_step();
         scan_cells();
         if (!bar.sync()) return false;
-        for_items(a.f.n, a.b.n,
+        for_items<Q>(queue, a.f.n, a.b.n,
             [&](int64_t i, int64_t) {
                 if (i < a.f.n) scatter_item(k, 0, a.f.neighb_cell_seq, F.slot, F.start, F.perm_u, i);
             },
@@ -368,7 +370,7 @@ struct SmallStep {
             });
         if (!bar.sync()) return false;
         clear_counts();
-        for_items(a.f.n, a.b.n,
+        for_items<Q>(queue, a.f.n, a.b.n,
                   [&](int64_t u, int64_t) { if (u < a.f.n) gather_fluid_item<DIM>(k, a.f, F, c, st(), u); },
                   [&](int64_t u) { if (u < a.b.n) gather_bound_item<DIM>(k, a.b, B, c, 0, u); });
         if (!bar.sync()) return false;
@@ -422,7 +424,7 @@ struct SmallStep {
         if (a.wc && !weakly_compressible()) return false;
         if (P && !mixture()) return false;
         double *en = a.x.sums;  // the solves' sums are done with
-        for_items(ns, a.b.n,
+        for_items<Q>(queue, ns, a.b.n,
             [&](int64_t pid, int64_t w) {
                 double ke = 0.0, pe = 0.0;
                 if (pid < c.f_n)
@@ -476,27 +478,32 @@ struct SmallStep {
 };
 
 // One block per SM; 64 registers let the largest block have 1,024 threads.
-template <int DIM, bool ST, int P, int L>
+template <int DIM, bool ST, int P, int L, bool Q>
 __global__ void __launch_bounds__(1024, 1) k_small_step(const __grid_constant__ KConst k,
                                                         const __grid_constant__ FluidBuf F,
                                                         const __grid_constant__ BoundBuf B,
                                                         const __grid_constant__ SmallArgs a) {
     __shared__ double sh_d[kSmallSums];
     __shared__ int sh_i[33];
-    SmallStep<DIM, ST, P, L> step{k, F, B, a, {a.x.bar, 0u}, sh_d, sh_i, (a.f.n + kBlock - 1) / kBlock * kBlock, 0};
+    __shared__ unsigned int sh_next;
+    if (Q) {
+        if (threadIdx.x == 0) sh_next = 0;
+        __syncthreads();
+    }
+    SmallStep<DIM, ST, P, L, Q> step{k, F, B, a, {a.x.bar, 0u}, {&sh_next, 0u}, sh_d, sh_i, (a.f.n + kBlock - 1) / kBlock * kBlock, 0};
     const bool done = step.run();
     step.leave(done);
 }
 
-// The instances with DIM and L (a translation unit each).
-template <int DIM, int L>
+// The instances with DIM, L and Q (a translation unit each).
+template <int DIM, int L, bool Q>
 cudaError_t launch_small_lanes(tsph_ctx &c, const SmallArgs &a, int threads, cudaStream_t st) {
     const bool fbm = c.p.fbm_enabled != 0;
     if (c.st_on)
-        return fbm ? launch_coop(k_small_step<DIM, true, 2, L>, c.sms, threads, st, c.k, c.F, c.B, a)
-                   : launch_coop(k_small_step<DIM, true, 0, L>, c.sms, threads, st, c.k, c.F, c.B, a);
-    return fbm ? launch_coop(k_small_step<DIM, false, 2, L>, c.sms, threads, st, c.k, c.F, c.B, a)
-               : launch_coop(k_small_step<DIM, false, 0, L>, c.sms, threads, st, c.k, c.F, c.B, a);
+        return fbm ? launch_coop(k_small_step<DIM, true, 2, L, Q>, c.sms, threads, st, c.k, c.F, c.B, a)
+                   : launch_coop(k_small_step<DIM, true, 0, L, Q>, c.sms, threads, st, c.k, c.F, c.B, a);
+    return fbm ? launch_coop(k_small_step<DIM, false, 2, L, Q>, c.sms, threads, st, c.k, c.F, c.B, a)
+               : launch_coop(k_small_step<DIM, false, 0, L, Q>, c.sms, threads, st, c.k, c.F, c.B, a);
 }
 
 }  // namespace tsph

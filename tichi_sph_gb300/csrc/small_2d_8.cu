@@ -2,5 +2,5 @@
 #include "small.cuh"
 
 namespace tsph {
-template cudaError_t launch_small_lanes<2, 8>(tsph_ctx &, const SmallArgs &, int, cudaStream_t);
+template cudaError_t launch_small_lanes<2, 8, false>(tsph_ctx &, const SmallArgs &, int, cudaStream_t);
 }  // namespace tsph
