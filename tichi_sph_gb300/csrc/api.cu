@@ -1,8 +1,9 @@
 // C ABI of the SPH hot path: context management and the per-substep schedule.
 //
 // The substep (run_step's body, main.py:348-352, around sph_step, main.py:175-256)
-// is captured once into a CUDA graph per (particle counts, array pointers) and
-// replayed.  Both data-dependent loops of the reference -- the two Jacobi solves
+// of one scene up to a size is one cooperative launch (small.cu has the rule).
+// Every other is captured once into a CUDA graph per (particle counts, array
+// pointers) and replayed.  Both data-dependent loops of the reference -- the two Jacobi solves
 // (main.py:201-213, 222-234) and the volume-fraction pass loop (main.py:244-248)
 // -- become device-side while nodes whose condition is set by the last block of
 // the loop body, so a substep runs without any host round trip.  The host-driven

@@ -1,11 +1,12 @@
-// Neighbour sweeps of one substep: density + alpha, the Jacobi pair of the two
-// pressure solves, and the advection forces (viscosity, surface tension).
+// Neighbour sweeps of one substep as separate kernels: density + alpha, the Jacobi
+// pair of the two pressure solves, and the advection forces (viscosity, surface
+// tension).  What a particle does in each is in sweeps.cuh.
 //
 // One thread (or TPP threads) per particle in cell-sorted order; a block never
 // straddles two scenes, so every block reads one scene's constants.  The
 // density sweep scans the (2r+1)^dim template rows of the fluid grid and, where
 // the reference pairs with the boundary set, of the boundary grid
-// (visit_candidates), and records every pair with 0 < r < h in the fluid
+// (visit_hits_r1 for radius 1, else visit_candidates), and records every pair with 0 < r < h in the fluid
 // particle's neighbour list.  The later sweeps of the step walk that list
 // (for_each_neighbor_tpp) -- about 30 entries instead of about 220 candidates in
 // 3D -- in the same order.  Per-particle sums are FP32 (the reference's
