@@ -761,7 +761,7 @@ def main():
                        "l2": "inputs larger than L2 (per-step state ~%d MB > 129 MB)" % round(400 * nf / 1e6),
                        "threads_per_particle": solver.tpp, "autotune_ms": tune,
                        "graph": "host-driven solver loops" if args.hostloop else
-                       "one CUDA graph per substep, device-side while nodes"},
+                       "one launch per substep (a cooperative kernel or a CUDA graph), solver loops on the device"},
             "roofline": roofline,
             "alu_roofline": alu,
             "cpu_baseline": cpu,
