@@ -260,13 +260,16 @@ struct SmallStep {
 
     // One pressure solve (k_solve_begin, k_psi, k_vel); psi_done: the first psi sweep
     // has run.  Every block makes the loop test from the compression that the
-    // last block derives while the others update velocities.
+    // last block derives while the others update velocities.  With psi_done the
+    // first test has been made, and held, before the barrier behind the density
+    // sweep; it is not made again here, where no barrier lies between it and the
+    // last block's new value.  Without, a psi sweep and its barrier do.
     __device__ __forceinline__ bool solve(int kind, bool psi_done) {
         const SceneConst &c = k.s0;
         const double tol = kind == kSolveDiv ? (double)c.div_tol : (double)c.comp_tol;
         const int slot = a.slot;
         int it = 0;
-        bool cond = 0 < c.iter_min || *(volatile double *)&k.sp[0].compression > tol;
+        bool cond = psi_done || 0 < c.iter_min || *(volatile double *)&k.sp[0].compression > tol;
         while (cond) {
             if (!psi_done) {
                 lane_sweep<true>(0, [&](const Lanes<L> &ln, int64_t s) {
