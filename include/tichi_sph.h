@@ -160,6 +160,13 @@ int tsph_set_graph_mode(tsph_ctx *ctx, int use_graph);
  * FP32 summation order, and deterministic for a given setting. */
 int tsph_set_threads_per_particle(tsph_ctx *ctx, int threads_per_particle);
 
+/* For tests of the failure path: with 1, the grid-wide waits of the steps enqueued
+ * from then on expect one block more than there is and give up after a few
+ * milliseconds; 0 (the default) ends that.  A step that gave up is unfinished:
+ * the next tsph_read_stats or tsph_read_scene_stats fails with TSPH_ERR_CUDA, once,
+ * however many steps were enqueued behind it. */
+int tsph_set_absent_blocks(tsph_ctx *ctx, int blocks);
+
 /* cfl_condition(fluid), sph.py:41-47: dt on the device.  Also adds dt to the
  * device clock, as run_step does on the host (main.py:348-349). */
 int tsph_cfl_condition(tsph_ctx *ctx, const tsph_set *fluid, void *stream);
@@ -342,7 +349,8 @@ enum {
     TSPH_TAPE_ITER_OVERFLOW = 1,   /* a solve ran more than max_iters iterations */
     TSPH_TAPE_LIST_OVERFLOW = 2,   /* a particle had more neighbours than its list holds */
     TSPH_TAPE_OUTSIDE_GRID = 4,    /* a fluid particle had no valid cell (one-sided pairs) */
-    TSPH_TAPE_BOUND_PSI = 8        /* the boundary's psi_adv was nonzero */
+    TSPH_TAPE_BOUND_PSI = 8,       /* the boundary's psi_adv was nonzero */
+    TSPH_TAPE_GAVE_UP = 16         /* the step, or one before it, gave up at a grid barrier */
 };
 
 int tsph_tape_create(tsph_ctx *ctx, int slots, int max_iters, tsph_tape **out);

@@ -4,10 +4,14 @@ state that the next call takes for another (needs a GPU).
 Each case is held to the separate kernels, or to a context that never met it, bit
 for bit.
 """
+import ctypes as C
+
 import pytest
+import torch
 
 import tests.test_gpu_one_launch as one
 from tests.test_gpu_grid_edges import _need_cuda
+from tichi_sph_gb300 import _native
 
 pytestmark = pytest.mark.gpu
 
@@ -55,3 +59,68 @@ def test_no_iteration_floor(monkeypatch, dim, n, nb):
     one._same(a, b)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("dim,n,nb", [(2, 700, 90), (3, 900, 300), (3, 45000, 0)])
+def test_given_up_step(dim, n, nb):
+    """A step whose first grid barrier waits in vain (for a block that there is not)
+    leaves the particles' state and clean counters: the step enqueued behind it is
+    the one that it would have been, and the next reading of the scalars fails, once."""
+    _need_cuda()
+    runs = []
+    for fault in (True, False):
+        s = one._solver(dim, n, nb, False, True, inside=n > 5000)
+        s.substep()
+        assert s.stats()["launches_per_step"] == 1
+        if fault:
+            _native.check(s._lib.tsph_set_absent_blocks(s.ctx, 1), "absent")
+            s.substep()
+            _native.check(s._lib.tsph_set_absent_blocks(s.ctx, 0), "absent")
+        s.substep()
+        if fault:
+            with pytest.raises(RuntimeError, match="gave up"):
+                s.stats()
+        stats = [s.stats()]
+        s.substep()
+        stats.append(s.stats())
+        runs.append((s, stats))
+    (a, sa), (b, sb) = runs
+    _same_scalars(sa, sb)
+    one._same(a, b)
+    a.close()
+    b.close()
+
+
+def test_recording_of_a_given_up_step():
+    """The recording of a step that gave up, and of one behind it, is refused; after
+    the failure has been read a new recording is not."""
+    _need_cuda()
+    s = one._solver(3, 900, 300, False, True, inside=True)
+    tape = C.c_void_p()
+    _native.check(s._lib.tsph_tape_create(s.ctx, 2, 110, C.byref(tape)), "tape")
+    f, b = s._sets()
+    g = torch.zeros(900, 3, device="cuda")
+    gmu = torch.zeros(1, dtype=torch.float64, device="cuda")
+    ptr = lambda t, c=C.c_float: C.cast(t.data_ptr(), C.POINTER(c))  # noqa: E731
+
+    def record(absent):
+        _native.check(s._lib.tsph_set_absent_blocks(s.ctx, absent), "absent")
+        _native.check(s._lib.tsph_substep_record(s.ctx, f, b, tape, 1 - absent, None), "record")
+
+    def reverse(slot):
+        rc = s._lib.tsph_substep_adjoint(s.ctx, tape, slot, ptr(g), ptr(g), ptr(g), ptr(g), ptr(gmu, C.c_double), None)
+        torch.cuda.synchronize()
+        return rc
+
+    start = s.fluid.pos.clone(), s.fluid.vel.clone()
+    record(1)
+    record(0)
+    assert reverse(0) == reverse(1) == _native.ERR_STATE
+    with pytest.raises(RuntimeError, match="gave up"):
+        s.stats()
+    s.fluid.pos.copy_(start[0])
+    s.fluid.vel.copy_(start[1])
+    record(0)
+    assert reverse(1) == _native.OK
+    s._lib.tsph_tape_destroy(tape)
+    s.close()

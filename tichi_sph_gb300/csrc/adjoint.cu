@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(1024, 1) k_adj_step(const __grid_constant__ Sl
                                                       const __grid_constant__ Lam lam,
                                                       const __grid_constant__ AdjArgs a) {
     __shared__ double sh[kBlock / 32];
-    GridBarrier bar{a.bar, 0u};
+    GridBarrier bar{a.bar, 0u, 0u};
     Lam l = lam;
     // item(slot) for every lane of the particles' lane groups; all lanes of a warp call
     auto sweep = [&](auto &&item) {

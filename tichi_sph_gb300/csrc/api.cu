@@ -679,6 +679,13 @@ int tsph_set_threads_per_particle(tsph_ctx *c, int tpp) {
     return TSPH_OK;
 }
 
+int tsph_set_absent_blocks(tsph_ctx *c, int blocks) {
+    if (!c) return fail(TSPH_ERR_INVALID, "null ctx");
+    if (blocks < 0 || blocks > 1) return fail(TSPH_ERR_INVALID, "absent blocks must be 0 or 1");
+    c->absent = (unsigned int)blocks;
+    return TSPH_OK;
+}
+
 int tsph_cfl_condition(tsph_ctx *c, const tsph_set *f, void *stream) {
     if (!c || !f) return fail(TSPH_ERR_INVALID, "null argument");
     cudaStream_t st = (cudaStream_t)stream;
@@ -895,9 +902,10 @@ int tsph_read_scene_stats(tsph_ctx *c, int first, int count, tsph_stats *out, vo
         TSPH_CK(cudaMemcpyAsync(c->host_sp, c->k.sp, sizeof(ScenePersist) * c->n_scenes, cudaMemcpyDeviceToHost, st));
     }
     TSPH_CK(cudaStreamSynchronize(st));
-    if (c->host_ss[0].status & kStGaveUp) {
-        c->counts_zero = 0;
-        return fail(TSPH_ERR_CUDA, "the step gave up at a grid barrier: a block did not arrive");
+    if (c->host_sp[0].gave_up) {
+        c->host_sp[0].gave_up = 0;
+        TSPH_CK(cudaMemsetAsync(&c->k.sp->gave_up, 0, sizeof(int32_t), st));
+        return fail(TSPH_ERR_CUDA, "a step gave up at a grid barrier: a block did not arrive");
     }
     for (int i = 0; i < count; ++i) fill_stats(c, first + i, out + i);
     return TSPH_OK;

@@ -65,7 +65,10 @@ struct ScenePersist {
     int32_t steps;
     // 1 once BoundBuf::bb holds the boundary-boundary sums of the scene's
     // boundary as gathered (bb_n particles)
-    int32_t bb_valid, pad1;
+    int32_t bb_valid;
+    // 1 from a step that gave up at a grid barrier until the caller
+    // has been told (tsph_read_scene_stats)
+    int32_t gave_up;
     long long bb_n;
 };
 
@@ -241,9 +244,6 @@ struct SmallScratch {
     int *totals;
     unsigned int *bar;
 };
-
-// Step status bit (internal): the one-launch step gave up at a grid barrier.
-constexpr int kStGaveUp = 1 << 30;
 
 struct Scratch {
     double *partials;        // per-block FP64 partial sums

@@ -18,6 +18,7 @@ struct tsph_ctx {
     int scalars_on_host;      // host_ss / host_sp hold what the last enqueued work leaves on the device
     int counts_zero;          // the grids' counts and X's counters are zero (the one-launch step leaves them so)
     int captured;             // a caller has captured launches of this context
+    unsigned int absent;      // blocks that grid barriers wait for in vain (tsph_set_absent_blocks)
     tsph::SceneConst *host_sc;  // host copy of the scene table (pinned)
     tsph::SceneStep *host_ss;   // pinned mirrors for host-loop mode and stats
     tsph::ScenePersist *host_sp;

@@ -41,6 +41,7 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
     a.st_on = c.st_on;
     a.wc = c.p.wcsph_enabled;
     a.density_out = density_out;
+    a.absent = c.absent;
     if (c.rec_tape) {
         a.tape = c.rec_tape->a;
         a.record = 1;

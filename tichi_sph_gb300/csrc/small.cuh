@@ -33,6 +33,7 @@ struct SmallArgs {
     float *density_out;  // not null: only the grid and the densities (in the caller's order), no step
     int slot;            // of the tape
     int record, with_cfl, st_on, wc;
+    unsigned int absent;  // GridBarrier's
 };
 
 // Inclusive scan over the block; total in every thread.
@@ -450,9 +451,15 @@ struct SmallStep {
     // The last block to leave: the energies, the running totals, the barrier's reset,
     // and the scalars' copies in pinned host memory, so that a caller who reads them
     // after every substep waits for the kernel alone (two small copies behind it
-    // cost a time loop about 25 us a substep).
+    // cost a time loop about 25 us a substep).  After a step that was given up, zero
+    // counts for the next one, which may be enqueued already, and marks that stay
+    // until the caller has been told.
     __device__ __forceinline__ void leave(bool done) {
         if (!last_block_done(a.x.bar + kBarLeft, gridDim.x)) return;
+        // (any block may have given up, whatever this one saw)
+        const bool ok = done && !__ldcg(a.x.bar + kBarGaveUp);
+        if (!ok)
+            for (int64_t i = threadIdx.x; i < k.total_nodes; i += blockDim.x) F.count[i] = B.count[i] = 0;
         double ke = 0.0, pe = 0.0;
         for (int64_t i = threadIdx.x; !a.density_out && i < ns / kBlock && threadIdx.x < kBlock; i += kBlock) {
             ke += coop_block_tree(a.x.sums + i * (kBlock / 32));
@@ -461,15 +468,16 @@ struct SmallStep {
         ke = coop_sum256(ke, sh_d);
         pe = coop_sum256(pe, sh_d);
         if (threadIdx.x == 0) {
-            if (done && !__ldcg(a.x.bar + kBarGaveUp)) {
-                if (!a.density_out) {
-                    st().kinetic_energy = ke;
-                    st().potential_energy = pe;
-                    step_totals(k.sp[0], st());
-                }
-            } else {
-                atomicOr(&st().status, kStGaveUp);
+            if (!ok) {
+                k.sp[0].gave_up = 1;
+                a.x.bar[kBarTailF] = a.x.bar[kBarTailB] = a.x.bar[kBarStatus] = 0;
+            } else if (!a.density_out) {
+                st().kinetic_energy = ke;
+                st().potential_energy = pe;
+                step_totals(k.sp[0], st());
             }
+            // (a recording behind a step given up starts from an unfinished state)
+            if (a.record && k.sp[0].gave_up) atomicOr(&a.tape.meta[a.slot].status, TSPH_TAPE_GAVE_UP);
             a.x.bar[kBarCount] = a.x.bar[kBarGaveUp] = a.x.bar[kBarLeft] = 0;
         }
         __syncthreads();
@@ -493,7 +501,7 @@ __global__ void __launch_bounds__(1024, 1) k_small_step(const __grid_constant__ 
         if (threadIdx.x == 0) sh_next = 0;
         __syncthreads();
     }
-    SmallStep<DIM, ST, P, L, Q> step{k, F, B, a, {a.x.bar, 0u}, {&sh_next, 0u}, sh_d, sh_i, (a.f.n + kBlock - 1) / kBlock * kBlock, 0};
+    SmallStep<DIM, ST, P, L, Q> step{k, F, B, a, {a.x.bar, a.absent, 0u}, {&sh_next, 0u}, sh_d, sh_i, (a.f.n + kBlock - 1) / kBlock * kBlock, 0};
     const bool done = step.run();
     step.leave(done);
 }
