@@ -160,11 +160,12 @@ int tsph_set_graph_mode(tsph_ctx *ctx, int use_graph);
  * FP32 summation order, and deterministic for a given setting. */
 int tsph_set_threads_per_particle(tsph_ctx *ctx, int threads_per_particle);
 
-/* For tests of the failure path: with 1, the grid-wide waits of the steps enqueued
- * from then on expect one block more than there is and give up after a few
- * milliseconds; 0 (the default) ends that.  A step that gave up is unfinished:
- * the next tsph_read_stats or tsph_read_scene_stats fails with TSPH_ERR_CUDA, once,
- * however many steps were enqueued behind it. */
+/* For tests of the failure path: with 1, the grid-wide waits of the steps and
+ * reverses enqueued from then on expect one block more than there is and give up
+ * after a few milliseconds; 0 (the default) ends that.  A step that gave up is
+ * unfinished, and so is a reverse, whose gradients are all NaN: the next
+ * tsph_read_stats or tsph_read_scene_stats fails with TSPH_ERR_CUDA, once, however
+ * many steps were enqueued behind it. */
 int tsph_set_absent_blocks(tsph_ctx *ctx, int blocks);
 
 /* cfl_condition(fluid), sph.py:41-47: dt on the device.  Also adds dt to the

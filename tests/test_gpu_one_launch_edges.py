@@ -124,3 +124,36 @@ def test_recording_of_a_given_up_step():
     assert reverse(1) == _native.OK
     s._lib.tsph_tape_destroy(tape)
     s.close()
+
+
+@pytest.mark.parametrize("dim,n", [(2, 700), (3, 25000), (3, 45000)])
+def test_given_up_reverse(dim, n):
+    """A reverse whose grid barrier waits in vain gives gradients that are all NaN and
+    a failure at the next reading of the scalars; the next reverse is not touched."""
+    _need_cuda()
+    s = one._solver(dim, n, 90, False, True, inside=True)
+    tape = C.c_void_p()
+    _native.check(s._lib.tsph_tape_create(s.ctx, 1, 110, C.byref(tape)), "tape")
+    f, b = s._sets()
+    _native.check(s._lib.tsph_substep_record(s.ctx, f, b, tape, 0, None), "record")
+    s.stats()
+    out = []
+    for absent in (0, 1, 0):
+        gen = torch.Generator("cuda").manual_seed(1)
+        gx, gv = (torch.randn(n, dim, generator=gen, device="cuda") for _ in range(2))
+        gmu = torch.zeros(1, dtype=torch.float64, device="cuda")
+        ptr = lambda t, c=C.c_float: C.cast(t.data_ptr(), C.POINTER(c))  # noqa: E731
+        _native.check(s._lib.tsph_set_absent_blocks(s.ctx, absent), "absent")
+        _native.check(s._lib.tsph_substep_adjoint(s.ctx, tape, 0, ptr(gx), ptr(gv), ptr(gx), ptr(gv),
+                                                  ptr(gmu, C.c_double), None), "reverse")
+        if absent:
+            with pytest.raises(RuntimeError, match="gave up"):
+                s.stats()
+            assert all(bool(t.isnan().all()) for t in (gx, gv, gmu))
+        else:
+            s.stats()
+            out.append((gx, gv, gmu))
+    for x, y in zip(*out):
+        assert bool(x.isfinite().all()) and torch.equal(x, y)
+    s._lib.tsph_tape_destroy(tape)
+    s.close()

@@ -588,6 +588,8 @@ struct AdjArgs {
     float *gx_in, *gv_in;
     double *gmu, *sums;  // sums: 32 per block, one per warp
     unsigned int *bar;
+    ScenePersist *sp, *host_sp;  // what a reverse that gives up marks; its pinned copy
+    unsigned int absent;         // GridBarrier's
     int kd, kp;
 };
 
@@ -599,7 +601,7 @@ __global__ void __launch_bounds__(1024, 1) k_adj_step(const __grid_constant__ Sl
                                                       const __grid_constant__ Lam lam,
                                                       const __grid_constant__ AdjArgs a) {
     __shared__ double sh[kBlock / 32];
-    GridBarrier bar{a.bar, 0u, 0u};
+    GridBarrier bar{a.bar, a.absent, 0u};
     Lam l = lam;
     // item(slot) for every lane of the particles' lane groups; all lanes of a warp call
     auto sweep = [&](auto &&item) {
@@ -651,9 +653,14 @@ __global__ void __launch_bounds__(1024, 1) k_adj_step(const __grid_constant__ Sl
         });
         return true;
     };
-    // (a barrier given up leaves the gradients unfinished: dL/dmu becomes NaN)
     const bool done = run();
     if (!last_block_done(a.bar + kBarLeft, gridDim.x)) return;
+    // A barrier given up (by any block, whatever this one saw) leaves the gradients
+    // unfinished: they all become NaN, and the next reading of the scalars fails.
+    const bool ok = done && !__ldcg(a.bar + kBarGaveUp);
+    if (!ok)
+        for (int64_t i = threadIdx.x; i < (int64_t)v.n * DIM; i += blockDim.x)
+            a.gx_in[i] = a.gv_in[i] = __int_as_float(0x7fffffff);
     // dL/dmu: the warps' sums, in a fixed order
     double g = 0.0;
     const int warps = blockDim.x >> 5;
@@ -661,7 +668,8 @@ __global__ void __launch_bounds__(1024, 1) k_adj_step(const __grid_constant__ Sl
         g += __ldcg(a.sums + i / warps * 32 + i % warps);
     g = coop_sum256(g, sh);
     if (threadIdx.x != 0) return;
-    *a.gmu += done ? g : __longlong_as_double(0x7ff8000000000000ll);
+    *a.gmu += ok ? g : __longlong_as_double(0x7ff8000000000000ll);
+    if (!ok) a.sp->gave_up = a.host_sp->gave_up = 1;
     a.bar[kBarCount] = a.bar[kBarGaveUp] = a.bar[kBarLeft] = 0;
 }
 
@@ -914,7 +922,8 @@ int tsph_substep_adjoint(tsph_ctx *c, tsph_tape *t, int slot, const float *gx_ou
     const int nb = blocks_for(v.n);
     Lam l = lam_of(*t);
     if (c->use_graph && c->sms && ((int64_t)v.n + 31) / 32 <= kAdjWarpsPerSm * c->sms) {
-        const AdjArgs a = {gx_out, gv_out, gx_in, gv_in, gmu, t->partials, t->bar, m.kd, m.kp};
+        const AdjArgs a = {gx_out, gv_out, gx_in, gv_in, gmu, t->partials, t->bar,
+                           c->k.sp, c->host_sp, c->absent, m.kd, m.kp};
         const cudaError_t e = c->k.dim == 3 ? launch_adj_step<3>(*c, v, l, a, st) : launch_adj_step<2>(*c, v, l, a, st);
         if (e == cudaSuccess) return TSPH_OK;
         // this process may not use every SM at once: separate launches

@@ -66,7 +66,7 @@ struct ScenePersist {
     // 1 once BoundBuf::bb holds the boundary-boundary sums of the scene's
     // boundary as gathered (bb_n particles)
     int32_t bb_valid;
-    // 1 from a step that gave up at a grid barrier until the caller
+    // 1 from a step (or its reverse) that gave up at a grid barrier until the caller
     // has been told (tsph_read_scene_stats)
     int32_t gave_up;
     long long bb_n;
