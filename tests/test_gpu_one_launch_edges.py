@@ -157,3 +157,39 @@ def test_given_up_reverse(dim, n):
         assert bool(x.isfinite().all()) and torch.equal(x, y)
     s._lib.tsph_tape_destroy(tape)
     s.close()
+
+
+def test_replay_of_a_density_captured_with_host_loops():
+    """A density evaluation captured while the solver loops run on the host: its
+    replays leave counts behind, also for the one-launch steps of later."""
+    _need_cuda()
+    n, runs = 900, []
+    for captured in (True, False):
+        s = one._solver(3, n, 300, False, False, inside=True)
+        tape = C.c_void_p()
+        _native.check(s._lib.tsph_tape_create(s.ctx, 1, 110, C.byref(tape)), "tape")
+        rho = torch.zeros(n, device="cuda")
+        s.substep()
+
+        def density():
+            f, b = s._sets()
+            _native.check(s._lib.tsph_density_record(s.ctx, f, b, tape, 0, C.cast(rho.data_ptr(), C.POINTER(C.c_float)),
+                                                     s._stream()), "density")
+
+        density()
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                density()
+        s.set_graph_mode(True)
+        for _ in range(3):
+            s.substep()
+            graph.replay() if captured else density()
+        s.substep()
+        assert s.stats()["launches_per_step"] == 1
+        runs.append((s, rho, tape))
+    one._same(runs[0][0], runs[1][0])
+    assert torch.equal(runs[0][1], runs[1][1])
+    for s, _, tape in runs:
+        s._lib.tsph_tape_destroy(tape)
+        s.close()

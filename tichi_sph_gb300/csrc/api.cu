@@ -252,7 +252,7 @@ bool capturing(tsph_ctx *c, cudaStream_t st) {
 // captured step fails there with the graph's launch, as one of any size).
 int small_step(tsph_ctx *c, const tsph_set *f, const tsph_set *b, bool with_cfl, float *density_out, cudaStream_t st,
                bool &taken) {
-    taken = c->use_graph && !capturing(c, st) && small_step_fits(*c, *f, *b);
+    taken = !capturing(c, st) && c->use_graph && small_step_fits(*c, *f, *b);
     if (!taken) return TSPH_OK;
     const cudaError_t e = launch_small_step(*c, *f, *b, with_cfl, density_out, st);
     if (e == cudaSuccess) return TSPH_OK;
