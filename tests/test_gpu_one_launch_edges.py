@@ -193,3 +193,21 @@ def test_replay_of_a_density_captured_with_host_loops():
     for s, _, tape in runs:
         s._lib.tsph_tape_destroy(tape)
         s.close()
+
+
+def test_scalars_after_the_rest_of_a_composed_step():
+    """Phase calls that go on after a whole step change the scalars on the device: a
+    reading gives those, not what the step left in host memory."""
+    _need_cuda()
+    runs = []
+    for use_graph in (True, False):
+        s = one._solver(3, 900, 300, False, use_graph, inside=True)
+        s.grid_build()
+        s.density_alpha()
+        s.substep()
+        s.update()
+        runs.append((s, [s.stats()]))
+    assert runs[0][1][0]["steps"] == 2
+    _same_scalars(runs[0][1], runs[1][1])
+    for s, _ in runs:
+        s.close()

@@ -255,6 +255,7 @@ int small_step(tsph_ctx *c, const tsph_set *f, const tsph_set *b, bool with_cfl,
     taken = !capturing(c, st) && c->use_graph && small_step_fits(*c, *f, *b);
     if (!taken) return TSPH_OK;
     const cudaError_t e = launch_small_step(*c, *f, *b, with_cfl, density_out, st);
+    c->counts_zero = c->scalars_on_host = e == cudaSuccess && !c->captured;
     if (e == cudaSuccess) return TSPH_OK;
     // this process may not use every SM at once: separate launches from here on
     if (e != cudaErrorCooperativeLaunchTooLarge) return fail_cuda(e, "the one-launch step");
@@ -711,6 +712,7 @@ int tsph_substep(tsph_ctx *c, const tsph_set *f, const tsph_set *b, void *stream
 static int kl_check(tsph_ctx *c, const char *what, void *stream) {
     if (!c) return fail(TSPH_ERR_INVALID, "null ctx");
     (void)capturing(c, (cudaStream_t)stream);
+    c->scalars_on_host = 0;
     if (c->n_scenes != 1) {
         std::snprintf(g_last_error, sizeof(g_last_error), "%s: kernel-level calls take a one-scene context", what);
         return TSPH_ERR_INVALID;

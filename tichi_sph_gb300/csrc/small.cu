@@ -65,7 +65,6 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
         if (e == cudaSuccess) e = cudaMemsetAsync(c.X.bar + kBarTailF, 0, 4 * (kBarWords - kBarTailF), st);
         if (e != cudaSuccess) return e;
     }
-    c.counts_zero = c.scalars_on_host = !c.captured;
     const bool d3 = c.k.dim == 3;
     switch (lanes) {
         case 8:
