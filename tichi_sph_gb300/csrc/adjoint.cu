@@ -589,7 +589,7 @@ struct AdjArgs {
     double *gmu, *sums;  // sums: 32 per block, one per warp
     unsigned int *bar;
     ScenePersist *sp, *host_sp;  // what a reverse that gives up marks; its pinned copy
-    unsigned int absent;         // GridBarrier's
+    unsigned int absent;         // blocks that will not come (GridBarrier)
     int kd, kp;
 };
 
@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(1024, 1) k_adj_step(const __grid_constant__ Sl
                                                       const __grid_constant__ Lam lam,
                                                       const __grid_constant__ AdjArgs a) {
     __shared__ double sh[kBlock / 32];
-    GridBarrier bar{a.bar, a.absent, 0u};
+    GridBarrier bar{a.bar, a.absent};
     Lam l = lam;
     // item(slot) for every lane of the particles' lane groups; all lanes of a warp call
     auto sweep = [&](auto &&item) {

@@ -13,14 +13,14 @@ namespace tsph {
 // a few seconds, after which the step is given up and the next reading of the
 // scalars says so.
 constexpr unsigned int kSpinLimit = 1u << 23;
-constexpr unsigned int kSpinLimitAbsent = 1u << 12;  // where blocks are known not to come (tests)
 
 // Barrier over the grid's blocks (all resident: a cooperative launch).  The
 // counter only grows within a launch; the launch's last block to leave sets it
 // back.  False: a block did not arrive within the limit; every block then leaves.
 struct GridBarrier {
     unsigned int *bar;  // words kBarCount, kBarGaveUp, kBarLeft
-    unsigned int absent;  // blocks waited for beyond the grid's (tsph_set_absent_blocks)
+    // the count to wait for; starts at the blocks that will not come (0 but in tests,
+    // tsph_set_absent_blocks), for which the wait is a short one
     unsigned int target;
     static __device__ __forceinline__ unsigned int acquire(const unsigned int *p) {
         unsigned int v;
@@ -31,8 +31,7 @@ struct GridBarrier {
         __shared__ int ok;
         __syncthreads();
         if (threadIdx.x == 0) {
-            target += gridDim.x + absent;
-            const unsigned int limit = absent ? kSpinLimitAbsent : kSpinLimit;
+            target += gridDim.x;
             // release / acquire at GPU scope, with the block's two barriers around
             // them, order everything before against everything after
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar + kBarCount) : "memory");
@@ -40,7 +39,7 @@ struct GridBarrier {
             unsigned int n = 0;
             while (acquire(bar + kBarCount) < target) {
                 if ((++n & 1023u) != 0) continue;
-                if (n > limit) atomicExch(bar + kBarGaveUp, 1u);
+                if (n > kSpinLimit || target % gridDim.x != 0) atomicExch(bar + kBarGaveUp, 1u);
                 if (acquire(bar + kBarGaveUp)) {
                     all = false;
                     break;

@@ -33,7 +33,7 @@ struct SmallArgs {
     float *density_out;  // not null: only the grid and the densities (in the caller's order), no step
     int slot;            // of the tape
     int record, with_cfl, st_on, wc;
-    unsigned int absent;  // GridBarrier's
+    unsigned int absent;  // blocks that will not come (GridBarrier)
 };
 
 // Inclusive scan over the block; total in every thread.
@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(1024, 1) k_small_step(const __grid_constant__ 
         if (threadIdx.x == 0) sh_next = 0;
         __syncthreads();
     }
-    SmallStep<DIM, ST, P, L, Q> step{k, F, B, a, {a.x.bar, a.absent, 0u}, {&sh_next, 0u}, sh_d, sh_i, (a.f.n + kBlock - 1) / kBlock * kBlock, 0};
+    SmallStep<DIM, ST, P, L, Q> step{k, F, B, a, {a.x.bar, a.absent}, {&sh_next, 0u}, sh_d, sh_i, (a.f.n + kBlock - 1) / kBlock * kBlock, 0};
     const bool done = step.run();
     step.leave(done);
 }
