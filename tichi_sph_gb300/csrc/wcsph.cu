@@ -45,18 +45,19 @@ __global__ void __launch_bounds__(kBlock) k_wc_acce(KConst k, FluidBuf F, BoundB
 }
 
 // What the velocity map reads of a particle, in sorted order: the caller's
-// current position with X / psi, and velocity.  A velocity that is not finite
-// makes X / psi NaN, so that the map need not read velocities beyond h, where
-// W = 0, to give the NaN that 0 times it is.
+// current position, and velocity with X / psi.  p.w is X / psi too, or NaN where a
+// component of the velocity is not finite: where it is finite the map need not
+// read what lies beyond h, where W = 0, and elsewhere it does, as 0 times such a
+// component is NaN.
 template <int DIM>
 __device__ __forceinline__ void map_record(const KConst &k, const tsph_set &U, int64_t pid, float4 &p, float4 &v) {
     const bool vf = k.vfsph != 0;
     const float X = vf ? U.rest_volume[pid] : U.mass[pid];
     const float psi = vf ? U.sph_compression[pid] : U.sph_density[pid];
     const float *x = U.pos + pid * DIM, *u = U.vel + pid * DIM;
-    v = make_float4(u[0], u[1], DIM == 3 ? u[2] : 0.f, 0.f);
+    v = make_float4(u[0], u[1], DIM == 3 ? u[2] : 0.f, X / psi);
     const bool fin = isfinite(v.x) && isfinite(v.y) && isfinite(v.z);
-    p = make_float4(x[0], x[1], DIM == 3 ? x[2] : 0.f, fin ? X / psi : __int_as_float(0x7fffffff));
+    p = make_float4(x[0], x[1], DIM == 3 ? x[2] : 0.f, fin ? v.w : __int_as_float(0x7fffffff));
 }
 
 template <int DIM>
@@ -98,8 +99,8 @@ __global__ void __launch_bounds__(kBlock) k_map_velocity(KConst k, FluidBuf F, t
             const float dx = gp.x - p.x, dy = gp.y - p.y, dz = DIM == 3 ? gp.z - p.z : 0.f;
             const float q = sqrtf(dx * dx + dy * dy + dz * dz) * g.inv_h;
             if (q >= 1.f && isfinite(p.w)) return;  // W = 0
-            const float f = p.w * (kw(q) * g.sig);
             if (PACKED) v = F.facc[j];
+            const float f = (isfinite(p.w) ? p.w : v.w) * (kw(q) * g.sig);
             vx += f * v.x;
             vy += f * v.y;
             if (DIM == 3) vz += f * v.z;
