@@ -680,6 +680,12 @@ int tsph_set_threads_per_particle(tsph_ctx *c, int tpp) {
     return TSPH_OK;
 }
 
+// Between volume-fraction passes called one at a time: the sums kept from the passes
+// before are those of the old time step.
+static void time_step_changed(tsph_ctx *c, cudaStream_t st) {
+    if (c->kl_phase == 5) launch_fbm_redo(*c, c->kl_fbm + 1, st);
+}
+
 int tsph_set_absent_blocks(tsph_ctx *c, int blocks) {
     if (!c) return fail(TSPH_ERR_INVALID, "null ctx");
     if (blocks < 0 || blocks > 1) return fail(TSPH_ERR_INVALID, "absent blocks must be 0 or 1");
@@ -693,6 +699,7 @@ int tsph_cfl_condition(tsph_ctx *c, const tsph_set *f, void *stream) {
     (void)capturing(c, st);
     TSPH_CK(cudaMemsetAsync(c->k.dg->ticket, 0, sizeof(unsigned int), st));
     launch_cfl(*c, *f, st);
+    time_step_changed(c, st);
     TSPH_CK(cudaGetLastError());
     return TSPH_OK;
 }
@@ -869,11 +876,9 @@ int tsph_fbm_pass(tsph_ctx *c, int32_t *general_flag_out, void *stream) {
     if (c->kl_phase < 3 || c->kl_phase > 5)
         return kl_state("tsph_fbm_pass", "the volume-fraction loop follows the density solve");
     cudaStream_t st = (cudaStream_t)stream;
-    if (!c->kl_fbm) {
-        launch_fbm_begin(*c, 0, 0, st);
-        c->kl_fbm = 1;
-    }
+    if (!c->kl_fbm) launch_fbm_begin(*c, 0, 0, st);
     launch_fbm_pass(*c, 0, 0, st);
+    c->kl_fbm++;
     TSPH_CK(cudaGetLastError());
     c->kl_phase = 5;
     rc = kl_read_step(c, st);
@@ -974,6 +979,7 @@ int tsph_set_state(tsph_ctx *c, double time_count, float dt, double compression,
     (void)capturing(c, (cudaStream_t)stream);
     c->scalars_on_host = 0;
     k_set_state<<<(c->n_scenes + 127) / 128, 128, 0, (cudaStream_t)stream>>>(c->k, time_count, dt, compression);
+    time_step_changed(c, (cudaStream_t)stream);
     TSPH_CK(cudaGetLastError());
     return TSPH_OK;
 }

@@ -49,8 +49,8 @@ struct tsph_ctx {
     // kernel-level composition (tsph_grid_build ... tsph_update): how far the
     // step has got (0: none in progress, 1 grid built, 2 density done, 3
     // non-pressure forces done, 4 weakly compressible block done, 5 in the
-    // volume-fraction loop), whether a sweep A awaits its sweep B, and whether
-    // the volume-fraction loop has begun
+    // volume-fraction loop), whether a sweep A awaits its sweep B, and the
+    // volume-fraction passes done
     int kl_phase, kl_psi, kl_fbm;
     // particle capacities given at create (the caller-order tables are this long)
     int64_t cap_f, cap_b;
@@ -133,5 +133,7 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
 // fbm.cu
 void launch_fbm_begin(tsph_ctx &c, cudaGraphConditionalHandle h, int use_cond, cudaStream_t st);
 void launch_fbm_pass(tsph_ctx &c, cudaGraphConditionalHandle h, int use_cond, cudaStream_t st);
+// Every particle sums again in pass `pass` (the time step has changed).
+void launch_fbm_redo(tsph_ctx &c, int pass, cudaStream_t st);
 
 }  // namespace tsph

@@ -107,6 +107,11 @@ __global__ void __launch_bounds__(kBlock, P <= 2 ? 5 : 1) k_fbm_pass(KConst k, F
     }
 }
 
+__global__ void __launch_bounds__(kBlock) k_fbm_redo(FluidBuf F, int pass) {
+    const int64_t s = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    if (s < F.cap) F.redo[(pass & 1) * F.cap + s] = pass;
+}
+
 template <int P>
 static void fbm_pass_dim(tsph_ctx &c, cudaGraphConditionalHandle h, int use_cond, cudaStream_t st, bool drift) {
     const int nb = blocks_for(c.F.cap);
@@ -142,6 +147,10 @@ void launch_fbm_begin(tsph_ctx &c, cudaGraphConditionalHandle h, int use_cond, c
 void launch_fbm_pass(tsph_ctx &c, cudaGraphConditionalHandle h, int use_cond, cudaStream_t st) {
     c.launches += 1;
     fbm_dispatch(c, h, use_cond, st, false);
+}
+
+void launch_fbm_redo(tsph_ctx &c, int pass, cudaStream_t st) {
+    k_fbm_redo<<<blocks_for(c.F.cap), kBlock, 0, st>>>(c.F, pass);
 }
 
 }  // namespace tsph
