@@ -160,6 +160,11 @@ int tsph_set_graph_mode(tsph_ctx *ctx, int use_graph);
  * FP32 summation order, and deterministic for a given setting. */
 int tsph_set_threads_per_particle(tsph_ctx *ctx, int threads_per_particle);
 
+/* Writes 1 if a substep of these sets would run as one launch with the context's
+ * present settings, else 0 (one scene up to a size, device-side solver loops, one
+ * thread per particle). */
+int tsph_one_launch(tsph_ctx *ctx, const tsph_set *fluid, const tsph_set *bound, int32_t *out);
+
 /* For tests of the failure path: with 1, the grid-wide waits of the steps and
  * reverses enqueued from then on expect one block more than there is and give up
  * after a few milliseconds; 0 (the default) ends that.  A step that gave up is

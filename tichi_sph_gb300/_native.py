@@ -112,6 +112,7 @@ SIGNATURES = {
     "tsph_destroy": (C.c_int, [CtxP]),
     "tsph_set_graph_mode": (C.c_int, [CtxP, C.c_int]),
     "tsph_set_threads_per_particle": (C.c_int, [CtxP, C.c_int]),
+    "tsph_one_launch": (C.c_int, [CtxP, C.POINTER(Set), C.POINTER(Set), C.POINTER(_i32)]),
     "tsph_set_absent_blocks": (C.c_int, [CtxP, C.c_int]),
     "tsph_cfl_condition": (C.c_int, [CtxP, C.POINTER(Set), C.c_void_p]),
     "tsph_sph_step": (C.c_int, [CtxP, C.POINTER(Set), C.POINTER(Set), C.c_void_p]),

@@ -680,6 +680,12 @@ int tsph_set_threads_per_particle(tsph_ctx *c, int tpp) {
     return TSPH_OK;
 }
 
+int tsph_one_launch(tsph_ctx *c, const tsph_set *f, const tsph_set *b, int32_t *out) {
+    if (!c || !f || !b || !out) return fail(TSPH_ERR_INVALID, "null argument");
+    *out = c->use_graph && small_step_fits(*c, *f, *b);
+    return TSPH_OK;
+}
+
 // Between volume-fraction passes called one at a time: the sums kept from the passes
 // before are those of the old time step.
 static void time_step_changed(tsph_ctx *c, cudaStream_t st) {

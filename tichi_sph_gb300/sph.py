@@ -119,8 +119,12 @@ class Solver:
         self.tpp = int(tpp)
 
     def autotune(self, candidates=(1, 2, 4, 8), reps=5):
-        """Times the neighbour-list sweeps (Jacobi pair + advection) for each
-        threads-per-particle setting on the current state and keeps the fastest.
+        """Times the neighbour-list sweeps (Jacobi pair + advection) of the separate
+        launches for each threads-per-particle setting on the current state and
+        keeps the fastest -- or one, if that is among the candidates and the substep
+        is then a single launch, which the separate ones do not reach with any
+        setting (us a substep, separate with the fastest setting and one launch:
+        5k particles in 2D 148 / 75, 8k 168 / 91, 97k 250 / 165).
         Returns {tpp: ms per Jacobi iteration + advection}."""
         res = {}
         for t in candidates:
@@ -128,6 +132,12 @@ class Solver:
             ph = self.profile_phases(reps=reps)
             res[t] = ph["psi"] + ph["vel"] + ph["advect"]
         best = min(res, key=res.get)
+        if 1 in res:
+            self.set_threads_per_particle(1)
+            one = _native.C.c_int32(0)
+            check(self._lib.tsph_one_launch(self.ctx, *self._sets(), _native.C.byref(one)), "tsph_one_launch")
+            if one.value:
+                best = 1
         self.set_threads_per_particle(best)
         return res
 
