@@ -10,7 +10,7 @@ import pytest
 import torch
 
 import tests.test_gpu_one_launch as one
-from tests.test_gpu_grid_edges import _need_cuda
+from tests.test_gpu_grid_edges import H, _need_cuda
 from tichi_sph_gb300 import _native
 
 pytestmark = pytest.mark.gpu
@@ -209,5 +209,33 @@ def test_scalars_after_the_rest_of_a_composed_step():
         runs.append((s, [s.stats()]))
     assert runs[0][1][0]["steps"] == 2
     _same_scalars(runs[0][1], runs[1][1])
+    for s, _ in runs:
+        s.close()
+
+
+@pytest.mark.parametrize("dim,cells,n", [(2, 1500, 700), (2, 1700, 700), (3, 130, 900), (3, 143, 900)])
+def test_few_particles_in_a_large_grid(monkeypatch, dim, cells, n):
+    """Grids below and above the size from which on a block takes all its threads (2.5M
+    cells with 152 SMs)."""
+    _need_cuda()
+    scene = one._scene
+
+    def wide(d, c):
+        cfg, scen, span = scene(d, c)
+        scen["sim_env"]["sim_space_rt"] = [cells * H] * d
+        return cfg, scen, span
+
+    monkeypatch.setattr(one, "_scene", wide)
+    runs = []
+    for use_graph in (True, False):
+        s = one._solver(dim, n, 90, False, use_graph)
+        stats = []
+        for _ in range(3):
+            s.substep()
+            stats.append(s.stats())
+        assert (stats[-1]["launches_per_step"] == 1) == use_graph
+        runs.append((s, stats))
+    _same_scalars(runs[0][1], runs[1][1])
+    one._same(runs[0][0], runs[1][0])
     for s, _ in runs:
         s.close()

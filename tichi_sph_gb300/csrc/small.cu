@@ -22,6 +22,8 @@ TSPH_SMALL(3, 1, true) TSPH_SMALL(3, 1, false) TSPH_SMALL(3, 4, false) TSPH_SMAL
 // 1M 1595 / 1528, 2.1M 2963 / 2963, 4.1M 5567 / 5721; in 2D 61k 189 / 111, 300k after
 // 1,500 substeps 491 / 363, 900k 1430 / 1371.
 constexpr int64_t kSmallWarpsPerSm = 512;
+// Cells per SM from which on a block takes all its threads (launch_small_step).
+constexpr int64_t kCellsPerSm = 16384;
 
 bool small_step_fits(const tsph_ctx &c, const tsph_set &f, const tsph_set &b) {
     if (c.n_scenes != 1 || c.batch || !c.sms || !c.scan_r1 || c.tpp != 1 || f.n < 1) return false;
@@ -57,7 +59,13 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
     // 1614 / 1385; 205k from rest 425 / 424).  In 2D, with less work a run, it gave
     // nothing: 300k 363 / 362, 900k 1371 / 1395.
     const int64_t bruns = ((b.n + 31) / 32 + c.sms - 1) / c.sms;
-    const int threads = coop_threads((runs * lanes + bruns) * c.sms, c.sms);
+    // Few particles in a large grid: the time is that of counting its cells, which all
+    // the threads that an SM holds share (us a substep with the particles' 256 or
+    // 512 threads, with 1,024 and in separate launches: 2k particles in 1M cells 91 / 92
+    // / 200, 4.1M 134 / 120 / 267, 64M 1637 / 1070 / 1243; 62k in 2D, 1M 110 / 111 / 183,
+    // 64M 1652 / 1083 / 1224).
+    const bool many_cells = c.k.total_nodes > kCellsPerSm * c.sms;
+    const int threads = many_cells ? 1024 : coop_threads((runs * lanes + bruns) * c.sms, c.sms);
     // the kernel leaves zero counters behind, other grid builds do not
     if (!c.counts_zero) {
         cudaError_t e = cudaMemsetAsync(c.F.count, 0, sizeof(int) * c.k.total_nodes, st);
