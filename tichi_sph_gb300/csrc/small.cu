@@ -58,14 +58,22 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
     // with fixed turns and with the queue: 216k 478 / 442, 439k 756 / 706, 1M
     // 1614 / 1385; 205k from rest 425 / 424).  In 2D, with less work a run, it gave
     // nothing: 300k 363 / 362, 900k 1371 / 1395.
-    const int64_t bruns = ((b.n + 31) / 32 + c.sms - 1) / c.sms;
+    // The boundary's runs have warps of their own beside them, unless one or two more
+    // would take a block past 512 threads: the next size, 1,024, is slower (5k in 2D
+    // 90 and 92 us for a substep and the copies of its start state) and takes all of
+    // an SM's registers, so that no other context's step fits beside it (four
+    // contexts of 5k on four streams, a substep each: 151 us with 512 threads, 287
+    // with 1,024, 212 in separate launches; of 8k 186, 344 and 298).
+    const int64_t lwarps = runs * lanes;
+    int64_t bruns = ((b.n + 31) / 32 + c.sms - 1) / c.sms;
+    if (lwarps <= 16 && lwarps + bruns > 16 && bruns <= 2) bruns = 16 - lwarps;
     // Few particles in a large grid: the time is that of counting its cells, which all
     // the threads that an SM holds share (us a substep with the particles' 256 or
     // 512 threads, with 1,024 and in separate launches: 2k particles in 1M cells 91 / 92
     // / 200, 4.1M 134 / 120 / 267, 64M 1637 / 1070 / 1243; 62k in 2D, 1M 110 / 111 / 183,
     // 64M 1652 / 1083 / 1224).
     const bool many_cells = c.k.total_nodes > kCellsPerSm * c.sms;
-    const int threads = many_cells ? 1024 : coop_threads((runs * lanes + bruns) * c.sms, c.sms);
+    const int threads = many_cells ? 1024 : coop_threads((lwarps + bruns) * c.sms, c.sms);
     // the kernel leaves zero counters behind, other grid builds do not
     if (!c.counts_zero) {
         cudaError_t e = cudaMemsetAsync(c.F.count, 0, sizeof(int) * c.k.total_nodes, st);
