@@ -5,6 +5,7 @@ Each case is held to the separate kernels, or to a context that never met it, bi
 for bit.
 """
 import ctypes as C
+import functools
 
 import pytest
 import torch
@@ -237,5 +238,33 @@ def test_few_particles_in_a_large_grid(monkeypatch, dim, cells, n):
         runs.append((s, stats))
     _same_scalars(runs[0][1], runs[1][1])
     one._same(runs[0][0], runs[1][0])
+    for s, _ in runs:
+        s.close()
+
+
+@pytest.mark.parametrize("dim,n,nb", [(2, 700, 90), (3, 5000, 700), (3, 25000, 400), (3, 45000, 90), (3, 160000, 700)])
+@pytest.mark.parametrize("block", ["weakly compressible", "surface tension"])
+def test_optional_blocks(monkeypatch, dim, n, nb, block):
+    """The weakly compressible block, and surface tension of one phase, with eight,
+    four and one lanes per particle and with runs from a queue."""
+    _need_cuda()
+    import tichi_sph_gb300
+    wc = block == "weakly compressible"
+    monkeypatch.setattr(tichi_sph_gb300, "Solver", functools.partial(tichi_sph_gb300.Solver, wcsph=wc))
+    runs = []
+    for use_graph in (True, False):
+        s = one._solver(dim, n, nb, False, use_graph, gamma=0.0 if wc else 0.07, inside=True)
+        stats = []
+        for _ in range(2):
+            s.substep()
+            stats.append(s.stats())
+        assert (stats[-1]["launches_per_step"] == 1) == use_graph
+        runs.append((s, stats))
+    _same_scalars(runs[0][1], runs[1][1])
+    one._same(runs[0][0], runs[1][0])
+    for f in ("pressure", "normal"):
+        x, y = (getattr(s.fluid, f) for s, _ in runs)
+        assert torch.equal(torch.nan_to_num(x.double()), torch.nan_to_num(y.double())), f
+        assert bool(x.abs().max() > 0) == ((f == "pressure") == wc)
     for s, _ in runs:
         s.close()
