@@ -657,16 +657,17 @@ __global__ void __launch_bounds__(1024, 1) k_adj_step(const __grid_constant__ Sl
     if (!last_block_done(a.bar + kBarLeft, gridDim.x)) return;
     // A barrier given up (by any block, whatever this one saw) leaves the gradients
     // unfinished: they all become NaN, and the next reading of the scalars fails.
-    const bool ok = done && !__ldcg(a.bar + kBarGaveUp);
-    if (!ok)
-        for (int64_t i = threadIdx.x; i < (int64_t)v.n * DIM; i += blockDim.x)
-            a.gx_in[i] = a.gv_in[i] = __int_as_float(0x7fffffff);
+    const unsigned int given_up = __ldcg(a.bar + kBarGaveUp);
     // dL/dmu: the warps' sums, in a fixed order
     double g = 0.0;
     const int warps = blockDim.x >> 5;
     for (int i = threadIdx.x; i < (int)gridDim.x * warps && threadIdx.x < kBlock; i += kBlock)
         g += __ldcg(a.sums + i / warps * 32 + i % warps);
     g = coop_sum256(g, sh);
+    const bool ok = done && !given_up;
+    if (!ok)
+        for (int64_t i = threadIdx.x; i < (int64_t)v.n * DIM; i += blockDim.x)
+            a.gx_in[i] = a.gv_in[i] = __int_as_float(0x7fffffff);
     if (threadIdx.x != 0) return;
     *a.gmu += ok ? g : __longlong_as_double(0x7ff8000000000000ll);
     if (!ok) a.sp->gave_up = a.host_sp->gave_up = 1;

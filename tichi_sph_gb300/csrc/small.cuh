@@ -457,9 +457,7 @@ struct SmallStep {
     __device__ __forceinline__ void leave(bool done) {
         if (!last_block_done(a.x.bar + kBarLeft, gridDim.x)) return;
         // (any block may have given up, whatever this one saw)
-        const bool ok = done && !__ldcg(a.x.bar + kBarGaveUp);
-        if (!ok)
-            for (int64_t i = threadIdx.x; i < k.total_nodes; i += blockDim.x) F.count[i] = B.count[i] = 0;
+        const unsigned int given_up = __ldcg(a.x.bar + kBarGaveUp);
         double ke = 0.0, pe = 0.0;
         for (int64_t i = threadIdx.x; !a.density_out && i < ns / kBlock && threadIdx.x < kBlock; i += kBlock) {
             ke += coop_block_tree(a.x.sums + i * (kBlock / 32));
@@ -467,6 +465,9 @@ struct SmallStep {
         }
         ke = coop_sum256(ke, sh_d);
         pe = coop_sum256(pe, sh_d);
+        const bool ok = done && !given_up;
+        if (!ok)
+            for (int64_t i = threadIdx.x; i < k.total_nodes; i += blockDim.x) F.count[i] = B.count[i] = 0;
         if (threadIdx.x == 0) {
             if (!ok) {
                 k.sp[0].gave_up = 1;
