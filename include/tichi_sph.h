@@ -150,9 +150,14 @@ int tsph_create_batch(const tsph_params *scenes, int n_scenes, const int64_t *fl
                       const int64_t *bound_counts, tsph_ctx **out);
 int tsph_destroy(tsph_ctx *ctx);
 
-/* Selects how the two solver loops run: 1 = one CUDA graph per substep with
- * device-side while nodes (default), 0 = host-driven loops that read the
- * convergence value every iteration like main.py:201,222. */
+/* Selects how the two solver loops run: 1 = on the device (default), inside one
+ * cooperative launch per substep where that is taken (tsph_one_launch), else as
+ * while nodes of one CUDA graph per substep; 0 = host-driven loops that read the
+ * convergence value every iteration like main.py:201,222.  A context is stepped by
+ * one thread at a time.  Steps of several contexts may be enqueued on streams of
+ * their own; one-launch steps of small scenes run two at a time, of larger ones
+ * (which fill the GPU) one after another, so for many scenes at a time
+ * tsph_create_batch is the faster form. */
 int tsph_set_graph_mode(tsph_ctx *ctx, int use_graph);
 
 /* Threads per particle of the neighbour-list sweeps (1, 2, 4 or 8; default 1).

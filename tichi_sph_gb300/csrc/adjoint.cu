@@ -741,8 +741,9 @@ Lam lam_of(const tsph_tape &t) {
     return {t.lam_u, t.lam_u2, t.lam_x, t.lam_beta, t.lam_us, t.lam_a1, t.lam_n, t.lam_psi, t.lam_alpha};
 }
 
-// Up to this many warps of particles per SM a substep is reversed in one launch
-// (the forward step's rule, small_step_fits).
+// Up to this many warps of fluid particles per SM a substep is reversed in one
+// launch.  (The forward step's limit, which counts the boundary's warps too; its other
+// conditions do not matter to the reverse, which reads the tape alone.)
 constexpr int64_t kAdjWarpsPerSm = 512;
 
 // Eight lanes per particle while the SMs' 32 warps hold them all, then four, then

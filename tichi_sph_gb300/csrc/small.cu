@@ -18,9 +18,9 @@ TSPH_SMALL(3, 1, true) TSPH_SMALL(3, 1, false) TSPH_SMALL(3, 4, false) TSPH_SMAL
 // particles for each SM.  Separate launches and one launch, us per substep (fluid
 // particles of a 3D dam break): after 500 substeps 216k 515 / 442, 439k 795 / 716,
 // 512k 893 / 809, 1M 1464 / 1385, 2.1M (past the line) 2596 / 2550, 4.1M
-// 4546 / 4668; from rest 8k 235 / 154, 27k 236 / 170, 99k 352 / 250, 205k 514 / 424,
-// 1M 1595 / 1528, 2.1M 2963 / 2963, 4.1M 5567 / 5721; in 2D 61k 189 / 111, 300k after
-// 1,500 substeps 491 / 363, 900k 1430 / 1371.
+// 4546 / 4668; from rest 1.3k 196 / 79, 8k 211 / 93, 27k 222 / 128, 99k 318 / 226, 205k
+// 487 / 409, 1M 1571 / 1497, 2.1M 2943 / 2936, 4.1M 5530 / 5631; in 2D 5k 171 / 81, 61k
+// 192 / 112, 300k after 1,500 substeps 491 / 363, 900k 1430 / 1371.
 constexpr int64_t kSmallWarpsPerSm = 512;
 // Cells per SM from which on a block takes all its threads (launch_small_step).
 constexpr int64_t kCellsPerSm = 16384;
@@ -54,10 +54,6 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
     // 93, 8k 155 / 95, 27k 177 / 143; in 2D, a third of the neighbours, 5k 132 / 122)
     const int64_t runs = ((f.n + kBlock - 1) / kBlock * (kBlock / 32) + c.sms - 1) / c.sms;
     const int lanes = runs * 8 <= 32 ? 8 : runs * 4 <= 32 ? 4 : 1;
-    // several runs a warp in 3D: taken from a queue (us a substep of a developed flow
-    // with fixed turns and with the queue: 216k 478 / 442, 439k 756 / 706, 1M
-    // 1614 / 1385; 205k from rest 425 / 424).  In 2D, with less work a run, it gave
-    // nothing: 300k 363 / 362, 900k 1371 / 1395.
     // The boundary's runs have warps of their own beside them, unless one or two more
     // would take a block past 512 threads: the next size, 1,024, is slower (5k in 2D
     // 90 and 92 us for a substep and the copies of its start state) and takes all of
@@ -81,6 +77,10 @@ cudaError_t launch_small_step(tsph_ctx &c, const tsph_set &f, const tsph_set &b,
         if (e == cudaSuccess) e = cudaMemsetAsync(c.X.bar + kBarTailF, 0, 4 * (kBarWords - kBarTailF), st);
         if (e != cudaSuccess) return e;
     }
+    // several runs a warp in 3D: taken from a queue (us a substep of a developed flow
+    // with fixed turns and with the queue: 216k 478 / 442, 439k 756 / 706, 1M
+    // 1614 / 1385; 205k from rest 425 / 424).  In 2D, with less work a run, it gave
+    // nothing: 300k 363 / 362, 900k 1371 / 1395.
     const bool d3 = c.k.dim == 3;
     switch (lanes) {
         case 8:

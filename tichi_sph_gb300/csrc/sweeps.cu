@@ -247,8 +247,11 @@ __global__ void __launch_bounds__(kBlock) k_normal(KConst k, FluidBuf F, BoundBu
     normal_item<DIM, TPP, M, true>(k, F, B, c, st, ln, ln.s, ln.s - c.f_slot < c.f_n);
 }
 
-// Held to 48 registers, 5 blocks per SM, without spills (64 batched scenes: 1,713 us
-// a substep, 1,739 with the 70 registers the batched instance takes unbounded).
+// Held to 48 registers, 5 blocks per SM (64 batched scenes: 1,713 us a substep, 1,739
+// with the 70 registers the batched instance takes unbounded).  Batched instances
+// with surface tension spill up to 236 bytes so and are faster all the same (the
+// phase, unbounded before and now, us, with one and eight lanes: 16 scenes of 64k
+// 583 / 412 and 1301 / 823, 32 of 4.9k in 2D 37 / 28 and 104 / 72).
 template <int DIM, bool ST, int TPP, bool M>
 __global__ void __launch_bounds__(kBlock, 5) k_advect(KConst k, FluidBuf F, BoundBuf B, float gs, float vs) {
     pdl_entry();

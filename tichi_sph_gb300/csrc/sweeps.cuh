@@ -163,29 +163,6 @@ __device__ __noinline__ void density_exact(const KConst &k, const FluidBuf &F, c
     out = a;
 }
 
-// SPH_clean_value + SPH_prepare_attr (f,f)(f,b) + SPH_prepare_alpha_1 (f,f)(f,b)
-// + SPH_prepare_alpha_2 (f,f) + SPH_prepare_alpha (sph.py:22-38, 50-105), and the
-// neighbour list of the step.
-//
-// Two phases keep the warps converged: the candidate scan only tests r < h and
-// records the pairs, then the recorded list is walked for the kernel
-// arithmetic.  Bound by instruction issue and, nearly as much, by L1 wavefronts
-// (about 290 warp instructions per particle, L1 at 68%): the scan tests without
-// a branch (visit_hits_r1), and what only a few particles need is out of line
-// (density_exact).  64 registers, 4 blocks per SM: at 80 or 48 registers 1M
-// particles take 391 and 395 us against 365 (48 registers spill the scan's
-// loads in flight); scan and arithmetic as two launches took 389 us.  From
-// 463 us before (one test and branch per candidate, 40 registers); 205k
-// particles 120 -> 100 us, 8k 78 -> 41 us.
-//
-// The divergence solve's first psi sweep (k_psi's work for its iteration 0) is
-// done here as well when that solve will run
-// (iter_min > 0 or the carried-over compression above the tolerance, the test
-// k_solve_begin makes): its pair terms need only positions and the v_adv the
-// solve starts from, both fixed here, and walk the same pairs in the same
-// order as k_psi with one thread per particle, with the same arithmetic; the
-// scene's psi_sum goes through the same partials and ticket.  psi_ready tells
-// k_psi to skip that iteration (64 batched scenes: 1,794 -> 1,739 us a substep).
 // Whether the density sweep does the divergence solve's first psi sweep.
 __device__ __forceinline__ bool density_does_psi(const SceneConst &c, double compression) {
     return c.f_n > 0 && ((0 < c.iter_min) || (compression > (double)c.div_tol));
@@ -223,6 +200,30 @@ __device__ __forceinline__ double density_store(const KConst &k, const FluidBuf 
     return 0.0;
 }
 
+// SPH_clean_value + SPH_prepare_attr (f,f)(f,b) + SPH_prepare_alpha_1 (f,f)(f,b)
+// + SPH_prepare_alpha_2 (f,f) + SPH_prepare_alpha (sph.py:22-38, 50-105), and the
+// neighbour list of the step.
+//
+// Two phases keep the warps converged: the candidate scan only tests r < h and
+// records the pairs, then the recorded list is walked for the kernel
+// arithmetic.  Bound by instruction issue and, nearly as much, by L1 wavefronts
+// (216k particles: 260 warp instructions per particle, L1 at 68%): the scan tests
+// without a branch (visit_hits_r1), and what only a few particles need is out of
+// line (density_exact).  64 registers, 4 blocks per SM: at 80 or 48 registers 1M
+// particles take 391 and 395 us against 365 (48 registers spill the scan's
+// loads in flight); scan and arithmetic as two launches took 389 us.  From
+// 463 us before (one test and branch per candidate, 40 registers); 205k
+// particles 120 -> 100 us, 8k 78 -> 41 us.
+//
+// The divergence solve's first psi sweep (k_psi's work for its iteration 0) is
+// done here as well when that solve will run
+// (iter_min > 0 or the carried-over compression above the tolerance, the test
+// k_solve_begin makes): its pair terms need only positions and the v_adv the
+// solve starts from, both fixed here, and walk the same pairs in the same
+// order as k_psi with one thread per particle, with the same arithmetic; the
+// scene's psi_sum goes through the same partials and ticket.  psi_ready tells
+// k_psi to skip that iteration (64 batched scenes: 1,794 -> 1,739 us a substep).
+//
 // Returns the particle's share of the scene's psi_sum (0 without psi0).
 template <int DIM, bool M, bool R1, bool NC>
 __device__ __forceinline__ double density_fluid_item(const KConst &k, const FluidBuf &F, const BoundBuf &B, int sc,

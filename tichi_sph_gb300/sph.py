@@ -2,7 +2,7 @@
 
 ``sph.py`` of Tichi_SPH exposes ~27 Taichi kernels that ``main.py:175-256``
 (``sph_step``) calls in a fixed order.  Here that whole sequence is one call of
-the C ABI (``tsph_sph_step`` / ``tsph_substep``), replayed as a CUDA graph with
+the C ABI (``tsph_sph_step`` / ``tsph_substep``), run as one launch with
 device-side solver loops.  :class:`Solver` owns the context; the module-level
 ``cfl_condition`` / ``sph_step`` mirror the reference's entry points.
 
@@ -170,7 +170,8 @@ class Solver:
                   "tsph_sph_step")
 
     def substep(self):
-        """cfl_condition + clock + sph_step (main.py:348-350) as one graph launch."""
+        """cfl_condition + clock + sph_step (main.py:348-350) as one launch: a
+        cooperative kernel, or a CUDA graph."""
         f, b = self._sets()
         with _on(self.device):
             check(self._lib.tsph_substep(self.ctx, f, b, _native.C.c_void_p(_stream_handle(self.device))),
