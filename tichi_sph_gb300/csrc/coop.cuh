@@ -70,7 +70,7 @@ struct WarpShare {
 // flow has developed, a share that lies together is all surface or all interior, and
 // a sweep waits for the interior's (us a substep of a dam break after 500
 // substeps, together and dealt: 439k 706 / 716, 512k 849 / 809, 1M
-// 1535 / 1385; with groups of 8 the 1M step from rest takes 1610 instead of 1528).
+// 1535 / 1385; with groups of 8 the 1M step from rest takes 5% longer).
 struct QueueShare {
     static constexpr unsigned int kGroup = 16, kDealt = 96;
     unsigned int first, runs, skip;  // skip: runs between the block's groups
